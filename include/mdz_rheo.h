@@ -664,6 +664,10 @@ int mdz_rheo_div_selftest(int device, const double *a, int64_t n, double b, doub
  * reciprocal estimate (within 2 ulp of the IEEE quotient; den outside [2^-1000, 2^1000]
  * takes the IEEE division), for n host pairs.  No reference counterpart. */
 int mdz_rheo_quotient_selftest(int device, const double *r, const double *den, int64_t n, double *out);
+/* Self-check of the fixed-point functions of the local update (fx64.cuh): out[k n + i] for
+ * k = 0..5 is exp, log, 1/x, sqrt, sin and cos of x[i], for n host arguments.  No reference
+ * counterpart. */
+int mdz_rheo_fx_selftest(int device, const double *x, int64_t n, double *out);
 /* Self-check of the cell-index ceil used by mdz_rheo_marker_stress: ceil(q[i]) from the
  * bits of q (saturated to +-2^30 beyond that range and for NaN) and CUDA's ceil, for n
  * host arguments.  No reference counterpart. */

@@ -11,6 +11,8 @@
 // mdz_rheo_quotient_selftest: the output quotient of fp64_div.cuh (two Newton steps on the
 // reciprocal estimate), for the accuracy test against IEEE division.
 // mdz_rheo_ceil_selftest: the integer-pipe ceil of fp64_bits.cuh next to CUDA's ceil.
+// mdz_rheo_fx_selftest: the fixed-point exp, log, reciprocal, square root, sine and cosine
+// of fx64.cuh, for the accuracy tests.
 // mdz_rheo_dd_selftest: the double-float conversion, exp and log of dd_math.cuh, for the
 // accuracy tests.
 #include <cuda_runtime.h>
@@ -19,6 +21,7 @@
 #include "dd_math.cuh"
 #include "fp64_div.cuh"
 #include "fp64_math.cuh"
+#include "fx64.cuh"
 
 namespace {
 
@@ -53,6 +56,18 @@ __global__ void k_div(const double *a, long long n, mdz::Divisor d, double *fast
   if (i >= n) return;
   fast[i] = mdz::div_by(a[i], d);
   plain[i] = a[i] / d.b;
+}
+
+// out[6][n]: exp, log, 1/x, sqrt, sin, cos of x
+__global__ void k_fx(const double *x, long long n, double *out) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double v = x[i];
+  out[i] = mdz::fx_exp(v);
+  out[n + i] = mdz::fx_log(v);
+  out[2 * n + i] = mdz::fx_recip(v);
+  out[3 * n + i] = mdz::fx_sqrt(v);
+  mdz::fx_sincos(v, &out[4 * n + i], &out[5 * n + i]);
 }
 
 __global__ void k_quotient(const double *r, const double *den, long long n, double *out) {
@@ -99,6 +114,24 @@ extern "C" int mdz_rheo_dd_selftest(int device, const double *x, int64_t n, floa
     if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) rc = MDZ_ECUDA;
   }
   if (rc == MDZ_OK && cudaMemcpy(out, dout, bo, cudaMemcpyDeviceToHost) != cudaSuccess) rc = MDZ_ECUDA;
+  cudaFree(d);
+  return rc;
+}
+
+extern "C" int mdz_rheo_fx_selftest(int device, const double *x, int64_t n, double *out) {
+  if (!x || n < 0 || !out) return MDZ_EINVAL;
+  if (n == 0) return MDZ_OK;
+  if (cudaSetDevice(device) != cudaSuccess) return MDZ_ECUDA;
+  const size_t bytes = (size_t)n * sizeof(double);
+  double *d = nullptr;
+  if (cudaMalloc(&d, 7 * bytes) != cudaSuccess) return MDZ_ENOMEM;
+  int rc = MDZ_OK;
+  if (cudaMemcpy(d, x, bytes, cudaMemcpyHostToDevice) != cudaSuccess) rc = MDZ_ECUDA;
+  if (rc == MDZ_OK) {
+    k_fx<<<(unsigned)((n + 255) / 256), 256>>>(d, n, d + n);
+    if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) rc = MDZ_ECUDA;
+  }
+  if (rc == MDZ_OK && cudaMemcpy(out, d + n, 6 * bytes, cudaMemcpyDeviceToHost) != cudaSuccess) rc = MDZ_ECUDA;
   cudaFree(d);
   return rc;
 }

@@ -46,17 +46,17 @@ __device__ __forceinline__ void phase_loop(const OpArgs &A, const OpNode &nd, bo
       IsoMid m;
       bool yields = false;
       if (active) {
-        iso_setup(A.M, A.ph[p], in, ctx, st, o, A.polish == 0);
-        iso_ve(A.M, A.ph[p], in, ctx, st, 1.0f, A.polish, o, m);
+        iso_setup<FdMath>(A.M, A.ph[p], in, ctx, st, o, A.polish == 0);
+        iso_ve<FdMath>(A.M, A.ph[p], in, ctx, st, 1.0f, A.polish, o, m);
         yields = iso_yields_dp(A.M, A.ph[p], ctx, m);
       }
       dp_compact(A.M, A.ph[p], *Q, *par, yields, m, in, ctx);
       if (!active) continue;
-      iso_post(A.M, A.ph[p], in, ctx, st, o, m);
+      iso_post<FdMath>(A.M, A.ph[p], in, ctx, st, o, m);
     } else if (ANISO) {
-      point_aniso(A.M, A.ph[p], in, ctx, an, A.polish, o);
+      point_aniso<FdMath>(A.M, A.ph[p], in, ctx, an, A.polish, o);
     } else {
-      point_iso(A.M, A.ph[p], in, ctx, A.polish, o);
+      point_iso<FdMath>(A.M, A.ph[p], in, ctx, A.polish, o);
     }
     const double eta_vep = o.etaVE;
     const int avg = A.M.eta_average;
@@ -87,8 +87,8 @@ __device__ __forceinline__ void fd_derivatives(const OpArgs &A, const OpNode &nd
   NodeCtx base;
   AnisoNode base_an;
   if (has) {
-    if (ANISO) node_setup_aniso(A.M, b, A.need_lnd != 0, base, base_an);
-    else node_setup_iso(A.M, b, A.need_lnd != 0, base);
+    if (ANISO) node_setup_aniso<FdMath>(A.M, b, A.need_lnd != 0, base, base_an);
+    else node_setup_iso<FdMath>(A.M, b, A.need_lnd != 0, base);
   }
 #pragma unroll 1
   for (int dir = 0; dir < 4; dir++) {
@@ -107,9 +107,9 @@ __device__ __forceinline__ void fd_derivatives(const OpArgs &A, const OpNode &nd
       NodeCtx ctx = base;
       AnisoNode an = base_an;
       if (has && dir < 3) {
-        if (ANISO) node_strain_aniso(in, ctx, an);
-        else node_strain_iso(A.M, in, ctx);
-        node_strain_update(ctx);
+        if (ANISO) node_strain_aniso<FdMath>(in, ctx, an);
+        else node_strain_iso<FdMath>(A.M, in, ctx);
+        node_strain_update<FdMath>(ctx);
       }
       phase_loop<ANISO, COMPACT>(A, nd, has, in, ctx, an, is_centroid, sign, denom, d[dir],
                                  nd.centroid ? v[dir] : vscratch, a[dir], &drhodp, Q, par);
@@ -212,7 +212,7 @@ __device__ __forceinline__ void newton_inputs(const OpArgs &A, NewtonNode &w) {
   const double exx = nd.centroid ? A.ci[CI_exxd][c] : A.vi[VI_exxd][c];
   const double ezz = nd.centroid ? A.ci[CI_ezzd][c] : A.vi[VI_ezzd][c];
   const double exz = nd.centroid ? A.ci[CI_exz][c] : A.vi[VI_exz][c];
-  effective_strain_rate(in.Exx, in.Ezz, in.Exz, exx, ezz, exz, in.Txx0, in.Tzz0, in.Txz0, w.d1, w.d2, w.aniS,
+  effective_strain_rate<FdMath>(in.Exx, in.Ezz, in.Exz, exx, ezz, exz, in.Txx0, in.Tzz0, in.Txz0, w.d1, w.d2, w.aniS,
                         eta_e, M.elastic);
 }
 

@@ -35,8 +35,37 @@
 #include "fp64_bits.cuh"
 #include "fp64_div.cuh"
 #include "fp64_math.cuh"
+#include "fx64.cuh"
 
 namespace mdz {
+
+// The elementary functions of the local update, in two kinds.
+//
+// FxMath (sweeps, points): 64-bit fixed point on the integer pipe (fx64.cuh), no FP64
+// instruction but the final product of a quotient.
+// FdMath (the operators' finite differences): the FP64 forms.  A central difference over a
+// step of 1e-7 magnifies a change of the last bit of its solves to 1e-9 and more of the
+// derivative, so the operators keep the bits of these forms.
+struct FxMath {
+  static __device__ __forceinline__ double exp(double x) { return fx_exp(x); }
+  static __device__ __forceinline__ double log(double x) { return fx_log(x); }
+  static __device__ __forceinline__ double recip(double x) { return fx_recip(x); }
+  static __device__ __forceinline__ double quotient(double r, double d) { return __dmul_rn(r, fx_recip(d)); }
+  static __device__ __forceinline__ double newton_quotient(double r, double d) { return __dmul_rn(r, fx_recip(d)); }
+  static __device__ __forceinline__ double divide(double r, double d) { return __dmul_rn(r, fx_recip(d)); }
+  static __device__ __forceinline__ double sqrt(double x) { return fx_sqrt(x); }
+  static __device__ __forceinline__ void sincos(double x, double *s, double *c) { fx_sincos(x, s, c); }
+};
+struct FdMath {
+  static __device__ __forceinline__ double exp(double x) { return fast_exp(x); }
+  static __device__ __forceinline__ double log(double x) { return fast_log(x); }
+  static __device__ __forceinline__ double recip(double x) { return mdz::quotient(1.0, x); }
+  static __device__ __forceinline__ double quotient(double r, double d) { return mdz::quotient(r, d); }
+  static __device__ __forceinline__ double newton_quotient(double r, double d) { return mdz::newton_quotient(r, d); }
+  static __device__ __forceinline__ double divide(double r, double d) { return r / d; }
+  static __device__ __forceinline__ double sqrt(double x) { return ::sqrt(x); }
+  static __device__ __forceinline__ void sincos(double x, double *s, double *c) { ::sincos(x, s, c); }
+};
 
 constexpr double kZeroC = 273.15;                 // MDLIB/include/mdoodz.h:4
 constexpr double kLn2 = 0.69314718055994530942;
@@ -127,47 +156,52 @@ __device__ __forceinline__ void set_status(int &st, int code) {
 // ---------------------------------------------------------------------------------------
 // node set-up: invariants and switches shared by the phases (RheologyDensity.c:461-496)
 // ---------------------------------------------------------------------------------------
+template <class FP>
 __device__ __forceinline__ void node_strain_update(NodeCtx &c);
 
+template <class FP>
 __device__ __forceinline__ void node_common(const ModelConst &M, const NodeIn &in, bool need_lnd, NodeCtx &c) {
-  node_strain_update(c);
+  node_strain_update<FP>(c);
   c.Traw = in.T;
   c.T = fp64_lt(in.T, M.Tmin) ? M.Tmin : in.T;
-  c.invT = quotient(1.0, c.T);
-  c.lnd = need_lnd ? fast_log(in.d) : 0.0;
+  c.invT = FP::recip(c.T);
+  c.lnd = need_lnd ? FP::log(in.d) : 0.0;
   c.inv_d = 0.0;
-  sincos(in.fric, &c.sin_fric, &c.cos_fric);
+  FP::sincos(in.fric, &c.sin_fric, &c.cos_fric);
   c.sin_dil = fp64_is_zero(c.dil) ? 0.0 : sin(c.dil);
 }
 
 // The strain-rate invariant and what depends on it (RheologyDensity.c:455-459); the
 // rest of the node set-up does not depend on the strain rate.
+template <class FP>
 __device__ __forceinline__ void node_strain_iso(const ModelConst &M, const NodeIn &in, NodeCtx &c) {
   const double Eyy = -(in.Exx + in.Ezz);
-  double Eii = sqrt(0.5 * (in.Exx * in.Exx + in.Ezz * in.Ezz + Eyy * Eyy) + in.Exz * in.Exz);
+  double Eii = FP::sqrt(0.5 * (in.Exx * in.Exx + in.Ezz * in.Ezz + Eyy * Eyy) + in.Exz * in.Exz);
   if (fp64_lt(Eii * M.scale_E, 1e-30)) Eii = M.Eii_floor;
   c.Eii = Eii;
 }
 
+template <class FP>
 __device__ __forceinline__ void node_strain_update(NodeCtx &c) {
-  c.lnEii = fast_log(c.Eii);
-  c.inv2Eii = quotient(0.5, c.Eii);
+  c.lnEii = FP::log(c.Eii);
+  c.inv2Eii = FP::quotient(0.5, c.Eii);
 }
 
+template <class FP>
 __device__ __forceinline__ void node_setup_iso(const ModelConst &M, const NodeIn &in, bool need_lnd,
                                                NodeCtx &c) {
-  node_strain_iso(M, in, c);
+  node_strain_iso<FP>(M, in, c);
   c.elastic = (M.step == 0) ? 0 : M.elastic;
   c.plastic_on = (M.step != 0);
-  c.K = quotient(1.0, in.beta);
+  c.K = FP::recip(in.beta);
   c.G = in.G;
   c.dil = in.dil;
   if (c.elastic == 0) { c.G = 1e1; c.dil = 0.0; c.K = 1e10; }
   c.eta_el = c.G * M.dt;
-  c.inv_eta_el = quotient(1.0, c.eta_el);
-  c.ln_eta_el = c.elastic ? fast_log(c.eta_el) : 0.0;
-  c.inv_Kdt = quotient(1.0, c.K * M.dt);
-  node_common(M, in, need_lnd, c);
+  c.inv_eta_el = FP::recip(c.eta_el);
+  c.ln_eta_el = c.elastic ? FP::log(c.eta_el) : 0.0;
+  c.inv_Kdt = FP::recip(c.K * M.dt);
+  node_common<FP>(M, in, need_lnd, c);
 }
 
 // EvaluateDensity, RheologyDensity.c:1761-1831 (models 0, 1, 3, 5)
@@ -204,8 +238,10 @@ struct Laws {
 };
 
 // 1/eta_k itself, where a caller needs it in linear form
-__device__ __forceinline__ double law_inv(const Laws &L, int k) { return fast_exp(L.ln_inv[k]); }
+template <class FP>
+__device__ __forceinline__ double law_inv(const Laws &L, int k) { return FP::exp(L.ln_inv[k]); }
 
+template <class FP>
 __device__ __forceinline__ void creep_laws(const ModelConst &M, const PhaseConst &ph, const NodeCtx &c, double P,
                                            double phi, double lnd, int peierls, Laws &L) {
   const int fl = ph.flags;
@@ -239,7 +275,7 @@ __device__ __forceinline__ void creep_laws(const ModelConst &M, const PhaseConst
     const double nE = L.ST + ph.exp_n;
     L.n[K_EXP] = nE;
     L.lnA_exp = ph.exp_lnA0 - ph.exp_EaR * ph.exp_om2 * c.invT;
-    L.ln_inv[K_EXP] = (kLn2 + ph.exp_ln_s3gS + lnEii) - quotient(lnEii - L.lnA_exp, nE);
+    L.ln_inv[K_EXP] = (kLn2 + ph.exp_ln_s3gS + lnEii) - FP::quotient(lnEii - L.lnA_exp, nE);
   }
   if (fl & F_GBS) {
     double lnB = ph.gbs_lnK + (ph.gbs_Q + P * ph.gbs_V) * ph.gbs_invRn * c.invT - ph.gbs_an * phi;
@@ -276,6 +312,7 @@ struct VeState {
   int iters, status;
 };
 
+template <class FP>
 __device__ __forceinline__ void ve_coef(const Laws &L, const NodeCtx &c, double eta_cst, double eta_up,
                                         double ln_eta_up, VeCoef &q) {
   const double Eii = c.Eii;
@@ -298,7 +335,7 @@ __device__ __forceinline__ void ve_coef(const Laws &L, const NodeCtx &c, double 
     q.nc[k] = 0.0;
     if (!(L.mech & bit)) continue;
     if (k != K_EXP && fp64_eq_nonzero(L.n[k], 1.0)) {  // Newtonian law: Eii eta / eta_k
-      const double a = Eii * law_inv(L, k);
+      const double a = Eii * law_inv<FP>(L, k);
       if (k == K_LIN) q.a_lin1 = a;
       else q.a_pwl1 = a;
       A += a;
@@ -325,6 +362,7 @@ __device__ __forceinline__ void ve_coef(const Laws &L, const NodeCtx &c, double 
 //     (1 + step)^n = 1 + n step (1 + (n - 1) step / 2) + O((n step)^3),
 // used only where |n step| < 1e-5, so the dropped term is below 2e-16 relative: the same
 // residual as a fresh evaluation to rounding, without its log and exps.
+template <class FP>
 __device__ __forceinline__ void ve_eval(const VeCoef &q, double sv, VeState &s, double &r, double step = -1.0) {
   double *e = s.e;
   if (fp64_ge(step, -0.5)) {
@@ -337,10 +375,10 @@ __device__ __forceinline__ void ve_eval(const VeCoef &q, double sv, VeState &s, 
   } else {
     e[0] = e[1] = e[2] = 0.0;
     if (q.nl) {
-      const double lx = fast_log(sv) + q.lp;
+      const double lx = FP::log(sv) + q.lp;
 #pragma unroll
       for (int k = 0; k < K_COUNT; k++)
-        if (q.nl >> k & 1) e[k] = q.Eii * fast_exp(fma(q.n[k], lx, q.nc[k]));
+        if (q.nl >> k & 1) e[k] = q.Eii * FP::exp(fma(q.n[k], lx, q.nc[k]));
     }
   }
   const double eta = sv * q.eta_up;
@@ -366,6 +404,7 @@ __device__ __forceinline__ double ve_S(const VeCoef &q, const VeState &s) {
 // A moved start (one the start stages chose) that has not converged within the cap is
 // abandoned: the iteration runs again from the upper bound eta_up (s_up), with the
 // reference's cap, and the evaluations of both runs count.
+template <class FP>
 __device__ __forceinline__ void ve_newton(const VeCoef &q, double sv, VeState &s, float s_up = 1.0f,
                                           bool moved = false) {
   const int nitmax = 20;
@@ -373,7 +412,7 @@ __device__ __forceinline__ void ve_newton(const VeCoef &q, double sv, VeState &s
   double step = -1.0;  // no previous point yet
   for (int it = 0; it < nitmax; it++) {
     double r;
-    ve_eval(q, sv, s, r, step);
+    ve_eval<FP>(q, sv, s, r, step);
     s.iters++;
     if (fp64_abs_lt(r, q.thr_conv)) break;
     if (it == nitmax - 1 && moved) {  // back to the upper bound
@@ -384,7 +423,7 @@ __device__ __forceinline__ void ve_newton(const VeCoef &q, double sv, VeState &s
       continue;
     }
     if (it == nitmax - 1 && fabs(r) > q.thr_fail) { set_status(s.status, MDZ_EVE_ITER); break; }
-    const double d = newton_quotient(r, fma(q.Aup, sv, ve_S(q, s)));
+    const double d = FP::newton_quotient(r, fma(q.Aup, sv, ve_S(q, s)));
     sv = fma(sv, d, sv);
     step = fp64_lt(fabs(d) * q.nmax, 1e-5) ? d : -1.0;
   }
@@ -688,6 +727,7 @@ struct IsoState {
 // Start point of the local solve (RheologyDensity.c:582-592, AnisotropyRoutines.c:409-415):
 // the smallest of the initial bound, eta_cst, the isolated creep viscosities and eta_el,
 // with its logarithm for the normalised residual.
+template <class FP>
 __device__ __forceinline__ void start_viscosity(const ModelConst &M, double ln_inv_max, bool constant,
                                                 double eta_cst, bool elastic, const NodeCtx &c, double &eta_up,
                                                 double &ln_eta_up) {
@@ -696,11 +736,11 @@ __device__ __forceinline__ void start_viscosity(const ModelConst &M, double ln_i
   bool from_cst = false;
   if (constant && fp64_lt(eta_cst, eta_up)) { eta_up = eta_cst; from_cst = true; }
   if (fp64_gt(ln_inv_max, -kInf)) {
-    const double e = fast_exp(-ln_inv_max);
+    const double e = FP::exp(-ln_inv_max);
     if (fp64_lt(e, eta_up)) { eta_up = e; ln_eta_up = -ln_inv_max; from_cst = false; }
   }
   if (elastic && fp64_lt(c.eta_el, eta_up)) { eta_up = c.eta_el; ln_eta_up = c.ln_eta_el; from_cst = false; }
-  if (from_cst) ln_eta_up = fast_log(eta_cst);
+  if (from_cst) ln_eta_up = FP::log(eta_cst);
 }
 
 // The start point and the normalisation of the local solve.  Exact (the reference's start,
@@ -710,12 +750,13 @@ __device__ __forceinline__ void start_viscosity(const ModelConst &M, double ln_i
 // smallest of the candidates' logarithms (compared on the integer pipe; no exp), and the
 // unknown is normalised by eta_n = 2^k, k the nearest integer to log2(eta_up), built from
 // bits, with ln(eta_n) = k ln2; s_up = exp(ln eta_up - k ln2) in [0.7, 1.42] in FP32.
+template <class FP>
 __device__ __forceinline__ void start_point(const ModelConst &M, double ln_inv_max, bool constant, double eta_cst,
                                             bool elastic, const NodeCtx &c, bool exact, IsoState &S) {
   if (!exact) {
     double ln = M.ln_eta_up0;
     if (constant) {
-      const double lc = fast_log(eta_cst);
+      const double lc = FP::log(eta_cst);
       if (fp64_lt(lc, ln)) ln = lc;
     }
     if (fp64_gt(ln_inv_max, -kInf) && fp64_lt(-ln_inv_max, ln)) ln = -ln_inv_max;
@@ -732,7 +773,7 @@ __device__ __forceinline__ void start_point(const ModelConst &M, double ln_inv_m
       return;
     }
   }
-  start_viscosity(M, ln_inv_max, constant, eta_cst, elastic, c, S.eta_up, S.ln_eta_up);
+  start_viscosity<FP>(M, ln_inv_max, constant, eta_cst, elastic, c, S.eta_up, S.ln_eta_up);
   S.eta_n = S.eta_up;
   S.ln_eta_n = S.ln_eta_up;
   S.s_up = 1.0f;
@@ -740,19 +781,21 @@ __device__ __forceinline__ void start_point(const ModelConst &M, double ln_inv_m
 
 // Lower end of the reference's bracket: the largest of the lower bound, eta_cst, eta_el and
 // the isolated creep viscosities (needed by the grain-size solve and the bisection only).
+template <class FP>
 __device__ __forceinline__ double lower_viscosity(const ModelConst &M, const Laws &L, bool constant, double eta_cst,
                                                   bool elastic, double eta_el, bool gbs) {
   double eta_lo = M.eta_lo0;
   if (constant) eta_lo = fmax(eta_lo, eta_cst);
-  if (L.mech & F_PWL) eta_lo = fmax(eta_lo, fast_exp(-L.ln_inv[K_PWL]));
+  if (L.mech & F_PWL) eta_lo = fmax(eta_lo, FP::exp(-L.ln_inv[K_PWL]));
   if (elastic) eta_lo = fmax(eta_lo, eta_el);
-  if (L.mech & F_EXPV) eta_lo = fmax(eta_lo, fast_exp(-L.ln_inv[K_EXP]));
-  if (L.mech & F_LIN) eta_lo = fmax(eta_lo, fast_exp(-L.ln_inv[K_LIN]));
-  if (gbs) eta_lo = fmax(eta_lo, fast_exp(-L.ln_inv_gbs));
+  if (L.mech & F_EXPV) eta_lo = fmax(eta_lo, FP::exp(-L.ln_inv[K_EXP]));
+  if (L.mech & F_LIN) eta_lo = fmax(eta_lo, FP::exp(-L.ln_inv[K_LIN]));
+  if (gbs) eta_lo = fmax(eta_lo, FP::exp(-L.ln_inv_gbs));
   return eta_lo;
 }
 
 // exact: the local solve starts where the reference's does (start descriptor 0)
+template <class FP>
 __device__ inline void iso_setup(const ModelConst &M, const PhaseConst &ph, const NodeIn &in, const NodeCtx &c,
                                  IsoState &S, PointOut &o, bool exact = true) {
   const int fl = ph.flags;
@@ -779,7 +822,7 @@ __device__ inline void iso_setup(const ModelConst &M, const PhaseConst &ph, cons
   if (diffusion && fp64_gt(ph.lin_m, 0.0) && fp64_lt(in.d, M.d_min)) set_status(o.status, MDZ_EGRAIN_ZERO);
 
   Laws &L = S.L;
-  creep_laws(M, ph, c, P, in.phi, c.lnd, peierls, L);
+  creep_laws<FP>(M, ph, c, P, in.phi, c.lnd, peierls, L);
   double Tyield = 0.0, C = in.C;
   if (plastic == 1) {  // :530-539 (products and sum rounded apart: the same bits in every kernel)
     Tyield = __dadd_rn(__dmul_rn(C, c.cos_fric), __dmul_rn(P, c.sin_fric));
@@ -796,7 +839,7 @@ __device__ inline void iso_setup(const ModelConst &M, const PhaseConst &ph, cons
   if (gs) {  // wattmeter grain size before eta_lin (:567-576)
     Ag = ph.Kpzm * exp(-ph.Qpzm / M.R / T);
     const double Tii0 = 2. * eta_el * Eii;
-    const double epwl0 = Tii0 / 2.0 * law_inv(L, K_PWL);
+    const double epwl0 = Tii0 / 2.0 * law_inv<FP>(L, K_PWL);
     const double d = exp(log(Ag * ph.Gpzm / (ph.Lpzm * (1.0 / ph.cpzm) * Tii0 * epwl0 * ph.ppzm)) / (1.0 + ph.ppzm));
     o.d1 = d;
     lnd = log(d);
@@ -808,7 +851,7 @@ __device__ inline void iso_setup(const ModelConst &M, const PhaseConst &ph, cons
   // bracket (:582-592): the smallest isolated viscosity is 1 / the largest reciprocal
   const double ln_inv_max =
       fp64_fmax(fp64_fmax(L.ln_inv[K_PWL], L.ln_inv[K_EXP]), fp64_fmax(L.ln_inv[K_LIN], L.ln_inv_gbs));
-  start_point(M, ln_inv_max, constant, eta_cst, elastic == 1, c, exact || gs, S);
+  start_point<FP>(M, ln_inv_max, constant, eta_cst, elastic == 1, c, exact || gs, S);
   S.eta_cst = eta_cst; S.Tyield = Tyield; S.C = C; S.Ag = Ag; S.lnd = lnd;
 }
 
@@ -902,6 +945,7 @@ __device__ inline void dp_return(const ModelConst &M, const PhaseConst &ph, DpIt
 // `polish` names (ve_start); s_start = 1 and polish = 0 is the reference's start) of one
 // (node, phase), up to its plastic corrections.  eta_conv (may be null) receives the
 // converged visco-elastic viscosity, before plasticity.
+template <class FP>
 __device__ inline void iso_ve(const ModelConst &M, const PhaseConst &ph, const NodeIn &in, const NodeCtx &c,
                               IsoState &S, float s_start, int polish, PointOut &o, IsoMid &m,
                               double *eta_conv = nullptr) {
@@ -917,16 +961,16 @@ __device__ inline void iso_ve(const ModelConst &M, const PhaseConst &ph, const N
   double eta_ve, Tii, e_cst, e_pwl, e_exp, e_lin;
   if (!gs) {  // LocalIterationViscoElastic (:646)
     VeCoef q;
-    ve_coef(L, c, eta_cst, S.eta_n, S.ln_eta_n, q);
+    ve_coef<FP>(L, c, eta_cst, S.eta_n, S.ln_eta_n, q);
     VeState s;
     s.status = MDZ_OK;
-    ve_newton(q, ve_start(q, s_start * S.s_up, start_fp32(polish), start_dd(polish), o.f32_steps, S.s_up), s,
+    ve_newton<FP>(q, ve_start(q, s_start * S.s_up, start_fp32(polish), start_dd(polish), o.f32_steps, S.s_up), s,
               S.s_up, polish != 0);
     set_status(o.status, s.status);
     eta_ve = s.eta; Tii = s.Tii; e_cst = s.e_cst; e_pwl = s.e_pwl; e_exp = s.e_exp; e_lin = s.e_lin;
     o.iters = s.iters;
   } else {  // LocalIterationViscoElasticGrainSize (:644)
-    const double eta_lo = lower_viscosity(M, L, constant, eta_cst, elastic == 1, eta_el, gbs);
+    const double eta_lo = lower_viscosity<FP>(M, L, constant, eta_cst, elastic == 1, eta_el, gbs);
     GseIn g;
     g.Eii = Eii; g.eta_el = eta_el; g.eta_cst = eta_cst;
     g.C_pwl = exp(-ph.pwl_n * (kLn2 + L.lnB_pwl)); g.n_pwl = ph.pwl_n;
@@ -954,6 +998,7 @@ __device__ inline void iso_ve(const ModelConst &M, const PhaseConst &ph, const N
 
 // Plastic corrections but the Drucker-Prager return (which dp_return does), and the
 // post-processing of one (node, phase) after its visco-elastic solve (:655-1073).
+template <class FP>
 __device__ inline void iso_post(const ModelConst &M, const PhaseConst &ph, const NodeIn &in, const NodeCtx &c,
                                 IsoState &S, PointOut &o, IsoMid &m) {
   const int fl = ph.flags;
@@ -992,21 +1037,21 @@ __device__ inline void iso_post(const ModelConst &M, const PhaseConst &ph, const
 
   double inv_eta_pl = 0.0;
   if (is_pl == 0) o.etaVE = eta_ve;
-  else if (plastic == 1) { o.etaVE = eta_vep; inv_eta_pl = quotient(gdot, Tii); }
+  else if (plastic == 1) { o.etaVE = eta_vep; inv_eta_pl = FP::quotient(gdot, Tii); }
   else { o.etaVE = eta_vep; inv_eta_pl = 2.0 * lam_dot * A_tau / Tii; }
   o.is_pl = is_pl;
   if (is_pl) o.mech |= MDZ_MECH_YIELD;
   o.Eii_cst = e_cst; o.Eii_pwl = e_pwl; o.Eii_exp = e_exp; o.Eii_lin = e_lin;
   // the dissipative viscosity: 1 / eta = sum_k 2 Eii_k / Tii (+ 1/eta_cst, 1/eta_pl)
   const auto dissipative = [&](double &inv_half_T) {
-    inv_half_T = quotient(2.0, Tii_ve);  // 1/eta_k = 2 Eii_k / Tii
+    inv_half_T = FP::quotient(2.0, Tii_ve);  // 1/eta_k = 2 Eii_k / Tii
     double inv = 0.0;
     if (peierls) inv = __fma_rn(e_exp, inv_half_T, inv);
     if (dislocation) inv = __fma_rn(e_pwl, inv_half_T, inv);
     if (diffusion) {
       // eta_lin = B pow(Eii_lin, 1/n-1) pow(d1, m/n) = Tii/(2 Eii_lin) (d1/d)^(m/n), d1 = gs_ref
       double inv_lin = e_lin * inv_half_T;
-      if (!fp64_is_zero(ph.lin_m) && !gs) inv_lin *= fast_exp(ph.lin_mn * (lnd - ph.ln_gs_ref));
+      if (!fp64_is_zero(ph.lin_m) && !gs) inv_lin *= FP::exp(ph.lin_mn * (lnd - ph.ln_gs_ref));
       inv += inv_lin;
     }
     if (constant) inv += (1.0 / eta_cst);
@@ -1017,7 +1062,7 @@ __device__ inline void iso_post(const ModelConst &M, const PhaseConst &ph, const
   double eta = 0.0;
   if (in.post_process == 2) {  // a vertex of the sweep: only etaVE, eta and X are kept
     double inv_half_T;
-    eta = quotient(1.0, dissipative(inv_half_T));
+    eta = FP::recip(dissipative(inv_half_T));
   } else {
     o.Txx = 2.0 * o.etaVE * in.Exx;
     o.Tzz = 2.0 * o.etaVE * in.Ezz;
@@ -1025,13 +1070,13 @@ __device__ inline void iso_post(const ModelConst &M, const PhaseConst &ph, const
     if (in.post_process == 1) {  // :986-1053
       double inv_half_T;
       const double inv = dissipative(inv_half_T);
-      eta = quotient(1.0, inv);
+      eta = FP::recip(inv);
       if (elastic) {
         const double h = 0.5 * c.inv_eta_el;
         const double Tyy = -(o.Txx + o.Tzz), Tyy0 = -(in.Txx0 + in.Tzz0);
         const double ex = (o.Txx - in.Txx0) * h, ez = (o.Tzz - in.Tzz0) * h;
         const double ey = (Tyy - Tyy0) * h, exz = (o.Txz - in.Txz0) * h;
-        o.Eii_el = sqrt(__fma_rn(0.5, __fma_rn(ey, ey, __fma_rn(ez, ez, __dmul_rn(ex, ex))), __dmul_rn(exz, exz)));
+        o.Eii_el = FP::sqrt(__fma_rn(0.5, __fma_rn(ey, ey, __fma_rn(ez, ez, __dmul_rn(ex, ex))), __dmul_rn(exz, exz)));
       }
       o.Eii_pl = (is_pl && plastic == 1) ? gdot / 2.0 : ((is_pl && plastic == 2) ? lam_dot * A_tau : 0.0);
       o.div_pl = divp;
@@ -1061,25 +1106,27 @@ __device__ inline void iso_post(const ModelConst &M, const PhaseConst &ph, const
 
 // Local solve, plastic corrections and post-processing of one (node, phase): iso_ve, the
 // Drucker-Prager return where the item yields, iso_post.
+template <class FP>
 __device__ inline void iso_finish(const ModelConst &M, const PhaseConst &ph, const NodeIn &in, const NodeCtx &c,
                                   IsoState &S, float s_start, int polish, PointOut &o,
                                   double *eta_conv = nullptr) {
   IsoMid m;
-  iso_ve(M, ph, in, c, S, s_start, polish, o, m, eta_conv);
+  iso_ve<FP>(M, ph, in, c, S, s_start, polish, o, m, eta_conv);
   if (iso_yields_dp(M, ph, c, m)) {
     DpItem d;
     dp_load(d, m, in, c);
     dp_return(M, ph, d);
     dp_store(m, d);
   }
-  iso_post(M, ph, in, c, S, o, m);
+  iso_post<FP>(M, ph, in, c, S, o, m);
 }
 
+template <class FP>
 __device__ inline void point_iso(const ModelConst &M, const PhaseConst &ph, const NodeIn &in, const NodeCtx &c,
                                  int polish, PointOut &o) {
   IsoState S;
-  iso_setup(M, ph, in, c, S, o, polish == 0);
-  iso_finish(M, ph, in, c, S, 1.0f, polish, o);
+  iso_setup<FP>(M, ph, in, c, S, o, polish == 0);
+  iso_finish<FP>(M, ph, in, c, S, 1.0f, polish, o);
 }
 
 // CTA-level compaction of the Drucker-Prager returns.  The return of an item that yields
@@ -1133,6 +1180,7 @@ struct AnisoNode {
 };
 
 // Rotated strain rate and its invariant (AnisotropyRoutines.c:379-390).
+template <class FP>
 __device__ __forceinline__ void node_strain_aniso(const NodeIn &in, NodeCtx &c, AnisoNode &a) {
   const double lx2 = in.lx2, lxlz = in.lxlz, nz2 = 1.0 - lx2;  // :379-383
   a.lx2 = lx2; a.lxlz = lxlz;
@@ -1140,26 +1188,28 @@ __device__ __forceinline__ void node_strain_aniso(const NodeIn &in, NodeCtx &c, 
   a.Er_zz = nz2 * in.Exx + lx2 * in.Ezz - 2. * lxlz * in.Exz;
   a.Er_xz = -lxlz * in.Exx + lxlz * in.Ezz + (lx2 - nz2) * in.Exz;
   const double Er_yy = -a.Er_xx - a.Er_zz;
-  c.Eii = sqrt(0.5 * (a.Er_xx * a.Er_xx + a.Er_zz * a.Er_zz + Er_yy * Er_yy) + a.Er_xz * a.Er_xz);
+  c.Eii = FP::sqrt(0.5 * (a.Er_xx * a.Er_xx + a.Er_zz * a.Er_zz + Er_yy * Er_yy) + a.Er_xz * a.Er_xz);
 }
 
+template <class FP>
 __device__ __forceinline__ void node_setup_aniso(const ModelConst &M, const NodeIn &in, bool need_lnd, NodeCtx &c,
                                                  AnisoNode &a) {
-  node_strain_aniso(in, c, a);
+  node_strain_aniso<FP>(in, c, a);
   c.elastic = (M.step == 0) ? 0 : M.elastic;
   c.plastic_on = 1;
-  c.K = quotient(1.0, in.beta);
+  c.K = FP::recip(in.beta);
   c.G = in.G;
   c.dil = in.dil;
   if (c.elastic == 0) { c.G = 1e1; c.dil = 0.0; }
   c.eta_el = c.elastic ? c.G * M.dt_model : 1e20;
-  c.inv_eta_el = quotient(1.0, c.eta_el);
-  c.ln_eta_el = c.elastic ? fast_log(c.eta_el) : 0.0;
-  c.inv_Kdt = quotient(1.0, c.K * M.dt_model);
-  node_common(M, in, need_lnd, c);
-  c.inv_d = 1.0 / in.d;
+  c.inv_eta_el = FP::recip(c.eta_el);
+  c.ln_eta_el = c.elastic ? FP::log(c.eta_el) : 0.0;
+  c.inv_Kdt = FP::recip(c.K * M.dt_model);
+  node_common<FP>(M, in, need_lnd, c);
+  c.inv_d = FP::divide(1.0, in.d);
 }
 
+template <class FP>
 __device__ inline void aniso_setup(const ModelConst &M, const PhaseConst &ph, const NodeIn &in, const NodeCtx &c,
                                    const AnisoNode &an, IsoState &S, PointOut &o, bool exact = true) {
   const int fl = ph.flags;
@@ -1183,7 +1233,7 @@ __device__ inline void aniso_setup(const ModelConst &M, const PhaseConst &ph, co
   if (diffusion && fp64_gt(ph.lin_m, 0.0) && fp64_lt(in.d, M.d_min)) set_status(o.status, MDZ_EGRAIN_ZERO);
 
   Laws &L = S.L;
-  creep_laws(M, ph, c, P, in.phi, c.lnd, peierls, L);
+  creep_laws<FP>(M, ph, c, P, in.phi, c.lnd, peierls, L);
   L.mech &= ~F_GBS;  // the anisotropic path has no grain-boundary sliding
   L.ln_inv_gbs = -kInf;
   double Tyield = 0.0, Coh = in.C;
@@ -1194,7 +1244,7 @@ __device__ inline void aniso_setup(const ModelConst &M, const PhaseConst &ph, co
   const double eta_cst = constant ? ph.eta0 : 0.0;
   // bracket (:409-415); its lower end is formed only where it is used
   const double ln_inv_max = fp64_fmax(fp64_fmax(L.ln_inv[K_PWL], L.ln_inv[K_EXP]), L.ln_inv[K_LIN]);
-  start_point(M, ln_inv_max, constant, eta_cst, elastic != 0, c, exact || (fl & F_GS), S);
+  start_point<FP>(M, ln_inv_max, constant, eta_cst, elastic != 0, c, exact || (fl & F_GS), S);
   S.eta_cst = eta_cst; S.Tyield = Tyield; S.C = Coh; S.Ag = 0.0;
   S.lnd = c.lnd;
   (void)an; (void)T; (void)K; (void)dt; (void)min_eta; (void)max_eta; (void)dislocation; (void)eta_el;
@@ -1203,6 +1253,7 @@ __device__ inline void aniso_setup(const ModelConst &M, const PhaseConst &ph, co
 // Local solve, plasticity, post-processing.  The Newton starts from the reference's
 // bisection when s_start <= 0 and polish == 0; otherwise from s_start * eta_up (eta_up
 // when s_start <= 0) moved by the start stages that the descriptor `polish` names.
+template <class FP>
 __device__ inline void aniso_finish(const ModelConst &M, const PhaseConst &ph, const NodeIn &in, const NodeCtx &c,
                                    const AnisoNode &an, IsoState &S, float s_start, int polish, PointOut &o,
                                    double *eta_conv = nullptr) {
@@ -1222,7 +1273,7 @@ __device__ inline void aniso_finish(const ModelConst &M, const PhaseConst &ph, c
     g.C_pwl = exp(-ph.pwl_n * (kLn2 + L.lnB_pwl)); g.n_pwl = ph.pwl_n;
     g.C_lin = exp(-ph.lin_n * (kLn2 + L.lnB_lin)); g.n_lin = ph.lin_n; g.m_lin = ph.lin_m;
     g.C_exp = exp(fma(L.n[K_EXP], log(ph.exp_s3gS), L.lnA_exp)); g.ST = L.ST; g.n_exp = ph.exp_n;
-    g.eta_up = eta_up; g.eta_lo = lower_viscosity(M, L, constant, eta_cst, elastic != 0, eta_el, false);
+    g.eta_up = eta_up; g.eta_lo = lower_viscosity<FP>(M, L, constant, eta_cst, elastic != 0, eta_el, false);
     g.Ag = ph.Kpzm * exp(-ph.Qpzm / (M.R * T));
     g.gam = ph.Gpzm; g.lam = ph.Lpzm; g.cg = ph.cpzm; g.pg = ph.ppzm; g.elastic = elastic; g.constant = constant;
     g.dislocation = dislocation; g.peierls = peierls; g.diffusion = diffusion;
@@ -1235,7 +1286,7 @@ __device__ inline void aniso_finish(const ModelConst &M, const PhaseConst &ph, c
   } else {  // :474-585: 10 log-space bisection steps on [min_eta 1e-3, 10 max(eta_lo, max_eta)], then Newton
     const double tol = 1e-11;
     VeCoef q;
-    ve_coef(L, c, eta_cst, S.eta_n, S.ln_eta_n, q);
+    ve_coef<FP>(L, c, eta_cst, S.eta_n, S.ln_eta_n, q);
     VeState s;
     s.status = MDZ_OK;
     double r, sv;  // sv = eta_ve / eta_n (eta_n = eta_up from the bisection: that start is exact)
@@ -1244,11 +1295,11 @@ __device__ inline void aniso_finish(const ModelConst &M, const PhaseConst &ph, c
                     o.f32_steps, S.s_up);
     } else {
       const double inv_up = 1.0 / eta_up;
-      const double eta_lo = lower_viscosity(M, L, constant, eta_cst, elastic != 0, eta_el, false);
+      const double eta_lo = lower_viscosity<FP>(M, L, constant, eta_cst, elastic != 0, eta_el, false);
       double lo = min_eta * 1.0e-3, hi = 10.0 * fmax(eta_lo, max_eta);
       for (int bit = 0; bit < 10; bit++) {
         eta_ve = sqrt(lo * hi);
-        ve_eval(q, eta_ve * inv_up, s, r);
+        ve_eval<FP>(q, eta_ve * inv_up, s, r);
         if (r > 0.0) lo = eta_ve;
         else hi = eta_ve;
         if (fabs(r) < q.thr_conv) break;
@@ -1261,10 +1312,10 @@ __device__ inline void aniso_finish(const ModelConst &M, const PhaseConst &ph, c
     o.iters = 0;
     double step = -1.0;  // binomial update of the previous point's terms (see ve_eval)
     for (int it = 0; it < 50; it++) {
-      ve_eval(q, sv, s, r, step);
+      ve_eval<FP>(q, sv, s, r, step);
       o.iters++;
       if (fp64_is_nan(r)) { set_status(o.status, MDZ_EANISO_NAN); break; }
-      const double d = newton_quotient(r, fma(q.Aup, sv, ve_S(q, s)));
+      const double d = FP::newton_quotient(r, fma(q.Aup, sv, ve_S(q, s)));
       sv = fma(sv, d, sv);
       step = fp64_lt(fabs(d) * q.nmax, 1e-5) ? d : -1.0;
       if (fp64_le(sv, 0.0)) { sv = min_eta / q.eta_up; step = -1.0; }
@@ -1295,7 +1346,7 @@ __device__ inline void aniso_finish(const ModelConst &M, const PhaseConst &ph, c
     is_pl = 1;
     // rounded one by one, as in the isotropic return
     const double Kdt_sd = __dmul_rn(__dmul_rn(K, dt), c.sin_dil);
-    gdot = quotient(Ft, __dadd_rn(__dadd_rn(eta_ve, ph.eta_vp), __dmul_rn(Kdt_sd, c.sin_fric)));
+    gdot = FP::quotient(Ft, __dadd_rn(__dadd_rn(eta_ve, ph.eta_vp), __dmul_rn(Kdt_sd, c.sin_fric)));
     const double Tiic = __dsub_rn(Tii, __dmul_rn(gdot, eta_ve));
     Pc = __dadd_rn(P, __dmul_rn(Kdt_sd, gdot));
     eta_vep = Tiic * c.inv2Eii;
@@ -1322,13 +1373,13 @@ __device__ inline void aniso_finish(const ModelConst &M, const PhaseConst &ph, c
   double eta = eta_vep;
   double inv = 0.0;
   if (in.post_process != 0) {  // :681-714 (eta_lin uses *d, the same d as the Newton: no correction)
-    const double inv_half_T = quotient(2.0, Tii_ve);
+    const double inv_half_T = FP::quotient(2.0, Tii_ve);
     if (diffusion) inv += e_lin * inv_half_T;
     if (peierls) inv += e_exp * inv_half_T;
     if (dislocation) inv += e_pwl * inv_half_T;
     if (constant) inv += 1.0 / eta_cst;
-    if (is_pl) inv += quotient(gdot, Tii);
-    eta = quotient(1.0, inv);
+    if (is_pl) inv += FP::quotient(gdot, Tii);
+    eta = FP::recip(inv);
   }
   if (in.post_process == 1) {
     if (elastic) o.Eii_el = Tii * Tii * (0.25 * c.inv_eta_el * c.inv_eta_el);
@@ -1348,14 +1399,16 @@ __device__ inline void aniso_finish(const ModelConst &M, const PhaseConst &ph, c
   o.eta = eta;
 }
 
+template <class FP>
 __device__ inline void point_aniso(const ModelConst &M, const PhaseConst &ph, const NodeIn &in, const NodeCtx &c,
                                    const AnisoNode &an, int polish, PointOut &o) {
   IsoState S;
-  aniso_setup(M, ph, in, c, an, S, o, polish == 0);
-  aniso_finish(M, ph, in, c, an, S, 0.0f, polish, o);
+  aniso_setup<FP>(M, ph, in, c, an, S, o, polish == 0);
+  aniso_finish<FP>(M, ph, in, c, an, S, 0.0f, polish, o);
 }
 
 // EffectiveStrainRate, RheologyDensity.c:116-146
+template <class FP>
 __device__ __forceinline__ void effective_strain_rate(double &Exx, double &Ezz, double &Exz, double exx, double ezz,
                                                       double exz, double Txx, double Tzz, double Txz, double d1,
                                                       double d2, double ani, double eta_e, int elastic) {
@@ -1364,8 +1417,8 @@ __device__ __forceinline__ void effective_strain_rate(double &Exx, double &Ezz, 
   const double Da22 = 2.0 - 2.0 * ani * d1, Da23 = 2.0 * ani * d2, Da33 = 1.0 + 2.0 * ani * (d1 - 0.5);
   const double a11 = Da33 * Da22 - Da23 * Da23, a12 = Da13 * Da23 - Da33 * Da12, a13 = Da12 * Da23 - Da13 * Da22;
   const double a22 = Da33 * Da11 - Da13 * Da13, a23 = Da12 * Da13 - Da11 * Da23, a33 = Da11 * Da22 - Da12 * Da12;
-  const double idet = 1.0 / ((Da11 * a11) + (Da12 * a12) + (Da13 * a13));
-  const double ie = 1.0 / eta_e;
+  const double idet = FP::divide(1.0, (Da11 * a11) + (Da12 * a12) + (Da13 * a13));
+  const double ie = FP::divide(1.0, eta_e);
   Exx = exx + (a11 * Txx + a12 * Tzz + a13 * Txz) * idet * ie;
   Ezz = ezz + (a12 * Txx + a22 * Tzz + a23 * Txz) * idet * ie;
   Exz = exz + (a13 * Txx + a23 * Tzz + a33 * Txz) * idet * ie * 0.5;

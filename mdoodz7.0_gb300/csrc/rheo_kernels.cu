@@ -100,7 +100,6 @@ __device__ __forceinline__ void node_prepare(const SweepArgs &A, long long i, No
                                              const PerturbKey *pk = nullptr) {
   const ModelConst &M = A.M;
   n.centroid = NODES == 1 ? true : (NODES == 2 ? false : i < M.Nc);
-  const double el = (M.elastic == 1) ? 1.0 : 0.0;
   double mu, exxd, ezzd, exz;
   if (pk) {
     double *x[3];
@@ -162,9 +161,9 @@ __device__ __forceinline__ void node_prepare(const SweepArgs &A, long long i, No
   }
   n.in.G = mu;
   n.eta_e = (M.elastic == 1) ? M.dt_model * mu : 1.0;
-  n.inv_eta_e = ANISO ? 1.0 / n.eta_e : 0.0;
+  n.inv_eta_e = ANISO ? FxMath::recip(n.eta_e) : 0.0;
   if (!ANISO) {
-    const double h = el * 0.5 / n.eta_e;  // el / eta_e / 2
+    const double h = (M.elastic == 1) ? 0.5 * FxMath::recip(n.eta_e) : 0.0;  // el / eta_e / 2
     n.in.Exx = exxd + n.in.Txx0 * h;
     n.in.Ezz = ezzd + n.in.Tzz0 * h;
     n.in.Exz = exz + n.in.Txz0 * h;
@@ -173,15 +172,15 @@ __device__ __forceinline__ void node_prepare(const SweepArgs &A, long long i, No
     double sn, cs;
     sincos(angle - M_PI / 2.0, &sn, &cs);
     n.in.lxlz = cs * sn; n.in.lx2 = cs * cs; n.in.ani_fac = n.anif;
-    effective_strain_rate(n.in.Exx, n.in.Ezz, n.in.Exz, exxd, ezzd, exz, n.in.Txx0, n.in.Tzz0, n.in.Txz0, n.d1,
+    effective_strain_rate<FxMath>(n.in.Exx, n.in.Ezz, n.in.Exz, exxd, ezzd, exz, n.in.Txx0, n.in.Tzz0, n.in.Txz0, n.d1,
                           n.d2, 1.0 - 1.0 / n.anif, n.eta_e, M.elastic);
   }
   n.in.centroid = n.centroid ? 1 : 0;
   n.in.final_update = A.final_update;
   n.in.post_process = n.centroid ? 1 : 2;  // a vertex keeps only etaVE, eta_phys and X
   n.in.want_rho = n.centroid && (M.density_variations == 1);
-  if (ANISO) node_setup_aniso(M, n.in, A.need_lnd, n.ctx, n.an);
-  else node_setup_iso(M, n.in, A.need_lnd, n.ctx);
+  if (ANISO) node_setup_aniso<FxMath>(M, n.in, A.need_lnd, n.ctx, n.an);
+  else node_setup_iso<FxMath>(M, n.in, A.need_lnd, n.ctx);
 }
 
 __device__ __forceinline__ double node_perc(const SweepArgs &A, const Node &n, int p) {
@@ -235,7 +234,7 @@ __device__ __forceinline__ void node_store(const SweepArgs &A, const Node &n, do
   const int avg = M.eta_average;
   if (n.solid) {
     if (n.centroid) {
-      out[CO_d] = 1.0 / out[CO_d];
+      out[CO_d] = FxMath::recip(out[CO_d]);
       if (!ANISO && !fp64_finite(out[CO_d])) set_status(status, MDZ_EEMPTY_CELL);
     }
     if (avg == 1) {
@@ -313,8 +312,8 @@ __device__ __forceinline__ void sweep_node(const SweepArgs &A, long long i, Acc 
         continue;
       }
       PointOut o;
-      if (ANISO) point_aniso(A.M, A.ph[p], n.in, n.ctx, n.an, A.polish, o);
-      else point_iso(A.M, A.ph[p], n.in, n.ctx, A.polish, o);
+      if (ANISO) point_aniso<FxMath>(A.M, A.ph[p], n.in, n.ctx, n.an, A.polish, o);
+      else point_iso<FxMath>(A.M, A.ph[p], n.in, n.ctx, A.polish, o);
       node_accumulate<ANISO>(A, n, p, perc, o, out, acc, status);
     }
   }
@@ -405,7 +404,7 @@ __device__ __forceinline__ void compact_node(const SweepArgs &A, bool valid, lon
 #pragma unroll
       for (int k = 0; k < kMlpIn; k++) f[k] = 0.0f;
       if (active) {
-        iso_setup(A.M, A.ph[p], n.in, n.ctx, st, o, polish == 0);
+        iso_setup<FxMath>(A.M, A.ph[p], n.in, n.ctx, st, o, polish == 0);
         warm_features(A.M, n.in, n.ctx, st, false, f);
       }
       warm_inputs(*W, f, kFeatIso, x);
@@ -413,16 +412,16 @@ __device__ __forceinline__ void compact_node(const SweepArgs &A, bool valid, lon
       const float y = mlp_warp_predict(*S, x);
       s_start = warm_start_point(y, W->z_scale, W->z_shift);
     } else if (active) {
-      iso_setup(A.M, A.ph[p], n.in, n.ctx, st, o, polish == 0);
+      iso_setup<FxMath>(A.M, A.ph[p], n.in, n.ctx, st, o, polish == 0);
     }
     bool yields = false;
     if (active) {
-      iso_ve(A.M, A.ph[p], n.in, n.ctx, st, s_start, polish, o, m);
+      iso_ve<FxMath>(A.M, A.ph[p], n.in, n.ctx, st, s_start, polish, o, m);
       yields = iso_yields_dp(A.M, A.ph[p], n.ctx, m);
     }
     dp_compact(A.M, A.ph[p], Q, par, yields, m, n.in, n.ctx);
     if (active) {
-      iso_post(A.M, A.ph[p], n.in, n.ctx, st, o, m);
+      iso_post<FxMath>(A.M, A.ph[p], n.in, n.ctx, st, o, m);
       node_accumulate<false>(A, n, p, perc, o, out, acc, status);
     }
   }
@@ -486,8 +485,8 @@ __device__ __forceinline__ void warm_node(const SweepArgs &A, MlpWarpShared &S, 
 #pragma unroll
     for (int k = 0; k < kMlpIn; k++) f[k] = 0.0f;
     if (active) {
-      if (ANISO) aniso_setup(A.M, A.ph[p], n.in, n.ctx, n.an, st, o, W.polish_iters == 0);
-      else iso_setup(A.M, A.ph[p], n.in, n.ctx, st, o, W.polish_iters == 0);
+      if (ANISO) aniso_setup<FxMath>(A.M, A.ph[p], n.in, n.ctx, n.an, st, o, W.polish_iters == 0);
+      else iso_setup<FxMath>(A.M, A.ph[p], n.in, n.ctx, st, o, W.polish_iters == 0);
       warm_features(A.M, n.in, n.ctx, st, ANISO, f);
     }
     warm_inputs(W, f, nfeat, x);
@@ -495,8 +494,8 @@ __device__ __forceinline__ void warm_node(const SweepArgs &A, MlpWarpShared &S, 
     const float y = mlp_warp_predict(S, x);
     if (!active) continue;
     const float s_start = warm_start_point(y, W.z_scale, W.z_shift);
-    if (ANISO) aniso_finish(A.M, A.ph[p], n.in, n.ctx, n.an, st, s_start, W.polish_iters, o);
-    else iso_finish(A.M, A.ph[p], n.in, n.ctx, st, s_start, W.polish_iters, o);
+    if (ANISO) aniso_finish<FxMath>(A.M, A.ph[p], n.in, n.ctx, n.an, st, s_start, W.polish_iters, o);
+    else iso_finish<FxMath>(A.M, A.ph[p], n.in, n.ctx, st, s_start, W.polish_iters, o);
     node_accumulate<ANISO>(A, n, p, perc, o, out, acc, status);
   }
   if (valid) node_store<ANISO>(A, n, out, status);
@@ -635,8 +634,8 @@ __global__ void __launch_bounds__(128, 2) k_sweep_tiles(const __grid_constant__ 
       float s_start = ANISO ? 0.0f : 1.0f;  // the reference's own start
       if (active) {
         const bool exact = (MODE == MODE_COLLECT) || W.mlp.polish_iters == 0;  // the pairs' targets need eta_up
-        if (ANISO) aniso_setup(A.M, A.ph[p], n.in, n.ctx, n.an, st, o, exact);
-        else iso_setup(A.M, A.ph[p], n.in, n.ctx, st, o, exact);
+        if (ANISO) aniso_setup<FxMath>(A.M, A.ph[p], n.in, n.ctx, n.an, st, o, exact);
+        else iso_setup<FxMath>(A.M, A.ph[p], n.in, n.ctx, st, o, exact);
         warm_features(A.M, n.in, n.ctx, st, ANISO, f);
       }
       if (MODE == MODE_WARM) {
@@ -652,8 +651,8 @@ __global__ void __launch_bounds__(128, 2) k_sweep_tiles(const __grid_constant__ 
       if (!active) continue;
       double eta_conv = 0.0;
       const int polish = (MODE == MODE_WARM) ? W.mlp.polish_iters : 0;
-      if (ANISO) aniso_finish(A.M, A.ph[p], n.in, n.ctx, n.an, st, s_start, polish, o, &eta_conv);
-      else iso_finish(A.M, A.ph[p], n.in, n.ctx, st, s_start, polish, o, &eta_conv);
+      if (ANISO) aniso_finish<FxMath>(A.M, A.ph[p], n.in, n.ctx, n.an, st, s_start, polish, o, &eta_conv);
+      else iso_finish<FxMath>(A.M, A.ph[p], n.in, n.ctx, st, s_start, polish, o, &eta_conv);
       node_accumulate<ANISO>(A, n, p, perc, o, out, acc, status);
       if (MODE == MODE_COLLECT) {
         const long long item = (long long)p * total + i;
@@ -705,11 +704,11 @@ __global__ void __launch_bounds__(128) k_points(const __grid_constant__ PointArg
     if (A.aniso) {
       in.lxlz = I.lxlz[i]; in.lx2 = I.lx2[i]; in.ani_fac = I.ani_fac[i];
       AnisoNode an;
-      node_setup_aniso(A.M, in, true, ctx, an);
-      point_aniso(A.M, A.ph[p], in, ctx, an, A.polish, o);
+      node_setup_aniso<FxMath>(A.M, in, true, ctx, an);
+      point_aniso<FxMath>(A.M, A.ph[p], in, ctx, an, A.polish, o);
     } else {
-      node_setup_iso(A.M, in, true, ctx);
-      point_iso(A.M, A.ph[p], in, ctx, A.polish, o);
+      node_setup_iso<FxMath>(A.M, in, true, ctx);
+      point_iso<FxMath>(A.M, A.ph[p], in, ctx, A.polish, o);
     }
     const mdz_point_outputs &O = A.out;
     double *dst[24] = {O.eta, O.Txx, O.Tzz, O.Txz, O.etaVE, O.VEcoeff, O.Eii_el, O.Eii_pl, O.Eii_pwl, O.Eii_exp,

@@ -407,6 +407,7 @@ def load_library(path: str = LIB_PATH):
     lib.mdz_rheo_ceil_selftest.argtypes = [C.c_int, C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p]
     lib.mdz_rheo_dd_selftest.argtypes = [C.c_int, C.c_void_p, C.c_int64, C.c_void_p]
     lib.mdz_rheo_quotient_selftest.argtypes = [C.c_int, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p]
+    lib.mdz_rheo_fx_selftest.argtypes = [C.c_int, C.c_void_p, C.c_int64, C.c_void_p]
     lib.mdz_rheo_points_static.argtypes = [C.POINTER(Model), C.POINTER(Materials), C.POINTER(PointInputs),
                                            C.POINTER(PointOutputs), C.c_int64, C.c_int, C.c_int, C.c_void_p,
                                            C.POINTER(SweepStats)]
@@ -517,6 +518,16 @@ def quotient_selftest(r: np.ndarray, den: np.ndarray, device: int = 0):
     if rc != MDZ_OK:
         raise RheoError(rc, "mdz_rheo_quotient_selftest")
     return out
+
+
+def fx_selftest(x: np.ndarray, device: int = 0):
+    """(exp, log, 1/x, sqrt, sin, cos) of the float64 array x by the fixed-point functions on the GPU."""
+    x = np.ascontiguousarray(x, np.float64)
+    out = np.empty((6, x.size), np.float64)
+    rc = load_library().mdz_rheo_fx_selftest(device, x.ctypes.data, x.size, out.ctypes.data)
+    if rc != MDZ_OK:
+        raise RheoError(rc, "mdz_rheo_fx_selftest")
+    return tuple(out)
 
 
 def ceil_selftest(q: np.ndarray, device: int = 0):
