@@ -143,11 +143,12 @@ FX_FN double fx_normalise(uint64_t V, int e) {
 }
 
 // ---- exp -----------------------------------------------------------------------------------
-// x as Q9.54 (towards zero), for |x| < 512; bits b of x
-FX_FN int64_t fx_q54(uint64_t b) {
+// x in fixed point with F fraction bits, rounded to nearest, for |x| < 2^(63 - F); bits b of x
+template <int F>
+FX_FN int64_t fx_fixed(uint64_t b) {
   const int E = (int)(fx_hi(b) >> 20) & 0x7ff;
-  const int sh = 1031 - E;  // >= 0 for |x| < 512
-  const uint64_t m = (fx_significand(b) << 10) >> (sh > 63 ? 63 : sh);
+  const int sh = 1085 - F - E > 63 ? 63 : 1085 - F - E;
+  const uint64_t m = ((fx_significand(b) << 10) + ((1ull << sh) >> 1)) >> sh;
   return (int64_t)b < 0 ? -(int64_t)m : (int64_t)m;
 }
 
@@ -181,7 +182,7 @@ FX_FN double fx_exp(double x) {
   const uint64_t b = fx_bits(x);
   if ((fx_hi(b) & 0x7fffffffu) >= 0x407f4000u) return exp(x);
   int m;
-  const uint64_t M = fx_exp_core(fx_q54(b), m);
+  const uint64_t M = fx_exp_core(fx_fixed<54>(b), m);
   return fx_exp_double(M, m);
 }
 

@@ -36,6 +36,7 @@
 #include "fp64_div.cuh"
 #include "fp64_math.cuh"
 #include "fx64.cuh"
+#include "ve_fx.cuh"
 
 namespace mdz {
 
@@ -47,6 +48,7 @@ namespace mdz {
 // step of 1e-7 magnifies a change of the last bit of its solves to 1e-9 and more of the
 // derivative, so the operators keep the bits of these forms.
 struct FxMath {
+  static constexpr bool kFixed = true;  // local solves in fixed point where the start asks for it (ve_solve_fx)
   static __device__ __forceinline__ double exp(double x) { return fx_exp(x); }
   static __device__ __forceinline__ double log(double x) { return fx_log(x); }
   static __device__ __forceinline__ double recip(double x) { return fx_recip(x); }
@@ -57,6 +59,7 @@ struct FxMath {
   static __device__ __forceinline__ void sincos(double x, double *s, double *c) { fx_sincos(x, s, c); }
 };
 struct FdMath {
+  static constexpr bool kFixed = false;
   static __device__ __forceinline__ double exp(double x) { return fast_exp(x); }
   static __device__ __forceinline__ double log(double x) { return fast_log(x); }
   static __device__ __forceinline__ double recip(double x) { return mdz::quotient(1.0, x); }
@@ -293,6 +296,22 @@ __device__ __forceinline__ void creep_laws(const ModelConst &M, const PhaseConst
 // the softest non-linear law p and nc_k = n_k ln(eta_p / eta_k) <= 0.  Every quantity
 // in the exponent is O(1) for the terms that carry strain rate, so nothing large cancels.
 // ---------------------------------------------------------------------------------------
+// Inputs of the general (FP64) form of the local solve: any start, any normalisation.
+struct VeArgs {
+  Laws L;
+  double Eii, inv2Eii, inv_eta_el, eta_cst, eta_n, ln_eta_n;
+  double min_eta, max_eta, eta_el;  // the anisotropic bracket
+  float s_start, s_up;
+  int elastic, polish;
+};
+
+__device__ __forceinline__ void ve_args(VeArgs &v, const Laws &L, const NodeCtx &c, double eta_cst, double eta_n,
+                                        double ln_eta_n, float s_start, float s_up, int polish) {
+  v.L = L;
+  v.Eii = c.Eii; v.inv2Eii = c.inv2Eii; v.inv_eta_el = c.inv_eta_el; v.elastic = c.elastic;
+  v.eta_cst = eta_cst; v.eta_n = eta_n; v.ln_eta_n = ln_eta_n; v.s_start = s_start; v.s_up = s_up; v.polish = polish;
+}
+
 struct VeCoef {
   double Eii, thr_conv, thr_fail;  // Eii * tol/100, Eii * tol
   double inv_Eii;                  // 1 / Eii
@@ -313,17 +332,17 @@ struct VeState {
 };
 
 template <class FP>
-__device__ __forceinline__ void ve_coef(const Laws &L, const NodeCtx &c, double eta_cst, double eta_up,
-                                        double ln_eta_up, VeCoef &q) {
-  const double Eii = c.Eii;
+__device__ __forceinline__ void ve_coef(const VeArgs &v, VeCoef &q) {
+  const Laws &L = v.L;
+  const double Eii = v.Eii, eta_cst = v.eta_cst, eta_up = v.eta_n, ln_eta_up = v.ln_eta_n;
   const double tol = 1.0e-11;  // hard-coded in LocalIterationViscoElastic (:154)
   q.Eii = Eii;
-  q.inv_Eii = 2.0 * c.inv2Eii;
+  q.inv_Eii = 2.0 * v.inv2Eii;
   q.thr_conv = Eii * (tol / 100);
   q.thr_fail = Eii * tol;
   q.eta_up = eta_up;
   q.a_cst = (L.mech & F_CST) ? Eii / eta_cst : 0.0;
-  double A = (c.elastic ? Eii * c.inv_eta_el : 0.0) + q.a_cst;
+  double A = (v.elastic ? Eii * v.inv_eta_el : 0.0) + q.a_cst;
   q.a_lin1 = q.a_pwl1 = 0.0;
   q.nl = 0;
   double ln_inv_p = -kInf;
@@ -464,26 +483,21 @@ __device__ __forceinline__ void start_coef(const VeCoef &q, StartCoef &sc) {
   for (int k = 0; k < K_COUNT; k++) sc.c[k] = (q.nl >> k & 1) ? fma(q.n[k], q.lp, q.nc[k]) : 0.0;
 }
 
-// s_hi: the upper bound the iteration falls back to
-__device__ __forceinline__ float ve_polish_f32(const VeCoef &q, const StartCoef &sc, float s0, int iters,
-                                               int &taken, float s_hi) {
+// The FP32 Newton steps on plain coefficients; s_hi: the upper bound the iteration falls
+// back to.  settle: up to this many more steps (not counted in `taken`) while the last one
+// moved the steepest law's argument by more than 5e-3 (nmax its exponent): after a Newton
+// step the argument is off by about half the square of its move.
+__device__ __forceinline__ float ve_polish_f32(int nl, float a, const float *n, const float *c, float s0, int iters,
+                                               int &taken, float s_hi, int settle = 0, float nmax = 0.0f) {
   taken = 0;
-  if (iters <= 0) return s0;
-  const float a = f32_trunc(sc.a);
-  float c[K_COUNT] = {0.f, 0.f, 0.f}, n[K_COUNT] = {0.f, 0.f, 0.f};
-  if (q.nl) {
-#pragma unroll
-    for (int k = 0; k < K_COUNT; k++)
-      if (q.nl >> k & 1) { n[k] = f32_trunc(q.n[k]); c[k] = f32_trunc(sc.c[k]); }
-  }
   float s = s0;
-  for (int it = 0; it < iters; it++) {
+  for (int it = 0; it < iters + settle; it++) {
     float e = 0.f, S = 0.f;
-    if (q.nl) {
+    if (nl) {
       const float ls = __logf(s);
 #pragma unroll
       for (int k = 0; k < K_COUNT; k++)
-        if (q.nl >> k & 1) {
+        if (nl >> k & 1) {
           const float ek = __expf(fmaf(n[k], ls, c[k]));
           e += ek;
           S = fmaf(n[k], ek, S);
@@ -492,11 +506,24 @@ __device__ __forceinline__ float ve_polish_f32(const VeCoef &q, const StartCoef 
     const float r = 1.0f - a * s - e;
     if (fabsf(r) < 1e-6f) break;
     const float sn = s + r * s / fmaf(a, s, S);
-    taken = it + 1;
+    if (it < iters) taken = it + 1;
     if (!(sn > 0.0f && sn <= 2.0f)) return s_hi;  // the upper bound eta_up: right of the root
+    const float move = fabsf(sn - s) * nmax;
     s = sn;
+    if (it >= iters - 1 && move < 5e-3f * sn) break;
   }
   return s;
+}
+
+__device__ __forceinline__ float ve_polish_f32(const VeCoef &q, const StartCoef &sc, float s0, int iters,
+                                               int &taken, float s_hi) {
+  float c[K_COUNT] = {0.f, 0.f, 0.f}, n[K_COUNT] = {0.f, 0.f, 0.f};
+  if (iters > 0 && q.nl) {
+#pragma unroll
+    for (int k = 0; k < K_COUNT; k++)
+      if (q.nl >> k & 1) { n[k] = f32_trunc(q.n[k]); c[k] = f32_trunc(sc.c[k]); }
+  }
+  return ve_polish_f32(q.nl, f32_trunc(sc.a), n, c, s0, iters, taken, s_hi);
 }
 
 // Stage 2 from the FP32 point s (see above).  Where s is not a positive normal number in
@@ -554,6 +581,102 @@ __device__ __forceinline__ double ve_start(const VeCoef &q, float s0, int fp32, 
 // start.
 __device__ __forceinline__ int start_fp32(int polish) { return polish & 0xff; }
 __device__ __forceinline__ bool start_dd(int polish) { return (polish & MDZ_START_DD) != 0; }
+
+// The local solve in fixed point (ve_fx.cuh) from the FP32 Newton steps: the coefficients of
+// the normalised residual, the FP32 steps, the fixed-point root, and the FP64 outputs at it.
+// eta_n must be a power of two.  false where the fixed-point form declines: the caller runs
+// the FP64 iteration.  Counts as one evaluation.
+template <class FP>
+__device__ __forceinline__ bool ve_solve_fx(const Laws &L, const NodeCtx &c, double eta_cst, double eta_n,
+                                            double ln_eta_n, float s_start, float s_hi, int fp32, int &f32_steps,
+                                            VeState &s) {
+  double A = c.elastic ? c.inv_eta_el : 0.0, inv_cst = 0.0, inv[K_COUNT] = {0.0, 0.0, 0.0}, a[K_COUNT];
+  float nf[K_COUNT] = {0.f, 0.f, 0.f}, cf[K_COUNT] = {0.f, 0.f, 0.f};
+  if (L.mech & F_CST) { inv_cst = FP::recip(eta_cst); A += inv_cst; }
+  int nl = 0, tiny = 0;  // tiny: laws below e^-150, left out of the residual
+  float nmax = 0.0f;
+#pragma unroll
+  for (int k = 0; k < K_COUNT; k++) {
+    const int bit = (k == K_PWL) ? F_PWL : ((k == K_EXP) ? F_EXPV : F_LIN);
+    a[k] = 0.0;
+    if (!(L.mech & bit)) continue;
+    if (k != K_EXP && fp64_eq_nonzero(L.n[k], 1.0)) {  // Newtonian law: Eii eta / eta_k
+      inv[k] = law_inv<FP>(L, k);
+      A += inv[k];
+    } else {
+      a[k] = L.n[k] * (ln_eta_n + L.ln_inv[k]);
+      if (fp64_lt(a[k], -150.0)) {
+        tiny |= 1 << k;
+      } else {
+        nl |= 1 << k;
+        nf[k] = f32_trunc(L.n[k]);
+        cf[k] = f32_trunc(a[k]);
+        nmax = fmaxf(nmax, nf[k]);
+      }
+    }
+  }
+  const double lin = A * eta_n;
+  const float s0 = ve_polish_f32(nl, f32_trunc(lin), nf, cf, s_start, fp32, f32_steps, s_hi, 3, nmax);
+  VeFxRoot r;
+  if (!ve_root_fx(nl, lin, L.n, a, nf, s0, r)) return false;
+  const int k2 = (int)(fp64_exponent(eta_n)) - 1023;
+  s.eta = fx_normalise(r.S, k2 - 62);
+  const double E_eta = s.eta * c.Eii;
+  s.Tii = 2.0 * E_eta;
+  s.e_cst = E_eta * inv_cst;
+#pragma unroll
+  for (int k = 0; k < K_COUNT; k++)
+    s.e[k] = (nl >> k & 1) ? c.Eii * fx_normalise(r.M[k], r.m[k] - 62) : E_eta * inv[k];
+  if (tiny) {
+    const double ln_s = FP::log(fx_normalise(r.S, -62));
+#pragma unroll
+    for (int k = 0; k < K_COUNT; k++)
+      if (tiny >> k & 1) s.e[k] = c.Eii * FP::exp(fma(L.n[k], ln_s, a[k]));
+  }
+  s.e_pwl = s.e[K_PWL]; s.e_exp = s.e[K_EXP]; s.e_lin = s.e[K_LIN];
+  s.iters = 1;
+  return true;
+}
+
+// LocalIterationViscoElastic from the start that `polish` names
+template <class FP>
+__device__ __forceinline__ void ve_general_inl(const VeArgs &v, VeState &s, int &f32_steps) {
+  VeCoef q;
+  ve_coef<FP>(v, q);
+  ve_newton<FP>(q, ve_start(q, v.s_start * v.s_up, start_fp32(v.polish), start_dd(v.polish), f32_steps, v.s_up), s,
+                v.s_up, v.polish != 0);
+}
+
+// The local solve in place.  Sweeps take the fixed-point form where the start allows it and
+// keep the general one out of line, where its registers do not weigh on them.
+struct VeOut {
+  VeState s;
+  int f32_steps;
+};
+static __device__ __noinline__ VeOut ve_general_fx(VeArgs v) {
+  VeOut o;
+  o.s.status = MDZ_OK;
+  ve_general_inl<FxMath>(v, o.s, o.f32_steps);
+  return o;
+}
+
+template <class FP>
+__device__ __forceinline__ void ve_solve(const Laws &L, const NodeCtx &c, double eta_cst, const double eta_n,
+                                         double ln_eta_n, bool pow2, float s_start, float s_up, int polish, VeState &s,
+                                         int &f32_steps) {
+  if (FP::kFixed && pow2 && start_dd(polish) && start_fp32(polish) > 0 &&
+      ve_solve_fx<FP>(L, c, eta_cst, eta_n, ln_eta_n, s_start * s_up, s_up, start_fp32(polish), f32_steps, s))
+    return;
+  VeArgs v;
+  ve_args(v, L, c, eta_cst, eta_n, ln_eta_n, s_start, s_up, polish);
+  if (FP::kFixed) {
+    const VeOut o = ve_general_fx(v);
+    s = o.s;
+    f32_steps = o.f32_steps;
+  } else {
+    ve_general_inl<FP>(v, s, f32_steps);
+  }
+}
 
 struct GseIn {
   double Eii, eta_el, eta_cst, C_pwl, n_pwl, C_lin, n_lin, m_lin, C_exp, ST, n_exp, eta_up, eta_lo, Ag,
@@ -722,6 +845,7 @@ struct IsoState {
   // start point eta_up in that unknown (1 when exact)
   double eta_n, ln_eta_n;
   float s_up;
+  bool pow2;  // eta_n is a power of two
 };
 
 // Start point of the local solve (RheologyDensity.c:582-592, AnisotropyRoutines.c:409-415):
@@ -770,6 +894,7 @@ __device__ __forceinline__ void start_point(const ModelConst &M, double ln_inv_m
       const double kd = __hiloint2double(0x43300000, k ^ (int)0x80000000) - 4503601774854144.0;  // (double)k
       S.ln_eta_n = fma(kd, MDZ_LN2_HI, kd * MDZ_LN2_LO);
       S.s_up = __expf(fmaf((float)-k, 0.693147182f, lf));
+      S.pow2 = true;
       return;
     }
   }
@@ -777,6 +902,7 @@ __device__ __forceinline__ void start_point(const ModelConst &M, double ln_inv_m
   S.eta_n = S.eta_up;
   S.ln_eta_n = S.ln_eta_up;
   S.s_up = 1.0f;
+  S.pow2 = false;
 }
 
 // Lower end of the reference's bracket: the largest of the lower bound, eta_cst, eta_el and
@@ -960,12 +1086,9 @@ __device__ inline void iso_ve(const ModelConst &M, const PhaseConst &ph, const N
   const double Tyield = S.Tyield;
   double eta_ve, Tii, e_cst, e_pwl, e_exp, e_lin;
   if (!gs) {  // LocalIterationViscoElastic (:646)
-    VeCoef q;
-    ve_coef<FP>(L, c, eta_cst, S.eta_n, S.ln_eta_n, q);
     VeState s;
     s.status = MDZ_OK;
-    ve_newton<FP>(q, ve_start(q, s_start * S.s_up, start_fp32(polish), start_dd(polish), o.f32_steps, S.s_up), s,
-              S.s_up, polish != 0);
+    ve_solve<FP>(L, c, eta_cst, S.eta_n, S.ln_eta_n, S.pow2, s_start, S.s_up, polish, s, o.f32_steps);
     set_status(o.status, s.status);
     eta_ve = s.eta; Tii = s.Tii; e_cst = s.e_cst; e_pwl = s.e_pwl; e_exp = s.e_exp; e_lin = s.e_lin;
     o.iters = s.iters;
@@ -1250,6 +1373,68 @@ __device__ inline void aniso_setup(const ModelConst &M, const PhaseConst &ph, co
   (void)an; (void)T; (void)K; (void)dt; (void)min_eta; (void)max_eta; (void)dislocation; (void)eta_el;
 }
 
+// The general form of the anisotropic local solve (AnisotropyRoutines.c:474-585): 10
+// log-space bisection steps on [min_eta 1e-3, 10 max(eta_lo, max_eta)] where the start is the
+// reference's, then Newton.
+template <class FP>
+__device__ __forceinline__ void aniso_general_inl(const ModelConst &M, const VeArgs &v, VeState &s, int &f32_steps) {
+  const double tol = 1e-11, Eii = v.Eii, min_eta = v.min_eta, max_eta = v.max_eta;
+  const int polish = v.polish;
+  const float s_start = v.s_start;
+  VeCoef q;
+  ve_coef<FP>(v, q);
+  double r, sv;  // sv = eta_ve / eta_n (eta_n = eta_up from the bisection: that start is exact)
+  f32_steps = 0;
+  if (s_start > 0.0f || polish > 0) {
+    sv = ve_start(q, ((s_start > 0.0f) ? s_start : 1.0f) * v.s_up, start_fp32(polish), start_dd(polish), f32_steps,
+                  v.s_up);
+  } else {
+    const double inv_up = 1.0 / v.eta_n;
+    const double eta_lo = lower_viscosity<FP>(M, v.L, (v.L.mech & F_CST) != 0, v.eta_cst, v.elastic != 0, v.eta_el, false);
+    double lo = min_eta * 1.0e-3, hi = 10.0 * fmax(eta_lo, max_eta);
+    for (int bit = 0; bit < 10; bit++) {
+      const double eta = sqrt(lo * hi);
+      ve_eval<FP>(q, eta * inv_up, s, r);
+      if (r > 0.0) lo = eta;
+      else hi = eta;
+      if (fabs(r) < q.thr_conv) break;
+    }
+    sv = sqrt(lo * hi) * inv_up;
+  }
+  // a moved start (not the bisection's) that has not converged within the cap is
+  // abandoned for the upper bound eta_up, above the root, with a fresh cap
+  bool moved = s_start > 0.0f || polish > 0;
+  s.iters = 0;
+  double step = -1.0;  // binomial update of the previous point's terms (see ve_eval)
+  for (int it = 0; it < 50; it++) {
+    ve_eval<FP>(q, sv, s, r, step);
+    s.iters++;
+    if (fp64_is_nan(r)) { set_status(s.status, MDZ_EANISO_NAN); break; }
+    const double d = FP::newton_quotient(r, fma(q.Aup, sv, ve_S(q, s)));
+    sv = fma(sv, d, sv);
+    step = fp64_lt(fabs(d) * q.nmax, 1e-5) ? d : -1.0;
+    if (fp64_le(sv, 0.0)) { sv = min_eta / q.eta_up; step = -1.0; }
+    const double ar = fabs(r);
+    if (fp64_abs_lt(r, q.thr_conv)) break;
+    if (it == 49 && moved && !(ar < 10.0 * tol * Eii)) {
+      moved = false;
+      sv = f64_of_f32(v.s_up);
+      step = -1.0;
+      it = -1;
+      continue;
+    }
+    if (it == 49 && ar < 10.0 * tol * Eii) break;
+    if (it == 49 && ar > q.thr_fail) { set_status(s.status, MDZ_EANISO_ITER); break; }
+  }
+  s.eta = sv * q.eta_up;
+}
+static __device__ __noinline__ VeOut aniso_general_fx(const ModelConst &M, VeArgs v) {
+  VeOut o;
+  o.s.status = MDZ_OK;
+  aniso_general_inl<FxMath>(M, v, o.s, o.f32_steps);
+  return o;
+}
+
 // Local solve, plasticity, post-processing.  The Newton starts from the reference's
 // bisection when s_start <= 0 and polish == 0; otherwise from s_start * eta_up (eta_up
 // when s_start <= 0) moved by the start stages that the descriptor `polish` names.
@@ -1283,55 +1468,26 @@ __device__ inline void aniso_finish(const ModelConst &M, const PhaseConst &ph, c
     set_status(o.status, st);
     o.d1 = dd;
     o.inv_d1 = 1.0 / dd;
-  } else {  // :474-585: 10 log-space bisection steps on [min_eta 1e-3, 10 max(eta_lo, max_eta)], then Newton
-    const double tol = 1e-11;
-    VeCoef q;
-    ve_coef<FP>(L, c, eta_cst, S.eta_n, S.ln_eta_n, q);
+  } else {  // :474-585
     VeState s;
     s.status = MDZ_OK;
-    double r, sv;  // sv = eta_ve / eta_n (eta_n = eta_up from the bisection: that start is exact)
-    if (s_start > 0.0f || polish > 0) {
-      sv = ve_start(q, ((s_start > 0.0f) ? s_start : 1.0f) * S.s_up, start_fp32(polish), start_dd(polish),
-                    o.f32_steps, S.s_up);
-    } else {
-      const double inv_up = 1.0 / eta_up;
-      const double eta_lo = lower_viscosity<FP>(M, L, constant, eta_cst, elastic != 0, eta_el, false);
-      double lo = min_eta * 1.0e-3, hi = 10.0 * fmax(eta_lo, max_eta);
-      for (int bit = 0; bit < 10; bit++) {
-        eta_ve = sqrt(lo * hi);
-        ve_eval<FP>(q, eta_ve * inv_up, s, r);
-        if (r > 0.0) lo = eta_ve;
-        else hi = eta_ve;
-        if (fabs(r) < q.thr_conv) break;
+    if (!(FP::kFixed && S.pow2 && start_dd(polish) && start_fp32(polish) > 0 &&
+          ve_solve_fx<FP>(L, c, eta_cst, S.eta_n, S.ln_eta_n, ((s_start > 0.0f) ? s_start : 1.0f) * S.s_up, S.s_up,
+                          start_fp32(polish), o.f32_steps, s))) {
+      VeArgs v;
+      ve_args(v, L, c, eta_cst, S.eta_n, S.ln_eta_n, s_start, S.s_up, polish);
+      v.min_eta = min_eta; v.max_eta = max_eta; v.eta_el = eta_el;
+      if (FP::kFixed) {
+        const VeOut g = aniso_general_fx(M, v);
+        s = g.s;
+        o.f32_steps = g.f32_steps;
+      } else {
+        aniso_general_inl<FP>(M, v, s, o.f32_steps);
       }
-      sv = sqrt(lo * hi) * inv_up;
     }
-    // a moved start (not the bisection's) that has not converged within the cap is
-    // abandoned for the upper bound eta_up, above the root, with a fresh cap
-    bool moved = s_start > 0.0f || polish > 0;
-    o.iters = 0;
-    double step = -1.0;  // binomial update of the previous point's terms (see ve_eval)
-    for (int it = 0; it < 50; it++) {
-      ve_eval<FP>(q, sv, s, r, step);
-      o.iters++;
-      if (fp64_is_nan(r)) { set_status(o.status, MDZ_EANISO_NAN); break; }
-      const double d = FP::newton_quotient(r, fma(q.Aup, sv, ve_S(q, s)));
-      sv = fma(sv, d, sv);
-      step = fp64_lt(fabs(d) * q.nmax, 1e-5) ? d : -1.0;
-      if (fp64_le(sv, 0.0)) { sv = min_eta / q.eta_up; step = -1.0; }
-      const double ar = fabs(r);
-      if (fp64_abs_lt(r, q.thr_conv)) break;
-      if (it == 49 && moved && !(ar < 10.0 * tol * Eii)) {
-        moved = false;
-        sv = f64_of_f32(S.s_up);
-        step = -1.0;
-        it = -1;
-        continue;
-      }
-      if (it == 49 && ar < 10.0 * tol * Eii) break;
-      if (it == 49 && ar > q.thr_fail) { set_status(o.status, MDZ_EANISO_ITER); break; }
-    }
-    eta_ve = sv * q.eta_up;
+    set_status(o.status, s.status);
+    eta_ve = s.eta;
+    o.iters = s.iters;
     Tii = s.Tii; e_cst = s.e_cst; e_pwl = s.e_pwl; e_exp = s.e_exp; e_lin = s.e_lin;
   }
   if (fp64_lt(eta_ve, min_eta)) eta_ve = min_eta;  // :589-603
