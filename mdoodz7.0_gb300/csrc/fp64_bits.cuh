@@ -107,6 +107,21 @@ __device__ __forceinline__ bool fp64_abs_gt(double x, double t) {
   return fp64_key_of_bits(ax) > fp64_key_of_bits(bt);
 }
 
+// The same comparisons against a bound that is positive (not NaN): the bits order as signed
+// integers there, so four to five instructions in place of twenty.
+__device__ __forceinline__ bool fp64_lt_pos(double x, double b) {
+  const unsigned long long bx = fp64_bits(x);
+  return (long long)bx < (long long)fp64_bits(b) && bx <= 0xfff0000000000000ull;  // the second: not a negative NaN
+}
+__device__ __forceinline__ bool fp64_gt_pos(double x, double b) {
+  const long long bx = (long long)fp64_bits(x);
+  return bx > (long long)fp64_bits(b) && bx <= (long long)kFp64InfBits;
+}
+__device__ __forceinline__ bool fp64_abs_gt_pos(double x, double b) {
+  const unsigned long long ax = fp64_bits(x) & kFp64AbsMask;
+  return ax > fp64_bits(b) && ax <= kFp64InfBits;
+}
+
 // x == y as IEEE numbers, for a y that is neither NaN nor zero (bit equality then)
 __device__ __forceinline__ bool fp64_eq_nonzero(double x, double y) { return fp64_bits(x) == fp64_bits(y); }
 
@@ -118,6 +133,17 @@ __device__ __forceinline__ double fp64_fmax(double a, double b) {
   if ((bb & kFp64AbsMask) > kFp64InfBits) return a;
   const unsigned long long ka = fp64_key_of_bits(ba), kb = fp64_key_of_bits(bb);
   return (ka > kb || (ka == kb && (ba >> 63) == 0ull)) ? a : b;
+}
+
+// x 2^k by the exponent field where x and the result are normal numbers; by a product of
+// powers of two elsewhere (zero, subnormal, Inf, NaN, overflow), out of line
+static __device__ __noinline__ double fp64_scale_rare(double x, int k) { return scalbn(x, k); }
+__device__ __forceinline__ double fp64_scale(double x, int k) {
+  unsigned lo, hi;
+  fp64_words(x, lo, hi);
+  const int e = (int)((hi >> 20) & 0x7ffu);
+  if (e == 0 || e == 0x7ff || (unsigned)(e + k - 1) >= 0x7feu) return fp64_scale_rare(x, k);
+  return __hiloint2double((int)(hi + ((unsigned)k << 20)), (int)lo);
 }
 
 constexpr int kFp64CeilSat = 1 << 30;

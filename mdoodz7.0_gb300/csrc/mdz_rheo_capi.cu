@@ -123,6 +123,8 @@ void fold_phase(const mdz_materials *m, const mdz_model *md, int p, PhaseConst &
   if (m->apwl[p] != 0.0) fl |= F_PWL_A;
   if (m->alin[p] != 0.0) fl |= F_LIN_A;
   if (1.0 / m->n_vp[p] - 1.0 == 0.0) fl |= F_VP1;
+  if (m->mlin[p] != 0.0) fl |= F_LIN_M;
+  if (m->Slim[p] > 0.0) fl |= F_SLIM;
   c.flags = fl;
   c.density_model = m->density_model[p];
   c.phase_two = m->phase_two[p];
@@ -136,6 +138,8 @@ void fold_phase(const mdz_materials *m, const mdz_model *md, int p, PhaseConst &
     if (m->rpwl[p] != 0.0) c.pwl_lnK += -(m->rpwl[p] / n) * log(m->fpwl[p]);
     c.pwl_Q = m->Qpwl[p]; c.pwl_V = m->Vpwl[p]; c.pwl_invRn = 1.0 / (R * n);
     c.pwl_mn = m->mpwl[p] / n; c.pwl_an = m->apwl[p] / n;
+    c.pwl_nf = (float)n;
+    c.pwl_om = 1.0 - 1.0 / n; c.pwl_QR = m->Qpwl[p] / (R * n); c.pwl_VR = m->Vpwl[p] / (R * n);
   }
   // diffusion: B = F A^(-1/n) exp((Q+PV)/(R n T)) f^(-r/n) exp(-a phi/n)
   {
@@ -145,6 +149,9 @@ void fold_phase(const mdz_materials *m, const mdz_model *md, int p, PhaseConst &
     if (m->rlin[p] != 0.0) c.lin_lnK += -(m->rlin[p] / n) * log(m->flin[p]);
     c.lin_Q = m->Qlin[p]; c.lin_V = m->Vlin[p]; c.lin_invRn = 1.0 / (R * n);
     c.lin_m = m->mlin[p]; c.lin_mn = m->mlin[p] / n; c.lin_an = m->alin[p] / n;
+    c.lin_nf = (float)n;
+    c.lin_om = 1.0 - 1.0 / n; c.lin_QR = m->Qlin[p] / (R * n); c.lin_VR = m->Vlin[p] / (R * n);
+    c.lin_lnd = -c.lin_mn * log(m->gs_ref[p]);
   }
   // grain-boundary sliding (bracket only)
   {
@@ -164,6 +171,7 @@ void fold_phase(const mdz_materials *m, const mdz_model *md, int p, PhaseConst &
     c.exp_lnA0 = kLnSqrt3 - kLn2 + log(m->Eexp[p]) + (m->nexp[p] != 0.0 ? m->nexp[p] * log(gS) : 0.0);
     c.exp_s3gS = kSqrt3 / gS;
     c.exp_ln_s3gS = log(c.exp_s3gS);
+    c.exp_E2 = c.exp_EaR * c.exp_g2; c.exp_Eo = c.exp_EaR * c.exp_om2; c.exp_ln2s = kLn2 + c.exp_ln_s3gS;
   }
   c.eta0 = m->eta0[p];
   const int p2 = m->phase_two[p];
@@ -198,6 +206,8 @@ int fold_model(const mdz_model *md, const mdz_materials *m, ModelConst &M) {
   M.Eii_floor = 1e-30 / md->scale_E;
   M.eta_up0 = 1.0e100 / md->scale_eta;
   M.ln_eta_up0 = log(M.eta_up0);
+  M.lf_eta_up0 = (float)M.ln_eta_up0;
+  M.eta_pos = M.min_eta > 0.0 && M.max_eta > 0.0;
   M.eta_lo0 = -1.0e100 / md->scale_eta;
   M.d_min = 1e-13 / md->scale_L;
   for (int p = 0; p < M.np; p++) {

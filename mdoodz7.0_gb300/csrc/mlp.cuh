@@ -196,7 +196,7 @@ __device__ __forceinline__ void mlp_forward(MlpShared &S, const float *x, float 
 __device__ __forceinline__ void warm_features(const ModelConst &M, const NodeIn &in, const NodeCtx &c,
                                               const IsoState &S, bool aniso, float *f) {
   const float lo = -40.0f;
-  const float ln_up = f32_trunc(S.ln_eta_up);
+  const float ln_up = S.lf_up;
   f[0] = f32_trunc(c.lnEii) + __logf(f32_trunc(M.scale_E));
   f[1] = 1000.0f * f32_trunc(c.invT) / f32_trunc(M.scale_T);
   f[2] = f32_trunc(in.P) * f32_trunc(M.scale_S) * 1e-9f;

@@ -47,15 +47,23 @@ namespace mdz {
 // FdMath (the operators' finite differences): the FP64 forms.  A central difference over a
 // step of 1e-7 magnifies a change of the last bit of its solves to 1e-9 and more of the
 // derivative, so the operators keep the bits of these forms.
+//
+// The functions of FxMath are called, not inlined: each has ten or more sites per kernel, a
+// node's code runs to thousands of instructions, and small launches wait for instruction
+// fetches (2000 points: 52.6 us inlined, 45 us called; large sweeps the same).
+static __device__ __noinline__ double fx_exp_call(double x) { return fx_exp(x); }
+static __device__ __noinline__ double fx_log_call(double x) { return fx_log(x); }
+static __device__ __noinline__ double fx_recip_call(double x) { return fx_recip(x); }
+static __device__ __noinline__ double fx_sqrt_call(double x) { return fx_sqrt(x); }
 struct FxMath {
   static constexpr bool kFixed = true;  // local solves in fixed point where the start asks for it (ve_solve_fx)
-  static __device__ __forceinline__ double exp(double x) { return fx_exp(x); }
-  static __device__ __forceinline__ double log(double x) { return fx_log(x); }
-  static __device__ __forceinline__ double recip(double x) { return fx_recip(x); }
-  static __device__ __forceinline__ double quotient(double r, double d) { return __dmul_rn(r, fx_recip(d)); }
-  static __device__ __forceinline__ double newton_quotient(double r, double d) { return __dmul_rn(r, fx_recip(d)); }
-  static __device__ __forceinline__ double divide(double r, double d) { return __dmul_rn(r, fx_recip(d)); }
-  static __device__ __forceinline__ double sqrt(double x) { return fx_sqrt(x); }
+  static __device__ __forceinline__ double exp(double x) { return fx_exp_call(x); }
+  static __device__ __forceinline__ double log(double x) { return fx_log_call(x); }
+  static __device__ __forceinline__ double recip(double x) { return fx_recip_call(x); }
+  static __device__ __forceinline__ double quotient(double r, double d) { return __dmul_rn(r, fx_recip_call(d)); }
+  static __device__ __forceinline__ double newton_quotient(double r, double d) { return quotient(r, d); }
+  static __device__ __forceinline__ double divide(double r, double d) { return quotient(r, d); }
+  static __device__ __forceinline__ double sqrt(double x) { return fx_sqrt_call(x); }
   static __device__ __forceinline__ void sincos(double x, double *s, double *c) { fx_sincos(x, s, c); }
 };
 struct FdMath {
@@ -94,6 +102,8 @@ enum : int {
   F_LIN_A = 1 << 13,// alin != 0
   F_VP1 = 1 << 14,  // n_vp == 1 (pow(x, 1/n_vp - 1) == 1)
   F_PWL1 = 1 << 15, // npwl == 1
+  F_LIN_M = 1 << 16,// mlin != 0
+  F_SLIM = 1 << 17, // Slim > 0
 };
 
 // Per-phase constants folded on the host (mdz_rheo_capi.cu: fold_phase).
@@ -101,12 +111,16 @@ struct PhaseConst {
   int flags, density_model, phase_two, reac_phase;
   // dislocation: ln B = lnK + (Q + P V) invRn / T + mn ln d - an phi
   double pwl_n, pwl_invn, pwl_lnK, pwl_Q, pwl_V, pwl_invRn, pwl_mn, pwl_an;
+  float pwl_nf, lin_nf;           // n in FP32
+  double pwl_om, pwl_QR, pwl_VR;  // 1 - 1/n, Q / (R n), V / (R n)
   // diffusion: ln B = lnK + (Q + P V) invRn / T - an phi; eta also carries d^(m/n)
   double lin_n, lin_invn, lin_lnK, lin_Q, lin_V, lin_invRn, lin_m, lin_mn, lin_an;
+  double lin_om, lin_QR, lin_VR, lin_lnd;  // as above; -(m/n) ln(gs_ref)
   // grain-boundary sliding (bracket only: C_gbs is never set by the reference)
   double gbs_n, gbs_invn, gbs_lnK, gbs_Q, gbs_V, gbs_invRn, gbs_m, gbs_mn, gbs_an;
   // Peierls: ST = EaR g2 / T; Eii_exp = exp(lnA0 - EaR om2 / T) (s3gS Tii)^(ST+n)
   double exp_EaR, exp_g2, exp_om2, exp_n, exp_lnA0, exp_s3gS, exp_ln_s3gS;
+  double exp_E2, exp_Eo, exp_ln2s;  // EaR g2, EaR om2, ln 2 + exp_ln_s3gS
   // constant viscosity
   double eta0, eta0_two;
   // plasticity
@@ -120,10 +134,12 @@ struct PhaseConst {
 struct ModelConst {
   int np, elastic, step, eta_average, periodic_x, density_variations, tensile_line_search;
   int diffuse_avg, Nx, Nz, Ncx, Ncz;
+  int eta_pos;  // min_eta > 0 and max_eta > 0
   long long Nc, Nv;
   double dt, dt_model, min_eta, max_eta, eta_tol, R;
   double scale_eta, scale_L, scale_T, scale_S, scale_E;
   double TmaxPeierls, Tmin, Tiimin, Eii_floor, eta_up0, ln_eta_up0, eta_lo0, d_min;
+  float lf_eta_up0;
 };
 
 // Per-node values shared by all phases of one node.
@@ -141,7 +157,11 @@ struct NodeCtx {
   double Eii, lnEii, T, Traw, invT, lnd, K, G, dil, eta_el, inv_eta_el, sin_fric, cos_fric, sin_dil;
   double inv2Eii, inv_Kdt, inv_d;
   double ln_eta_el;         // ln(eta_el), set where elasticity is on
+  float lf_eta_el;          // the same in FP32
+  double Tyield;            // C cos(fric) + P sin(fric) (RheologyDensity.c:530-539), before the phase's limit
   int elastic, plastic_on;  // plastic_on = (step != 0)
+  bool cold;                // T below the Peierls cut-off
+  bool d_zero;              // grain size below the smallest one
 };
 
 struct PointOut {
@@ -156,6 +176,18 @@ __device__ __forceinline__ void set_status(int &st, int code) {
   if (st == MDZ_OK) st = code;
 }
 
+// limiters (RheologyDensity.c:1058-1073)
+__device__ __forceinline__ double clamp_eta(const ModelConst &M, double x) {
+  if (M.eta_pos) {
+    if (fp64_gt_pos(x, M.max_eta)) x = M.max_eta;
+    if (fp64_lt_pos(x, M.min_eta)) x = M.min_eta;
+  } else {
+    if (fp64_gt(x, M.max_eta)) x = M.max_eta;
+    if (fp64_lt(x, M.min_eta)) x = M.min_eta;
+  }
+  return x;
+}
+
 // ---------------------------------------------------------------------------------------
 // node set-up: invariants and switches shared by the phases (RheologyDensity.c:461-496)
 // ---------------------------------------------------------------------------------------
@@ -166,12 +198,16 @@ template <class FP>
 __device__ __forceinline__ void node_common(const ModelConst &M, const NodeIn &in, bool need_lnd, NodeCtx &c) {
   node_strain_update<FP>(c);
   c.Traw = in.T;
-  c.T = fp64_lt(in.T, M.Tmin) ? M.Tmin : in.T;
+  c.T = fp64_lt_pos(in.T, M.Tmin) ? M.Tmin : in.T;
+  c.cold = fp64_lt_pos(in.T, M.TmaxPeierls);
+  c.d_zero = fp64_lt_pos(in.d, M.d_min);
   c.invT = FP::recip(c.T);
   c.lnd = need_lnd ? FP::log(in.d) : 0.0;
   c.inv_d = 0.0;
   FP::sincos(in.fric, &c.sin_fric, &c.cos_fric);
   c.sin_dil = fp64_is_zero(c.dil) ? 0.0 : sin(c.dil);
+  // products and sum rounded apart: the same bits in every kernel
+  c.Tyield = __dadd_rn(__dmul_rn(in.C, c.cos_fric), __dmul_rn(in.P, c.sin_fric));
 }
 
 // The strain-rate invariant and what depends on it (RheologyDensity.c:455-459); the
@@ -180,7 +216,7 @@ template <class FP>
 __device__ __forceinline__ void node_strain_iso(const ModelConst &M, const NodeIn &in, NodeCtx &c) {
   const double Eyy = -(in.Exx + in.Ezz);
   double Eii = FP::sqrt(0.5 * (in.Exx * in.Exx + in.Ezz * in.Ezz + Eyy * Eyy) + in.Exz * in.Exz);
-  if (fp64_lt(Eii * M.scale_E, 1e-30)) Eii = M.Eii_floor;
+  if (fp64_lt_pos(Eii * M.scale_E, 1e-30)) Eii = M.Eii_floor;
   c.Eii = Eii;
 }
 
@@ -203,6 +239,7 @@ __device__ __forceinline__ void node_setup_iso(const ModelConst &M, const NodeIn
   c.eta_el = c.G * M.dt;
   c.inv_eta_el = FP::recip(c.eta_el);
   c.ln_eta_el = c.elastic ? FP::log(c.eta_el) : 0.0;
+  c.lf_eta_el = f32_trunc(c.ln_eta_el);
   c.inv_Kdt = FP::recip(c.K * M.dt);
   node_common<FP>(M, in, need_lnd, c);
 }
@@ -248,12 +285,35 @@ template <class FP>
 __device__ __forceinline__ void creep_laws(const ModelConst &M, const PhaseConst &ph, const NodeCtx &c, double P,
                                            double phi, double lnd, int peierls, Laws &L) {
   const int fl = ph.flags;
-  L.mech = (fl & (F_CST | F_PWL | F_LIN | F_GBS)) | (peierls ? F_EXPV : 0);
+  L.mech = (fl & (F_CST | F_PWL | F_LIN | F_GBS | F_PWL1 | F_LIN1)) | (peierls ? F_EXPV : 0);
   L.ln_inv[0] = L.ln_inv[1] = L.ln_inv[2] = -kInf;
   L.n[0] = ph.pwl_n; L.n[1] = 0.0; L.n[2] = ph.lin_n;
   L.lnB_pwl = L.lnB_lin = L.lnA_exp = L.ST = 0.0;
   L.ln_inv_gbs = -kInf;
   const double lnEii = c.lnEii;
+  if (FP::kFixed) {  // the forms below with folded constants: fewer FP64 instructions, other last bits
+    if (fl & F_PWL) {
+      double lnB = fma(fma(P, ph.pwl_VR, ph.pwl_QR), c.invT, ph.pwl_lnK);
+      if (fl & F_PWL_M) lnB = fma(ph.pwl_mn, lnd, lnB);
+      if (fl & F_PWL_A) lnB -= ph.pwl_an * phi;
+      L.lnB_pwl = lnB;
+      L.ln_inv[K_PWL] = fma(lnEii, ph.pwl_om, -lnB);
+    }
+    if (fl & F_LIN) {
+      double lnB = fma(fma(P, ph.lin_VR, ph.lin_QR), c.invT, ph.lin_lnK);
+      if (fl & F_LIN_A) lnB -= ph.lin_an * phi;
+      L.lnB_lin = lnB;
+      const double lnBd = (fl & F_LIN_M) ? fma(ph.lin_mn, lnd, lnB) : lnB;
+      L.ln_inv[K_LIN] = (fl & F_LIN1) ? -lnBd : fma(lnEii, ph.lin_om, -lnBd);
+    }
+    if (peierls) {
+      L.ST = ph.exp_E2 * c.invT;
+      const double nE = L.ST + ph.exp_n;
+      L.n[K_EXP] = nE;
+      L.lnA_exp = fma(-ph.exp_Eo, c.invT, ph.exp_lnA0);
+      L.ln_inv[K_EXP] = (ph.exp_ln2s + lnEii) - FP::quotient(lnEii - L.lnA_exp, nE);
+    }
+  } else {
   if (fl & F_PWL) {
     // B = pref F A^(-1/n) exp((Q+PV)/(RnT)) d^(m/n) f^(-r/n) exp(-a phi/n);
     // 1/eta_pwl = Eii^(1-1/n) / B:  ln(1/eta_pwl) = lnEii - lnEii/n - lnB
@@ -268,7 +328,7 @@ __device__ __forceinline__ void creep_laws(const ModelConst &M, const PhaseConst
     double lnB = ph.lin_lnK + (ph.lin_Q + P * ph.lin_V) * ph.lin_invRn * c.invT;
     if (fl & F_LIN_A) lnB -= ph.lin_an * phi;
     L.lnB_lin = lnB;
-    const double lnBd = !fp64_is_zero(ph.lin_m) ? fma(ph.lin_mn, lnd, lnB) : lnB;
+    const double lnBd = (fl & F_LIN_M) ? fma(ph.lin_mn, lnd, lnB) : lnB;
     L.ln_inv[K_LIN] = lnEii - fma(lnEii, ph.lin_invn, lnBd);
   }
   if (peierls) {
@@ -279,6 +339,7 @@ __device__ __forceinline__ void creep_laws(const ModelConst &M, const PhaseConst
     L.n[K_EXP] = nE;
     L.lnA_exp = ph.exp_lnA0 - ph.exp_EaR * ph.exp_om2 * c.invT;
     L.ln_inv[K_EXP] = (kLn2 + ph.exp_ln_s3gS + lnEii) - FP::quotient(lnEii - L.lnA_exp, nE);
+  }
   }
   if (fl & F_GBS) {
     double lnB = ph.gbs_lnK + (ph.gbs_Q + P * ph.gbs_V) * ph.gbs_invRn * c.invT - ph.gbs_an * phi;
@@ -296,6 +357,13 @@ __device__ __forceinline__ void creep_laws(const ModelConst &M, const PhaseConst
 // the softest non-linear law p and nc_k = n_k ln(eta_p / eta_k) <= 0.  Every quantity
 // in the exponent is O(1) for the terms that carry strain rate, so nothing large cancels.
 // ---------------------------------------------------------------------------------------
+// eta_n = 2^k and its logarithm
+__device__ __forceinline__ void pow2_normalisation(int k, double &eta_n, double &ln_eta_n) {
+  eta_n = __hiloint2double((k + 1023) << 20, 0);
+  const double kd = __hiloint2double(0x43300000, k ^ (int)0x80000000) - 4503601774854144.0;  // (double)k
+  ln_eta_n = fma(kd, MDZ_LN2_HI, kd * MDZ_LN2_LO);
+}
+
 // Inputs of the general (FP64) form of the local solve: any start, any normalisation.
 struct VeArgs {
   Laws L;
@@ -325,11 +393,19 @@ struct VeCoef {
   int nl;                          // bit k: law k is non-linear and active
 };
 
+// Strain rates over Eii where the caller is a sweep or a point (FP::kFixed; ve_solve), as
+// they are otherwise.
 struct VeState {
   double eta, Tii, e_cst, e_pwl, e_exp, e_lin;
   double e[K_COUNT];  // strain rates of the non-linear laws at the last evaluated point
   int iters, status;
 };
+
+// strain rates over Eii
+__device__ __forceinline__ void ve_normalise(VeState &s, double Eii) {
+  const double i = fx_recip_call(Eii);
+  s.e_cst *= i; s.e_pwl *= i; s.e_exp *= i; s.e_lin *= i;
+}
 
 template <class FP>
 __device__ __forceinline__ void ve_coef(const VeArgs &v, VeCoef &q) {
@@ -584,56 +660,68 @@ __device__ __forceinline__ bool start_dd(int polish) { return (polish & MDZ_STAR
 
 // The local solve in fixed point (ve_fx.cuh) from the FP32 Newton steps: the coefficients of
 // the normalised residual, the FP32 steps, the fixed-point root, and the FP64 outputs at it.
-// eta_n must be a power of two.  false where the fixed-point form declines: the caller runs
-// the FP64 iteration.  Counts as one evaluation.
+// eta_n = 2^k2.  false where the fixed-point form declines: the caller runs the FP64
+// iteration.  Counts as one evaluation.
 template <class FP>
-__device__ __forceinline__ bool ve_solve_fx(const Laws &L, const NodeCtx &c, double eta_cst, double eta_n,
-                                            double ln_eta_n, float s_start, float s_hi, int fp32, int &f32_steps,
-                                            VeState &s) {
-  double A = c.elastic ? c.inv_eta_el : 0.0, inv_cst = 0.0, inv[K_COUNT] = {0.0, 0.0, 0.0}, a[K_COUNT];
+__device__ __forceinline__ bool ve_solve_fx(const PhaseConst &ph, const Laws &L, const NodeCtx &c, double eta_cst, int k2, float s_start,
+                                            float s_hi, int fp32, int &f32_steps, VeState &s) {
+  double A = c.elastic ? c.inv_eta_el : 0.0, inv_cst = 0.0, inv[K_COUNT] = {0.0, 0.0, 0.0};
   float nf[K_COUNT] = {0.f, 0.f, 0.f}, cf[K_COUNT] = {0.f, 0.f, 0.f};
+  int64_t N[K_COUNT], X[K_COUNT];
   if (L.mech & F_CST) { inv_cst = FP::recip(eta_cst); A += inv_cst; }
   int nl = 0, tiny = 0;  // tiny: laws below e^-150, left out of the residual
   float nmax = 0.0f;
+  // k2 ln 2 = k2 - k2 (1 - ln 2) in Q.54; 1 - ln2 = 0x4e8de808 2e308654 2^-64
+  const int64_t p0 = (int64_t)k2 * 0x2e308654, p1 = (int64_t)k2 * 0x4e8de808 + (p0 >> 32);
+  const int64_t kln2 = (int64_t)((uint64_t)(int64_t)k2 << 54) - (int64_t)((uint64_t)p1 << 22) -
+                       (int64_t)(fx_lo((uint64_t)p0) >> 10);
 #pragma unroll
   for (int k = 0; k < K_COUNT; k++) {
     const int bit = (k == K_PWL) ? F_PWL : ((k == K_EXP) ? F_EXPV : F_LIN);
-    a[k] = 0.0;
     if (!(L.mech & bit)) continue;
-    if (k != K_EXP && fp64_eq_nonzero(L.n[k], 1.0)) {  // Newtonian law: Eii eta / eta_k
+    if (k != K_EXP && (L.mech & (k == K_PWL ? F_PWL1 : F_LIN1))) {  // Newtonian law: Eii eta / eta_k
       inv[k] = law_inv<FP>(L, k);
       A += inv[k];
     } else {
-      a[k] = L.n[k] * (ln_eta_n + L.ln_inv[k]);
-      if (fp64_lt(a[k], -150.0)) {
+      // the argument at s = 1, n (ln eta_n + ln(1/eta_k)), in Q9.54
+      const uint64_t nb = fx_bits(L.n[k]), lb = fx_bits(L.ln_inv[k]);
+      if (fx_hi(nb) >= 0x40600000u || (fx_hi(lb) & 0x7fffffffu) >= 0x40800000u) return false;  // n < 128, |ln| < 512
+      nf[k] = k == K_PWL ? ph.pwl_nf : (k == K_LIN ? ph.lin_nf : f32_trunc(L.n[k]));
+      const float df = fmaf((float)k2, 0.693147182f, f32_trunc(L.ln_inv[k]));
+      cf[k] = nf[k] * df;
+      if (cf[k] < -149.0f) {
         tiny |= 1 << k;
       } else {
+        if (!(cf[k] < 149.0f && fabsf(df) < 500.0f)) return false;
         nl |= 1 << k;
-        nf[k] = f32_trunc(L.n[k]);
-        cf[k] = f32_trunc(a[k]);
+        N[k] = fx_fixed<56>(nb);
+        X[k] = fx_mul_nd(N[k], fx_fixed<54>(lb) + kln2);
+        cf[k] = (float)(int32_t)(X[k] >> 31) * 1.1920929e-7f;  // 2^-23
         nmax = fmaxf(nmax, nf[k]);
       }
     }
   }
-  const double lin = A * eta_n;
+  const double lin = fp64_scale(A, k2);
   const float s0 = ve_polish_f32(nl, f32_trunc(lin), nf, cf, s_start, fp32, f32_steps, s_hi, 3, nmax);
   VeFxRoot r;
-  if (!ve_root_fx(nl, lin, L.n, a, nf, s0, r)) return false;
-  const int k2 = (int)(fp64_exponent(eta_n)) - 1023;
+  if (!ve_root_fx(nl, lin, N, X, nf, s0, r)) return false;
   s.eta = fx_normalise(r.S, k2 - 62);
-  const double E_eta = s.eta * c.Eii;
-  s.Tii = 2.0 * E_eta;
-  s.e_cst = E_eta * inv_cst;
+  s.Tii = fp64_scale(s.eta * c.Eii, 1);
+  s.e_cst = (L.mech & F_CST) ? s.eta * inv_cst : 0.0;
+  double e[K_COUNT];
 #pragma unroll
-  for (int k = 0; k < K_COUNT; k++)
-    s.e[k] = (nl >> k & 1) ? c.Eii * fx_normalise(r.M[k], r.m[k] - 62) : E_eta * inv[k];
+  for (int k = 0; k < K_COUNT; k++) {
+    const int bit = (k == K_PWL) ? F_PWL : ((k == K_EXP) ? F_EXPV : F_LIN);
+    e[k] = (nl >> k & 1) ? fx_normalise(r.M[k], r.m[k] - 62)
+                         : ((k != K_EXP && (L.mech & bit) && !(tiny >> k & 1)) ? s.eta * inv[k] : 0.0);
+  }
   if (tiny) {
-    const double ln_s = FP::log(fx_normalise(r.S, -62));
+    const double ln_eta = FP::log(s.eta);
 #pragma unroll
     for (int k = 0; k < K_COUNT; k++)
-      if (tiny >> k & 1) s.e[k] = c.Eii * FP::exp(fma(L.n[k], ln_s, a[k]));
+      if (tiny >> k & 1) e[k] = FP::exp(L.n[k] * (ln_eta + L.ln_inv[k]));
   }
-  s.e_pwl = s.e[K_PWL]; s.e_exp = s.e[K_EXP]; s.e_lin = s.e[K_LIN];
+  s.e_pwl = e[K_PWL]; s.e_exp = e[K_EXP]; s.e_lin = e[K_LIN];
   s.iters = 1;
   return true;
 }
@@ -657,16 +745,18 @@ static __device__ __noinline__ VeOut ve_general_fx(VeArgs v) {
   VeOut o;
   o.s.status = MDZ_OK;
   ve_general_inl<FxMath>(v, o.s, o.f32_steps);
+  ve_normalise(o.s, v.Eii);
   return o;
 }
 
 template <class FP>
-__device__ __forceinline__ void ve_solve(const Laws &L, const NodeCtx &c, double eta_cst, const double eta_n,
-                                         double ln_eta_n, bool pow2, float s_start, float s_up, int polish, VeState &s,
+__device__ __forceinline__ void ve_solve(const PhaseConst &ph, const Laws &L, const NodeCtx &c, double eta_cst, double eta_n,
+                                         double ln_eta_n, bool pow2, int k2, float s_start, float s_up, int polish, VeState &s,
                                          int &f32_steps) {
   if (FP::kFixed && pow2 && start_dd(polish) && start_fp32(polish) > 0 &&
-      ve_solve_fx<FP>(L, c, eta_cst, eta_n, ln_eta_n, s_start * s_up, s_up, start_fp32(polish), f32_steps, s))
+      ve_solve_fx<FP>(ph, L, c, eta_cst, k2, s_start * s_up, s_up, start_fp32(polish), f32_steps, s))
     return;
+  if (FP::kFixed && pow2) pow2_normalisation(k2, eta_n, ln_eta_n);
   VeArgs v;
   ve_args(v, L, c, eta_cst, eta_n, ln_eta_n, s_start, s_up, polish);
   if (FP::kFixed) {
@@ -845,7 +935,9 @@ struct IsoState {
   // start point eta_up in that unknown (1 when exact)
   double eta_n, ln_eta_n;
   float s_up;
-  bool pow2;  // eta_n is a power of two
+  bool pow2;  // eta_n = 2^k2 (sweeps and points form it, and its logarithm, only where they are used)
+  int k2;
+  float lf_up;  // ln(eta_up) in FP32
 };
 
 // Start point of the local solve (RheologyDensity.c:582-592, AnisotropyRoutines.c:409-415):
@@ -875,9 +967,33 @@ __device__ __forceinline__ void start_viscosity(const ModelConst &M, double ln_i
 // unknown is normalised by eta_n = 2^k, k the nearest integer to log2(eta_up), built from
 // bits, with ln(eta_n) = k ln2; s_up = exp(ln eta_up - k ln2) in [0.7, 1.42] in FP32.
 template <class FP>
-__device__ __forceinline__ void start_point(const ModelConst &M, double ln_inv_max, bool constant, double eta_cst,
+__device__ __forceinline__ void start_point(const ModelConst &M, const Laws &L, bool constant, double eta_cst,
                                             bool elastic, const NodeCtx &c, bool exact, IsoState &S) {
-  if (!exact) {
+  if (FP::kFixed && !exact) {
+    // the same bound in FP32: truncation keeps the order, and k and s_up need no more
+    float li = -3.4e38f;
+    if (L.mech & F_PWL) li = f32_trunc(L.ln_inv[K_PWL]);
+    if (L.mech & F_EXPV) li = fmaxf(li, f32_trunc(L.ln_inv[K_EXP]));
+    if (L.mech & F_LIN) li = fmaxf(li, f32_trunc(L.ln_inv[K_LIN]));
+    if (L.mech & F_GBS) li = fmaxf(li, f32_trunc(L.ln_inv_gbs));
+    float lf = M.lf_eta_up0;
+    if (constant) lf = fminf(lf, f32_trunc(FP::log(eta_cst)));
+    if (li > -3.3e38f) lf = fminf(lf, -li);
+    if (elastic) lf = fminf(lf, c.lf_eta_el);
+    if (fabsf(lf) < 690.0f) {  // finite, and 2^k a normal double
+      const int k = __float2int_rn(lf * 1.44269504f);
+      S.lf_up = lf;
+      S.ln_eta_up = S.eta_up = S.eta_n = S.ln_eta_n = 0.0;  // not formed
+      S.k2 = k;
+      S.s_up = __expf(fmaf((float)-k, 0.693147182f, lf));
+      S.pow2 = true;
+      return;
+    }
+  }
+  // the smallest isolated viscosity is 1 / the largest reciprocal
+  const double ln_inv_max = fp64_fmax(fp64_fmax(L.ln_inv[K_PWL], L.ln_inv[K_EXP]),
+                                      fp64_fmax(L.ln_inv[K_LIN], L.ln_inv_gbs));
+  if (!FP::kFixed && !exact) {
     double ln = M.ln_eta_up0;
     if (constant) {
       const double lc = FP::log(eta_cst);
@@ -890,9 +1006,8 @@ __device__ __forceinline__ void start_point(const ModelConst &M, double ln_inv_m
       const int k = __float2int_rn(lf * 1.44269504f);
       S.ln_eta_up = ln;
       S.eta_up = 0.0;  // not formed
-      S.eta_n = __hiloint2double((k + 1023) << 20, 0);
-      const double kd = __hiloint2double(0x43300000, k ^ (int)0x80000000) - 4503601774854144.0;  // (double)k
-      S.ln_eta_n = fma(kd, MDZ_LN2_HI, kd * MDZ_LN2_LO);
+      S.k2 = k;
+      pow2_normalisation(k, S.eta_n, S.ln_eta_n);
       S.s_up = __expf(fmaf((float)-k, 0.693147182f, lf));
       S.pow2 = true;
       return;
@@ -901,6 +1016,7 @@ __device__ __forceinline__ void start_point(const ModelConst &M, double ln_inv_m
   start_viscosity<FP>(M, ln_inv_max, constant, eta_cst, elastic, c, S.eta_up, S.ln_eta_up);
   S.eta_n = S.eta_up;
   S.ln_eta_n = S.ln_eta_up;
+  S.lf_up = f32_trunc(S.ln_eta_up);
   S.s_up = 1.0f;
   S.pow2 = false;
 }
@@ -926,7 +1042,7 @@ __device__ inline void iso_setup(const ModelConst &M, const PhaseConst &ph, cons
                                  IsoState &S, PointOut &o, bool exact = true) {
   const int fl = ph.flags;
   const int constant = (fl & F_CST) != 0, diffusion = (fl & F_LIN) != 0, gs = (fl & F_GS) != 0;
-  const int peierls = ((fl & F_EXPV) != 0) && fp64_lt(c.Traw, M.TmaxPeierls);
+  const int peierls = ((fl & F_EXPV) != 0) && c.cold;
   const int plastic = c.plastic_on ? ((fl & F_PL1) ? 1 : ((fl & F_PL2) ? 2 : 0)) : 0;
   const int elastic = c.elastic;
   const double T = c.T, P = in.P, Eii = c.Eii, eta_el = c.eta_el;
@@ -945,14 +1061,14 @@ __device__ inline void iso_setup(const ModelConst &M, const PhaseConst &ph, cons
   o.rho = 0.0;
   o.d1 = ph.gs_ref;
   o.inv_d1 = ph.inv_gs_ref;
-  if (diffusion && fp64_gt(ph.lin_m, 0.0) && fp64_lt(in.d, M.d_min)) set_status(o.status, MDZ_EGRAIN_ZERO);
+  if (c.d_zero && diffusion && fp64_gt(ph.lin_m, 0.0)) set_status(o.status, MDZ_EGRAIN_ZERO);
 
   Laws &L = S.L;
   creep_laws<FP>(M, ph, c, P, in.phi, c.lnd, peierls, L);
   double Tyield = 0.0, C = in.C;
-  if (plastic == 1) {  // :530-539 (products and sum rounded apart: the same bits in every kernel)
-    Tyield = __dadd_rn(__dmul_rn(C, c.cos_fric), __dmul_rn(P, c.sin_fric));
-    if (fp64_lt(ph.Slim, Tyield)) { C = ph.Slim; Tyield = ph.Slim; }
+  if (plastic == 1) {  // :530-539 (the operators perturb P after the node's set-up)
+    Tyield = FP::kFixed ? c.Tyield : __dadd_rn(__dmul_rn(C, c.cos_fric), __dmul_rn(P, c.sin_fric));
+    if ((fl & F_SLIM) ? fp64_gt_pos(Tyield, ph.Slim) : fp64_lt(ph.Slim, Tyield)) { C = ph.Slim; Tyield = ph.Slim; }
   }
   double eta_cst = 0.0, Ag = 0.0, lnd = c.lnd;
   if (constant) eta_cst = ph.eta0;
@@ -970,22 +1086,22 @@ __device__ inline void iso_setup(const ModelConst &M, const PhaseConst &ph, cons
     o.d1 = d;
     lnd = log(d);
     if (diffusion) {
-      const double lnBd = !fp64_is_zero(ph.lin_m) ? fma(ph.lin_mn, lnd, L.lnB_lin) : L.lnB_lin;
+      const double lnBd = (fl & F_LIN_M) ? fma(ph.lin_mn, lnd, L.lnB_lin) : L.lnB_lin;
       L.ln_inv[K_LIN] = c.lnEii - fma(c.lnEii, ph.lin_invn, lnBd);
     }
   }
-  // bracket (:582-592): the smallest isolated viscosity is 1 / the largest reciprocal
-  const double ln_inv_max =
-      fp64_fmax(fp64_fmax(L.ln_inv[K_PWL], L.ln_inv[K_EXP]), fp64_fmax(L.ln_inv[K_LIN], L.ln_inv_gbs));
-  start_point<FP>(M, ln_inv_max, constant, eta_cst, elastic == 1, c, exact || gs, S);
+  start_point<FP>(M, L, constant, eta_cst, elastic == 1, c, exact || gs, S);  // bracket (:582-592)
   S.eta_cst = eta_cst; S.Tyield = Tyield; S.C = C; S.Ag = Ag; S.lnd = lnd;
 }
 
 // The state of one (node, phase) between its visco-elastic solve and its post-processing.
 struct IsoMid {
-  double eta_ve, Tii, Tii_ve, Tyield, e_cst, e_pwl, e_exp, e_lin;
+  double eta_ve, Tii, Tii_ve, Tyield, e_cst, e_pwl, e_exp, e_lin;  // e_*: over Eii (sweeps, points)
   double gdot, divp, Pc, eta_vep, lam_dot, A_tau, A_P, eta_vp;
   int is_pl;
+  // what the sweeps' averages need of a yielding item (dp_extra): eta_ve gdot / Tii (the
+  // plastic rate beside the creep rates, over the stress) and Tii / eta_ve
+  double pl_share, T_over_eta;
 };
 
 // Inputs and results of the Drucker-Prager return of one (node, phase) (plastic == 1,
@@ -995,12 +1111,13 @@ struct IsoMid {
 struct DpItem {
   double Tii, Tyield, eta_ve, P, K, sin_fric, sin_dil, Eii, inv2Eii;  // in; Tii, Tyield out
   double gdot, divp, Pc, eta_vp, eta_vep;                              // out
+  double pl_share, T_over_eta;                                         // out (dp_extra)
 };
 
 __device__ __forceinline__ bool iso_yields_dp(const ModelConst &M, const PhaseConst &ph, const NodeCtx &c,
                                               const IsoMid &m) {
   const int plastic = c.plastic_on ? ((ph.flags & F_PL1) ? 1 : ((ph.flags & F_PL2) ? 2 : 0)) : 0;
-  return plastic == 1 && fp64_gt(m.Tii - m.Tyield, 1e-17);
+  return plastic == 1 && fp64_gt_pos(m.Tii - m.Tyield, 1e-17);
 }
 
 __device__ __forceinline__ void dp_load(DpItem &d, const IsoMid &m, const NodeIn &in, const NodeCtx &c) {
@@ -1012,6 +1129,7 @@ __device__ __forceinline__ void dp_store(IsoMid &m, const DpItem &d) {
   m.is_pl = 1;
   m.Tii = d.Tii; m.Tyield = d.Tyield; m.gdot = d.gdot; m.divp = d.divp; m.Pc = d.Pc; m.eta_vp = d.eta_vp;
   m.eta_vep = d.eta_vep;
+  m.pl_share = d.pl_share; m.T_over_eta = d.T_over_eta;
 }
 
 // The Drucker-Prager return (:655-707) of an item that yields (Tii - Tyield > 1e-17).
@@ -1067,6 +1185,11 @@ __device__ inline void dp_return(const ModelConst &M, const PhaseConst &ph, DpIt
   d.Tii = Tiic;
 }
 
+__device__ __forceinline__ void dp_extra(DpItem &d) {
+  d.pl_share = d.eta_ve * d.gdot * fx_recip_call(d.Tii);
+  d.T_over_eta = d.Tii * fx_recip_call(d.eta_ve);
+}
+
 // Local solve (from s_start * eta_up, moved by the start stages that the descriptor
 // `polish` names (ve_start); s_start = 1 and polish = 0 is the reference's start) of one
 // (node, phase), up to its plastic corrections.  eta_conv (may be null) receives the
@@ -1078,7 +1201,7 @@ __device__ inline void iso_ve(const ModelConst &M, const PhaseConst &ph, const N
   const int fl = ph.flags;
   const int constant = (fl & F_CST) != 0, dislocation = (fl & F_PWL) != 0, diffusion = (fl & F_LIN) != 0;
   const int gbs = (fl & F_GBS) != 0, gs = (fl & F_GS) != 0;
-  const int peierls = ((fl & F_EXPV) != 0) && fp64_lt(c.Traw, M.TmaxPeierls);
+  const int peierls = ((fl & F_EXPV) != 0) && c.cold;
   const int elastic = c.elastic;
   const double P = in.P, Eii = c.Eii, eta_el = c.eta_el;
   Laws &L = S.L;
@@ -1088,7 +1211,7 @@ __device__ inline void iso_ve(const ModelConst &M, const PhaseConst &ph, const N
   if (!gs) {  // LocalIterationViscoElastic (:646)
     VeState s;
     s.status = MDZ_OK;
-    ve_solve<FP>(L, c, eta_cst, S.eta_n, S.ln_eta_n, S.pow2, s_start, S.s_up, polish, s, o.f32_steps);
+    ve_solve<FP>(ph, L, c, eta_cst, S.eta_n, S.ln_eta_n, S.pow2, S.k2, s_start, S.s_up, polish, s, o.f32_steps);
     set_status(o.status, s.status);
     eta_ve = s.eta; Tii = s.Tii; e_cst = s.e_cst; e_pwl = s.e_pwl; e_exp = s.e_exp; e_lin = s.e_lin;
     o.iters = s.iters;
@@ -1110,6 +1233,10 @@ __device__ inline void iso_ve(const ModelConst &M, const PhaseConst &ph, const N
     set_status(o.status, st);
     o.d1 = dd;
     o.inv_d1 = 1.0 / dd;
+    if (FP::kFixed) {
+      const double i = FP::recip(Eii);
+      e_cst *= i; e_pwl *= i; e_exp *= i; e_lin *= i;
+    }
   }
   if (eta_conv) *eta_conv = eta_ve;
   m.eta_ve = eta_ve; m.Tii = Tii; m.Tii_ve = Tii; m.Tyield = Tyield;
@@ -1117,6 +1244,23 @@ __device__ inline void iso_ve(const ModelConst &M, const PhaseConst &ph, const N
   m.gdot = 0.0; m.divp = 0.0; m.Pc = P; m.eta_vep = 0.0; m.lam_dot = 0.0; m.A_tau = 1.0; m.A_P = 0.0;
   m.eta_vp = ph.eta_vp;
   m.is_pl = 0;
+  m.pl_share = 0.0;
+  m.T_over_eta = FP::kFixed ? fp64_scale(Eii, 1) : 0.0;
+}
+
+// The Popov return (plastic == 2) of one (node, phase), into m.
+__device__ __forceinline__ void popov_return(const ModelConst &M, const PhaseConst &ph, const NodeIn &in,
+                                             const NodeCtx &c, const IsoState &S, PointOut &o, IsoMid &m) {
+  int st = MDZ_OK;
+  double Tn = m.Tii, A_P = 0.0;
+  m.is_pl = plastic_popov(M, ph, m.Tii, in.P, S.C, c.cos_fric, c.sin_fric, c.sin_dil, m.eta_ve, c.K, Tn, m.Pc,
+                          m.lam_dot, m.A_tau, A_P, m.eta_vp, st);
+  set_status(o.status, st);
+  if (m.is_pl) {
+    m.eta_vep = Tn * c.inv2Eii;
+    m.Tii = Tn;
+    m.divp = m.lam_dot * A_P;
+  }
 }
 
 // Plastic corrections but the Drucker-Prager return (which dp_return does), and the
@@ -1127,32 +1271,24 @@ __device__ inline void iso_post(const ModelConst &M, const PhaseConst &ph, const
   const int fl = ph.flags;
   const int constant = (fl & F_CST) != 0, dislocation = (fl & F_PWL) != 0, diffusion = (fl & F_LIN) != 0;
   const int gs = (fl & F_GS) != 0;
-  const int peierls = ((fl & F_EXPV) != 0) && fp64_lt(c.Traw, M.TmaxPeierls);
+  const int peierls = ((fl & F_EXPV) != 0) && c.cold;
   const int plastic = c.plastic_on ? ((fl & F_PL1) ? 1 : ((fl & F_PL2) ? 2 : 0)) : 0;
   const int elastic = c.elastic;
   const double T = c.T, P = in.P, Eii = c.Eii, K = c.K;
   const double eta_cst = S.eta_cst, C = S.C, lnd = S.lnd;
   (void)T;
   const double eta_ve = m.eta_ve, Tii_ve = m.Tii_ve;
-  const double e_cst = m.e_cst, e_pwl = m.e_pwl, e_exp = m.e_exp, e_lin = m.e_lin;
+  const double unit = FP::kFixed ? Eii : 1.0;
+  const double e_cst = m.e_cst * unit, e_pwl = m.e_pwl * unit, e_exp = m.e_exp * unit, e_lin = m.e_lin * unit;
   double Tii = m.Tii;
   int is_pl = m.is_pl;
   double gdot = m.gdot, divp = m.divp, Pc = m.Pc, eta_vep = m.eta_vep, lam_dot = m.lam_dot, A_tau = m.A_tau;
   double eta_vp = m.eta_vp;
   if (is_pl && plastic == 1) o.Pcorr = Pc;
-  double A_P = 0.0;
   if (plastic == 2) {
-    int st = MDZ_OK;
-    double Tn = Tii;
-    is_pl = plastic_popov(M, ph, Tii, P, C, c.cos_fric, c.sin_fric, c.sin_dil, eta_ve, K, Tn, Pc, lam_dot, A_tau,
-                          A_P, eta_vp, st);
-    set_status(o.status, st);
-    if (is_pl) {
-      o.Pcorr = Pc;
-      eta_vep = Tn * c.inv2Eii;
-      Tii = Tn;
-      divp = lam_dot * A_P;
-    }
+    popov_return(M, ph, in, c, S, o, m);
+    is_pl = m.is_pl; Pc = m.Pc; lam_dot = m.lam_dot; A_tau = m.A_tau; eta_vp = m.eta_vp;
+    if (is_pl) { o.Pcorr = Pc; eta_vep = m.eta_vep; Tii = m.Tii; divp = m.divp; }
   }
 
   // density on centroids (:934-960); only density_variations==1 lets it reach the grid
@@ -1174,7 +1310,7 @@ __device__ inline void iso_post(const ModelConst &M, const PhaseConst &ph, const
     if (diffusion) {
       // eta_lin = B pow(Eii_lin, 1/n-1) pow(d1, m/n) = Tii/(2 Eii_lin) (d1/d)^(m/n), d1 = gs_ref
       double inv_lin = e_lin * inv_half_T;
-      if (!fp64_is_zero(ph.lin_m) && !gs) inv_lin *= FP::exp(ph.lin_mn * (lnd - ph.ln_gs_ref));
+      if ((fl & F_LIN_M) && !gs) inv_lin *= FP::exp(ph.lin_mn * (lnd - ph.ln_gs_ref));
       inv += inv_lin;
     }
     if (constant) inv += (1.0 / eta_cst);
@@ -1219,12 +1355,8 @@ __device__ inline void iso_post(const ModelConst &M, const PhaseConst &ph, const
       o.div_el = 0.0;
     }
   }
-  // limiters (:1058-1073)
-  if (fp64_gt(o.etaVE, M.max_eta)) o.etaVE = M.max_eta;
-  if (fp64_lt(o.etaVE, M.min_eta)) o.etaVE = M.min_eta;
-  if (fp64_gt(eta, M.max_eta)) eta = M.max_eta;
-  if (fp64_lt(eta, M.min_eta)) eta = M.min_eta;
-  o.eta = eta;
+  o.etaVE = clamp_eta(M, o.etaVE);
+  o.eta = clamp_eta(M, eta);
 }
 
 // Local solve, plastic corrections and post-processing of one (node, phase): iso_ve, the
@@ -1273,6 +1405,7 @@ __device__ __forceinline__ void compact_init(CompactQueue &Q) {
 
 // par: the phase parity, flipped here.  count[par ^ 1] is cleared between the two
 // barriers, where no thread touches it; count[par] is read only between them.
+template <bool EXTRA>
 __device__ __forceinline__ void dp_compact(const ModelConst &M, const PhaseConst &ph, CompactQueue &Q, int &par,
                                            bool yields, IsoMid &m, const NodeIn &in, const NodeCtx &c) {
   const int t = threadIdx.x, lane = t & 31;
@@ -1287,6 +1420,7 @@ __device__ __forceinline__ void dp_compact(const ModelConst &M, const PhaseConst
   if (t < q) {
     DpItem d = Q.item[t];
     dp_return(M, ph, d);
+    if (EXTRA) dp_extra(d);
     Q.item[t] = d;
   }
   __syncthreads();
@@ -1327,6 +1461,7 @@ __device__ __forceinline__ void node_setup_aniso(const ModelConst &M, const Node
   c.eta_el = c.elastic ? c.G * M.dt_model : 1e20;
   c.inv_eta_el = FP::recip(c.eta_el);
   c.ln_eta_el = c.elastic ? FP::log(c.eta_el) : 0.0;
+  c.lf_eta_el = f32_trunc(c.ln_eta_el);
   c.inv_Kdt = FP::recip(c.K * M.dt_model);
   node_common<FP>(M, in, need_lnd, c);
   c.inv_d = FP::divide(1.0, in.d);
@@ -1337,7 +1472,7 @@ __device__ inline void aniso_setup(const ModelConst &M, const PhaseConst &ph, co
                                    const AnisoNode &an, IsoState &S, PointOut &o, bool exact = true) {
   const int fl = ph.flags;
   const int constant = (fl & F_CST) != 0, dislocation = (fl & F_PWL) != 0, diffusion = (fl & F_LIN) != 0;
-  const int peierls = ((fl & F_EXPV) != 0) && fp64_lt(c.Traw, M.TmaxPeierls);
+  const int peierls = ((fl & F_EXPV) != 0) && c.cold;
   const int plastic = (fl & F_PLANY) != 0;
   const int elastic = c.elastic;
   const double T = c.T, P = in.P, eta_el = c.eta_el, K = c.K, dt = M.dt_model;
@@ -1353,21 +1488,20 @@ __device__ inline void aniso_setup(const ModelConst &M, const PhaseConst &ph, co
   o.OverS = 0.0; o.Wtot = o.Wel = o.Wdiss = 0.0;
   o.d1 = in.d;
   o.inv_d1 = c.inv_d;
-  if (diffusion && fp64_gt(ph.lin_m, 0.0) && fp64_lt(in.d, M.d_min)) set_status(o.status, MDZ_EGRAIN_ZERO);
+  if (c.d_zero && diffusion && fp64_gt(ph.lin_m, 0.0)) set_status(o.status, MDZ_EGRAIN_ZERO);
 
   Laws &L = S.L;
   creep_laws<FP>(M, ph, c, P, in.phi, c.lnd, peierls, L);
   L.mech &= ~F_GBS;  // the anisotropic path has no grain-boundary sliding
   L.ln_inv_gbs = -kInf;
   double Tyield = 0.0, Coh = in.C;
-  if (plastic) {  // :370-377 (products and sum rounded apart: the same bits in every kernel)
-    Tyield = __dadd_rn(__dmul_rn(Coh, c.cos_fric), __dmul_rn(P, c.sin_fric));
+  if (plastic) {  // :370-377 (the operators perturb P after the node's set-up)
+    Tyield = FP::kFixed ? c.Tyield : __dadd_rn(__dmul_rn(Coh, c.cos_fric), __dmul_rn(P, c.sin_fric));
     if (ph.Slim < Tyield) { Coh = ph.Slim; Tyield = ph.Slim; }
   }
   const double eta_cst = constant ? ph.eta0 : 0.0;
   // bracket (:409-415); its lower end is formed only where it is used
-  const double ln_inv_max = fp64_fmax(fp64_fmax(L.ln_inv[K_PWL], L.ln_inv[K_EXP]), L.ln_inv[K_LIN]);
-  start_point<FP>(M, ln_inv_max, constant, eta_cst, elastic != 0, c, exact || (fl & F_GS), S);
+  start_point<FP>(M, L, constant, eta_cst, elastic != 0, c, exact || (fl & F_GS), S);
   S.eta_cst = eta_cst; S.Tyield = Tyield; S.C = Coh; S.Ag = 0.0;
   S.lnd = c.lnd;
   (void)an; (void)T; (void)K; (void)dt; (void)min_eta; (void)max_eta; (void)dislocation; (void)eta_el;
@@ -1432,6 +1566,7 @@ static __device__ __noinline__ VeOut aniso_general_fx(const ModelConst &M, VeArg
   VeOut o;
   o.s.status = MDZ_OK;
   aniso_general_inl<FxMath>(M, v, o.s, o.f32_steps);
+  ve_normalise(o.s, v.Eii);
   return o;
 }
 
@@ -1444,7 +1579,7 @@ __device__ inline void aniso_finish(const ModelConst &M, const PhaseConst &ph, c
                                    double *eta_conv = nullptr) {
   const int fl = ph.flags;
   const int constant = (fl & F_CST) != 0, dislocation = (fl & F_PWL) != 0, diffusion = (fl & F_LIN) != 0;
-  const int peierls = ((fl & F_EXPV) != 0) && fp64_lt(c.Traw, M.TmaxPeierls);
+  const int peierls = ((fl & F_EXPV) != 0) && c.cold;
   const int plastic = (fl & F_PLANY) != 0;
   const int elastic = c.elastic;
   const double T = c.T, P = in.P, Eii = c.Eii, eta_el = c.eta_el, K = c.K, dt = M.dt_model;
@@ -1472,10 +1607,12 @@ __device__ inline void aniso_finish(const ModelConst &M, const PhaseConst &ph, c
     VeState s;
     s.status = MDZ_OK;
     if (!(FP::kFixed && S.pow2 && start_dd(polish) && start_fp32(polish) > 0 &&
-          ve_solve_fx<FP>(L, c, eta_cst, S.eta_n, S.ln_eta_n, ((s_start > 0.0f) ? s_start : 1.0f) * S.s_up, S.s_up,
+          ve_solve_fx<FP>(ph, L, c, eta_cst, S.k2, ((s_start > 0.0f) ? s_start : 1.0f) * S.s_up, S.s_up,
                           start_fp32(polish), o.f32_steps, s))) {
       VeArgs v;
-      ve_args(v, L, c, eta_cst, S.eta_n, S.ln_eta_n, s_start, S.s_up, polish);
+      double eta_n = S.eta_n, ln_eta_n = S.ln_eta_n;
+      if (FP::kFixed && S.pow2) pow2_normalisation(S.k2, eta_n, ln_eta_n);
+      ve_args(v, L, c, eta_cst, eta_n, ln_eta_n, s_start, S.s_up, polish);
       v.min_eta = min_eta; v.max_eta = max_eta; v.eta_el = eta_el;
       if (FP::kFixed) {
         const VeOut g = aniso_general_fx(M, v);
@@ -1488,17 +1625,17 @@ __device__ inline void aniso_finish(const ModelConst &M, const PhaseConst &ph, c
     set_status(o.status, s.status);
     eta_ve = s.eta;
     o.iters = s.iters;
-    Tii = s.Tii; e_cst = s.e_cst; e_pwl = s.e_pwl; e_exp = s.e_exp; e_lin = s.e_lin;
+    const double unit = FP::kFixed ? Eii : 1.0;
+    Tii = s.Tii; e_cst = s.e_cst * unit; e_pwl = s.e_pwl * unit; e_exp = s.e_exp * unit; e_lin = s.e_lin * unit;
   }
-  if (fp64_lt(eta_ve, min_eta)) eta_ve = min_eta;  // :589-603
-  if (fp64_gt(eta_ve, max_eta)) eta_ve = max_eta;
+  eta_ve = clamp_eta(M, eta_ve);  // :589-603
   const double Tii_ve = Tii;
   if (eta_conv) *eta_conv = eta_ve;
   double Tr_xx = 2.0 * eta_ve * an.Er_xx, Tr_zz = 2.0 * eta_ve * an.Er_zz, Tr_xz = 2.0 * eta_ve * an.Er_xz / in.ani_fac;
   double eta_vep = eta_ve, gdot = 0.0, Pc = P;
   const double Ft = Tii - Tyield;
   int is_pl = 0;
-  if (fp64_gt(Ft, 1e-17) && plastic) {  // :625-648
+  if (plastic && fp64_gt_pos(Ft, 1e-17)) {  // :625-648
     is_pl = 1;
     // rounded one by one, as in the isotropic return
     const double Kdt_sd = __dmul_rn(__dmul_rn(K, dt), c.sin_dil);
@@ -1520,8 +1657,7 @@ __device__ inline void aniso_finish(const ModelConst &M, const PhaseConst &ph, c
     o.Txz = lxlz * Tr_xx - lxlz * Tr_zz + (lx2 - nz2) * Tr_xz;
   }
   o.Pcorr = Pc;
-  if (fp64_lt(eta_vep, min_eta)) eta_vep = min_eta;
-  if (fp64_gt(eta_vep, max_eta)) eta_vep = max_eta;
+  eta_vep = clamp_eta(M, eta_vep);
   o.etaVE = eta_vep;
   o.is_pl = is_pl;
   if (is_pl) o.mech |= MDZ_MECH_YIELD;
@@ -1550,9 +1686,7 @@ __device__ inline void aniso_finish(const ModelConst &M, const PhaseConst &ph, c
       o.Wdiss = T2 * inv;
     }
   }
-  if (fp64_gt(eta, max_eta)) eta = max_eta;  // :720-721
-  if (fp64_lt(eta, min_eta)) eta = min_eta;
-  o.eta = eta;
+  o.eta = clamp_eta(M, eta);  // :720-721
 }
 
 template <class FP>

@@ -45,6 +45,15 @@ FX_FN int64_t fx_mul_nl(int64_t N, int64_t L) {
   return ((int64_t)nh * lh << 2) + ((mid + 8) >> 4);
 }
 
+// n d in Q9.54 for n = N in Q7.56 and d = L in Q9.54 (signed), |n d| < 512
+FX_FN int64_t fx_mul_nd(int64_t N, int64_t L) {
+  const int32_t nh = (int32_t)(N >> 32), lh = (int32_t)(L >> 32);
+  const uint32_t nl = fx_lo((uint64_t)N), ll = fx_lo((uint64_t)L);
+  const int64_t mid = (int64_t)((uint64_t)(uint32_t)nh * ll >> 20) + (((int64_t)lh * (int32_t)(nl >> 1)) >> 19) +
+                      (int64_t)(fx_umulhi(nl, ll) >> 20);
+  return (int64_t)((uint64_t)((int64_t)nh * lh) << 8) + ((mid + 8) >> 4);
+}
+
 // n L in Q.62 for n = N in Q7.56 and L in Q.62 with |L| < 2^50 (signed)
 FX_FN int64_t fx_mul_ntiny(int64_t N, int64_t L) {
   const int32_t nh = (int32_t)(N >> 32), lh = (int32_t)(L >> 32);
@@ -67,10 +76,10 @@ struct VeFxRoot {
   int m[3];
 };
 
-// nl: bit k set: law k is non-linear and active.  a: the linear coefficient; n, c: exponent
-// and argument at s = 1 of each law, nf their FP32 truncations; s0 the FP32 point.
-FX_FN bool ve_root_fx(int nl, double a, const double *n, const double *c, const float *nf,
-                                           float s0, VeFxRoot &o) {
+// nl: bit k set: law k is non-linear and active.  a: the linear coefficient; N, C: exponent
+// (Q7.56) and argument at s = 1 (Q9.54, below 150 in magnitude) of each law, nf the exponents
+// in FP32; s0 the FP32 point.
+FX_FN bool ve_root_fx(int nl, double a, const int64_t *N, const int64_t *C, const float *nf, float s0, VeFxRoot &o) {
   const uint32_t sb = fx_float_bits(s0);
   const int e0 = (int)(sb >> 23) - 127;  // s0 > 0
   if (e0 > 0 || e0 < -4) return false;
@@ -86,17 +95,13 @@ FX_FN bool ve_root_fx(int nl, double a, const double *n, const double *c, const 
   ok = ok && (int64_t)A0 >= 0;
   int64_t R = (int64_t)0x4000000000000000ll - (int64_t)A0;
   float D = (float)fx_hi(A0) * 9.31322575e-10f, Q = 0.0f;  // 2^-30
-  int64_t N[3];
   if (nl) {
     // ln s0 in Q4.60
     const int64_t L = (int64_t)(fx_log_significand((uint64_t)m24 << 29) >> 4) + (int64_t)e0 * 0xb17217f7d1cf79all;
 #pragma unroll
     for (int k = 0; k < 3; k++)
       if (nl >> k & 1) {
-        const uint64_t nb = fx_bits(n[k]), cb = fx_bits(c[k]);
-        ok = ok && fx_hi(nb) < 0x40600000u && (fx_hi(cb) & 0x7fffffffu) < 0x4062c000u;  // 0 <= n < 128, |c| < 150
-        N[k] = fx_fixed<56>(nb);
-        const int64_t X = fx_mul_nl(N[k], L) + fx_fixed<54>(cb);
+        const int64_t X = fx_mul_nl(N[k], L) + C[k];
         ok = ok && (int32_t)(X >> 32) < 2516582;  // X < 0.6 (and above -505)
         o.M[k] = fx_exp_core(X, o.m[k]);
         const int sh = -o.m[k];

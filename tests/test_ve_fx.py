@@ -39,8 +39,12 @@ def test_root_on_the_host(tmp_path):
     src = tmp_path / "v.cpp"
     src.write_text('#include "ve_fx.cuh"\nextern "C" void run(long n, const int *nl, const double *a, const double *nk, const '
                    "double *c, const float *s0, int *ok, double *s, double *e) {\n  for (long i = 0; i < n; i++) {\n"
-                   "    double N[3], C[3]; float F[3]; mdz::VeFxRoot r;\n"
-                   "    for (int k = 0; k < 3; k++) { N[k] = nk[k * n + i]; C[k] = c[k * n + i]; F[k] = (float)N[k]; }\n"
+                   "    int64_t N[3], C[3]; float F[3]; mdz::VeFxRoot r;\n"
+                   "    ok[i] = 0; bool in = true;\n"
+                   "    for (int k = 0; k < 3; k++) {\n"
+                   "      in = in && (!(nl[i] >> k & 1) || (c[k * n + i] < 149 && c[k * n + i] > -149));\n"
+                   "      N[k] = mdz::fx_fixed<56>(mdz::fx_bits(nk[k * n + i])); F[k] = (float)nk[k * n + i];\n"
+                   "      if (in) C[k] = mdz::fx_fixed<54>(mdz::fx_bits(c[k * n + i]));\n    }\n    if (!in) continue;\n"
                    "    ok[i] = mdz::ve_root_fx(nl[i], a[i], N, C, F, s0[i], r);\n    if (!ok[i]) continue;\n"
                    "    s[i] = mdz::fx_normalise(r.S, -62);\n"
                    "    for (int k = 0; k < 3; k++) e[k * n + i] = (nl[i] >> k & 1) ? mdz::fx_normalise(r.M[k], r.m[k] - 62) : 0.0;\n"
@@ -55,7 +59,7 @@ def test_root_on_the_host(tmp_path):
     f.argtypes = [ctypes.c_long] + [ctypes.c_void_p] * 8
     nk, c = np.ascontiguousarray(nk), np.ascontiguousarray(c)
     f(n, *[x.ctypes.data for x in (nl, a, nk, c, s0, ok, s, e)])
-    inside = (np.abs(c) < 150).all(axis=0) | (nl == 0)
+    inside = (np.abs(np.where(nl >> np.arange(3)[:, None] & 1, c, 0)) < 149).all(axis=0)
     assert ok[inside].mean() > 0.995  # what is near its root and in range is taken
     sel = ok == 1
     x, on = s0[sel].astype(LD), (nl[sel] >> np.arange(3)[:, None] & 1) == 1
