@@ -37,15 +37,19 @@ struct Divisor {
   unsigned long long bman;
 };
 
-// host side: the divisor as the kernels use it
-inline Divisor make_divisor(double b) {
+// the divisor as the kernels use it
+__host__ __device__ inline Divisor make_divisor(double b) {
   Divisor d;
   d.b = b;
   d.y = 1.0 / b;
   const double m = b < 0 ? -b : b;
   d.fast = (m >= 0x1p-400 && m <= 0x1p400) ? 1 : 0;
   unsigned long long bits;
+#if defined(__CUDA_ARCH__)
+  bits = fp64_bits(m);
+#else
   memcpy(&bits, &m, sizeof(bits));
+#endif
   d.eb = (int)((bits >> 52) & 0x7ffu);
   d.bman = bits & 0xfffffffffffffull;
   return d;

@@ -216,13 +216,8 @@ FX_FN uint64_t fx_log_significand(uint64_t m53) {
   return FX_TAB(logc, j) + Z + (uint64_t)fx_log1p_tail((int64_t)Z);
 }
 
-// positive normal x with |log x| >= 2^-3; CUDA's log elsewhere
-FX_FN double fx_log(double x) {
-  const uint64_t b = fx_bits(x);
-  const uint32_t hi = fx_hi(b);
-  if (hi < 0x00100000u || hi >= 0x7ff00000u) return log(x);
-  const int m = (int)(hi >> 20) - 1023;
-  const uint64_t F = fx_log_significand(fx_significand(b));
+// m ln2 + F 2^-64 as a double; false where its magnitude is below least 2^-32
+FX_FN bool fx_log_of(int m, uint64_t F, uint32_t least, double &out) {
   // m ln2 + F = m - m (1 - ln2) + F; 1 - ln2 = 0x4e8de808 2e308654 2^-64
   const int64_t p0 = (int64_t)m * 0x2e308654;
   const int64_t p1 = (int64_t)m * 0x4e8de808 + (p0 >> 32);
@@ -232,15 +227,34 @@ FX_FN double fx_log(double x) {
   const bool neg = H < 0;
   if (neg) { f = ~f; H = ~H; }  // one unit of 2^-64 off the negation
   uint32_t w2 = (uint32_t)H, w1 = fx_hi(f), w0 = fx_lo(f);
-  int e = -64 + 32;  // the value of w2:w1 in units of 2^-32
+  int e = -32;  // w2:w1 is the value in units of 2^-32
   if (w2 == 0) {
-    if (w1 < 0x20000000u) return log(x);  // |log x| < 1/8: the leading bits have cancelled
+    if (w1 < least) return false;  // the leading bits have cancelled
     w2 = w1; w1 = w0; w0 = 0; e -= 32;
   }
   const int s = fx_clz(w2);
   const uint64_t V = ((uint64_t)fx_funnel(w1, w2, s) << 32) | fx_funnel(w0, w1, s);
   const double r = fx_assemble(V, e - s);
-  return neg ? -r : r;
+  out = neg ? -r : r;
+  return true;
+}
+
+// positive normal x with |log x| >= 2^-3; CUDA's log elsewhere
+FX_FN double fx_log(double x) {
+  const uint64_t b = fx_bits(x);
+  const uint32_t hi = fx_hi(b);
+  if (hi < 0x00100000u || hi >= 0x7ff00000u) return log(x);
+  double r;
+  if (!fx_log_of((int)(hi >> 20) - 1023, fx_log_significand(fx_significand(b)), 0x20000000u, r)) return log(x);
+  return r;
+}
+
+// k ln 2 rounded to nearest, for 0 < |k| <= 1100 (checked for every such k: the bits of
+// fma(k, ln2_hi, k ln2_lo)), and 0
+FX_FN double fx_k_ln2(int k) {
+  double r = 0.0;
+  if (k != 0) fx_log_of(k, 0, 0, r);
+  return r;
 }
 
 // ---- reciprocal ----------------------------------------------------------------------------

@@ -34,8 +34,8 @@ struct OpNode {
 template <bool ANISO, bool COMPACT>
 __device__ __forceinline__ void phase_loop(const OpArgs &A, const OpNode &nd, bool has, const NodeIn &in,
                                            const NodeCtx &ctx, const AnisoNode &an, int is_centroid, double sign,
-                                           double denom, double &detadE, double &ddivpdE, double &danidE,
-                                           double *drhodP, CompactQueue *Q, int *par) {
+                                           const Divisor &denom, double &detadE, double &ddivpdE, double &danidE,
+                                           double *drhodP, CompactQueue *Q, int *par, FdLaw *laws, bool fresh) {
   for (int p = 0; p < A.M.np; p++) {
     const double vol = has ? (nd.centroid ? A.perc_n[p][nd.idx] : A.perc_s[p][nd.idx]) : 0.0;
     const bool active = fp64_abs_gt(vol, 1e-13);
@@ -46,7 +46,7 @@ __device__ __forceinline__ void phase_loop(const OpArgs &A, const OpNode &nd, bo
       IsoMid m;
       bool yields = false;
       if (active) {
-        iso_setup<FdMath>(A.M, A.ph[p], in, ctx, st, o, A.polish == 0);
+        iso_setup<FdMath>(A.M, A.ph[p], in, ctx, st, o, A.polish == 0, laws ? laws + p : nullptr, fresh);
         iso_ve<FdMath>(A.M, A.ph[p], in, ctx, st, 1.0f, A.polish, o, m);
         yields = iso_yields_dp(A.M, A.ph[p], ctx, m);
       }
@@ -60,15 +60,20 @@ __device__ __forceinline__ void phase_loop(const OpArgs &A, const OpNode &nd, bo
     }
     const double eta_vep = o.etaVE;
     const int avg = A.M.eta_average;
-    if (avg == 0) detadE += sign * vol * eta_vep / denom;
+    // the quotients by the step, correctly rounded (fp64_div.cuh)
+    const double sv = sign * vol, de = div_by(sv * eta_vep, denom);
+    if (avg == 0) detadE += de;
     else {
       const double ep = nd.centroid ? A.peta_n[p][nd.idx] : A.peta_s[p][nd.idx];
-      if (avg == 1) detadE += sign * vol * eta_vep / denom / (ep * ep);
-      else detadE += sign * vol * eta_vep / denom / ep;
+      if (avg == 1) detadE += de / (ep * ep);
+      else detadE += de / ep;
     }
-    danidE += sign * vol / denom;
-    if (is_centroid > 0) ddivpdE += sign * vol * o.div_pl / denom;
-    if (is_centroid == 2) *drhodP += sign * vol * o.rho / denom;
+    danidE += div_by(sv, denom);
+    if (is_centroid > 0) {  // a zero correction (no dilation) adds a zero
+      const double dv = sv * o.div_pl;
+      if (!(fp64_is_zero(dv) && denom.fast)) ddivpdE += div_by(dv, denom);
+    }
+    if (in.want_rho) *drhodP += div_by(sv * o.rho, denom);
   }
 }
 
@@ -86,12 +91,14 @@ __device__ __forceinline__ void fd_derivatives(const OpArgs &A, const OpNode &nd
   // the node set-up once; a strain-rate perturbation then only changes the invariant
   NodeCtx base;
   AnisoNode base_an;
+  FdLaw laws[COMPACT ? MDZ_MAX_PHASES : 1];  // of the base pressure, formed by the first perturbation
   if (has) {
     if (ANISO) node_setup_aniso<FdMath>(A.M, b, A.need_lnd != 0, base, base_an);
     else node_setup_iso<FdMath>(A.M, b, A.need_lnd != 0, base);
   }
 #pragma unroll 1
   for (int dir = 0; dir < 4; dir++) {
+    const Divisor denom = make_divisor((dir == 2 ? 4.0 : 2.0) * pert[dir]);
 #pragma unroll 1
     for (int s = 0; s < 2; s++) {
       const double sign = s == 0 ? 1.0 : -1.0;
@@ -102,8 +109,7 @@ __device__ __forceinline__ void fd_derivatives(const OpArgs &A, const OpNode &nd
       if (dir == 3) in.P = b.P + sign * pert[3];
       const int is_centroid = nd.centroid ? (dir == 3 ? 2 : 1) : 0;
       in.centroid = is_centroid;
-      in.want_rho = (is_centroid == 2);
-      const double denom = (dir == 2 ? 4.0 : 2.0) * pert[dir];
+      in.want_rho = (is_centroid == 2 && A.D[OP_DRHODP] != nullptr);
       NodeCtx ctx = base;
       AnisoNode an = base_an;
       if (has && dir < 3) {
@@ -112,7 +118,8 @@ __device__ __forceinline__ void fd_derivatives(const OpArgs &A, const OpNode &nd
         node_strain_update<FdMath>(ctx);
       }
       phase_loop<ANISO, COMPACT>(A, nd, has, in, ctx, an, is_centroid, sign, denom, d[dir],
-                                 nd.centroid ? v[dir] : vscratch, a[dir], &drhodp, Q, par);
+                                 nd.centroid ? v[dir] : vscratch, a[dir], &drhodp, Q, par,
+                                 COMPACT && dir < 3 ? laws : nullptr, !COMPACT || dir == 3 || (dir == 0 && s == 0));
     }
   }
   if (A.M.eta_average == 1)
@@ -303,9 +310,12 @@ __global__ void __launch_bounds__(128, ANISO ? 3 : 4) k_operators(const __grid_c
 // The isotropic Newton operator with its Drucker-Prager returns compacted per CTA: the
 // node loop, the 8 perturbations and the phase loop are uniform over the CTA, and the
 // returns of each phase's yielding items run packed into the first warps (dp_compact).
-// The same bits as k_operators<false, true>.  5 CTAs per SM: 103.4 ms per 2049 x 2049
-// launch against 104.9 ms at 4.
-__global__ void __launch_bounds__(128, 5) k_operators_compact(const __grid_constant__ OpArgs A) {
+// The same bits as k_operators<false, true>.  Per perturbed solve it takes about 100 FP64
+// instructions (149 before the convergence test of the default start moved to fixed point,
+// the quotients by the step to the known-divisor form, and the strain-rate-independent part
+// of the laws out of the strain-rate perturbations: 513 x 513 cells 6.98 -> 5.44 ms).  CTAs
+// per SM: 5.59, 5.44 and 5.41 ms at 5, 6 and 8.
+__global__ void __launch_bounds__(128, 6) k_operators_compact(const __grid_constant__ OpArgs A) {
   __shared__ CompactQueue Q;
   compact_init(Q);
   int par = 0;

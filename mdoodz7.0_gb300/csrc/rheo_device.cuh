@@ -281,9 +281,18 @@ struct Laws {
 template <class FP>
 __device__ __forceinline__ double law_inv(const Laws &L, int k) { return FP::exp(L.ln_inv[k]); }
 
+//
+// What of a phase's laws does not depend on the strain rate: the operators' strain-rate
+// perturbations form it once per node and phase (the same operations, so the same bits).
+struct FdLaw {
+  double lnB_pwl, lnB_lin, lnBd, ST, nE, lnA, Tyield;
+};
+
+// fd (operators only; may be null): filled where `fresh`, taken from it where not
 template <class FP>
 __device__ __forceinline__ void creep_laws(const ModelConst &M, const PhaseConst &ph, const NodeCtx &c, double P,
-                                           double phi, double lnd, int peierls, Laws &L) {
+                                           double phi, double lnd, int peierls, Laws &L, FdLaw *fd = nullptr,
+                                           bool fresh = true) {
   const int fl = ph.flags;
   L.mech = (fl & (F_CST | F_PWL | F_LIN | F_GBS | F_PWL1 | F_LIN1)) | (peierls ? F_EXPV : 0);
   L.ln_inv[0] = L.ln_inv[1] = L.ln_inv[2] = -kInf;
@@ -314,32 +323,48 @@ __device__ __forceinline__ void creep_laws(const ModelConst &M, const PhaseConst
       L.ln_inv[K_EXP] = (ph.exp_ln2s + lnEii) - FP::quotient(lnEii - L.lnA_exp, nE);
     }
   } else {
-  if (fl & F_PWL) {
-    // B = pref F A^(-1/n) exp((Q+PV)/(RnT)) d^(m/n) f^(-r/n) exp(-a phi/n);
-    // 1/eta_pwl = Eii^(1-1/n) / B:  ln(1/eta_pwl) = lnEii - lnEii/n - lnB
-    double lnB = ph.pwl_lnK + (ph.pwl_Q + P * ph.pwl_V) * ph.pwl_invRn * c.invT;
-    if (fl & F_PWL_M) lnB += ph.pwl_mn * lnd;
-    if (fl & F_PWL_A) lnB -= ph.pwl_an * phi;
-    L.lnB_pwl = lnB;
-    L.ln_inv[K_PWL] = lnEii - fma(lnEii, ph.pwl_invn, lnB);
-  }
-  if (fl & F_LIN) {
-    // 1/eta_lin = Eii^(1-1/n) / (B d^(m/n))
-    double lnB = ph.lin_lnK + (ph.lin_Q + P * ph.lin_V) * ph.lin_invRn * c.invT;
-    if (fl & F_LIN_A) lnB -= ph.lin_an * phi;
-    L.lnB_lin = lnB;
-    const double lnBd = (fl & F_LIN_M) ? fma(ph.lin_mn, lnd, lnB) : lnB;
-    L.ln_inv[K_LIN] = lnEii - fma(lnEii, ph.lin_invn, lnBd);
-  }
-  if (peierls) {
-    // Eii_exp(Tii) = A (sqrt3 Tii / (gamma S))^nE, A = (sqrt3/2) E Arr (gamma S)^n;
-    // isolated: Tii* = (gamma S / sqrt3) (Eii/A)^(1/nE), 1/eta_exp = 2 Eii / Tii*
-    L.ST = ph.exp_EaR * c.invT * ph.exp_g2;
-    const double nE = L.ST + ph.exp_n;
-    L.n[K_EXP] = nE;
-    L.lnA_exp = ph.exp_lnA0 - ph.exp_EaR * ph.exp_om2 * c.invT;
-    L.ln_inv[K_EXP] = (kLn2 + ph.exp_ln_s3gS + lnEii) - FP::quotient(lnEii - L.lnA_exp, nE);
-  }
+    if (fl & F_PWL) {
+      // B = pref F A^(-1/n) exp((Q+PV)/(RnT)) d^(m/n) f^(-r/n) exp(-a phi/n);
+      // 1/eta_pwl = Eii^(1-1/n) / B:  ln(1/eta_pwl) = lnEii - lnEii/n - lnB
+      if (fresh) {
+        double lnB = ph.pwl_lnK + (ph.pwl_Q + P * ph.pwl_V) * ph.pwl_invRn * c.invT;
+        if (fl & F_PWL_M) lnB += ph.pwl_mn * lnd;
+        if (fl & F_PWL_A) lnB -= ph.pwl_an * phi;
+        L.lnB_pwl = lnB;
+        if (fd) fd->lnB_pwl = lnB;
+      } else {
+        L.lnB_pwl = fd->lnB_pwl;
+      }
+      L.ln_inv[K_PWL] = lnEii - fma(lnEii, ph.pwl_invn, L.lnB_pwl);
+    }
+    if (fl & F_LIN) {
+      // 1/eta_lin = Eii^(1-1/n) / (B d^(m/n))
+      double lnBd;
+      if (fresh) {
+        double lnB = ph.lin_lnK + (ph.lin_Q + P * ph.lin_V) * ph.lin_invRn * c.invT;
+        if (fl & F_LIN_A) lnB -= ph.lin_an * phi;
+        L.lnB_lin = lnB;
+        lnBd = (fl & F_LIN_M) ? fma(ph.lin_mn, lnd, lnB) : lnB;
+        if (fd) { fd->lnB_lin = lnB; fd->lnBd = lnBd; }
+      } else {
+        L.lnB_lin = fd->lnB_lin;
+        lnBd = fd->lnBd;
+      }
+      L.ln_inv[K_LIN] = lnEii - fma(lnEii, ph.lin_invn, lnBd);
+    }
+    if (peierls) {
+      // Eii_exp(Tii) = A (sqrt3 Tii / (gamma S))^nE, A = (sqrt3/2) E Arr (gamma S)^n;
+      // isolated: Tii* = (gamma S / sqrt3) (Eii/A)^(1/nE), 1/eta_exp = 2 Eii / Tii*
+      if (fresh) {
+        L.ST = ph.exp_EaR * c.invT * ph.exp_g2;
+        L.n[K_EXP] = L.ST + ph.exp_n;
+        L.lnA_exp = ph.exp_lnA0 - ph.exp_EaR * ph.exp_om2 * c.invT;
+        if (fd) { fd->ST = L.ST; fd->nE = L.n[K_EXP]; fd->lnA = L.lnA_exp; }
+      } else {
+        L.ST = fd->ST; L.n[K_EXP] = fd->nE; L.lnA_exp = fd->lnA;
+      }
+      L.ln_inv[K_EXP] = (kLn2 + ph.exp_ln_s3gS + lnEii) - FP::quotient(lnEii - L.lnA_exp, L.n[K_EXP]);
+    }
   }
   if (fl & F_GBS) {
     double lnB = ph.gbs_lnK + (ph.gbs_Q + P * ph.gbs_V) * ph.gbs_invRn * c.invT - ph.gbs_an * phi;
@@ -360,8 +385,7 @@ __device__ __forceinline__ void creep_laws(const ModelConst &M, const PhaseConst
 // eta_n = 2^k and its logarithm
 __device__ __forceinline__ void pow2_normalisation(int k, double &eta_n, double &ln_eta_n) {
   eta_n = __hiloint2double((k + 1023) << 20, 0);
-  const double kd = __hiloint2double(0x43300000, k ^ (int)0x80000000) - 4503601774854144.0;  // (double)k
-  ln_eta_n = fma(kd, MDZ_LN2_HI, kd * MDZ_LN2_LO);
+  ln_eta_n = fx_k_ln2(k);
 }
 
 // Inputs of the general (FP64) form of the local solve: any start, any normalisation.
@@ -381,14 +405,13 @@ __device__ __forceinline__ void ve_args(VeArgs &v, const Laws &L, const NodeCtx 
 }
 
 struct VeCoef {
-  double Eii, thr_conv, thr_fail;  // Eii * tol/100, Eii * tol
+  double Eii, thr_conv;            // Eii * tol/100
   double inv_Eii;                  // 1 / Eii
   double eta_up;                   // eta = s eta_up
   double Aup;                      // eta_up x the sum of the linear coefficients (el, cst, Newtonian laws)
   double a_cst, a_lin1, a_pwl1;    // e_cst = eta a_cst, e_lin = eta a_lin1 (n_lin==1), e_pwl = eta a_pwl1 (n_pwl==1)
   double lp;                       // ln(eta_up / eta_p)
   double n[K_COUNT], nc[K_COUNT];  // exponent and n_k * ln(eta_p / eta_k) per non-linear law
-  double hn[K_COUNT];              // (n_k - 1) / 2
   double nmax;                     // largest exponent of the non-linear laws (0 without)
   int nl;                          // bit k: law k is non-linear and active
 };
@@ -415,7 +438,6 @@ __device__ __forceinline__ void ve_coef(const VeArgs &v, VeCoef &q) {
   q.Eii = Eii;
   q.inv_Eii = 2.0 * v.inv2Eii;
   q.thr_conv = Eii * (tol / 100);
-  q.thr_fail = Eii * tol;
   q.eta_up = eta_up;
   q.a_cst = (L.mech & F_CST) ? Eii / eta_cst : 0.0;
   double A = (v.elastic ? Eii * v.inv_eta_el : 0.0) + q.a_cst;
@@ -444,7 +466,6 @@ __device__ __forceinline__ void ve_coef(const VeArgs &v, VeCoef &q) {
   q.nmax = 0.0;
 #pragma unroll
   for (int k = 0; k < K_COUNT; k++) {
-    q.hn[k] = 0.5 * (q.n[k] - 1.0);
     if (q.nl >> k & 1) q.nmax = fp64_fmax(q.nmax, q.n[k]);
     if ((q.nl >> k & 1) && k != p) q.nc[k] = q.n[k] * (L.ln_inv[k] - ln_inv_p);
   }
@@ -465,7 +486,7 @@ __device__ __forceinline__ void ve_eval(const VeCoef &q, double sv, VeState &s, 
     for (int k = 0; k < K_COUNT; k++)
       if (q.nl >> k & 1) {
         const double t = step * q.n[k];
-        e[k] = fma(e[k] * t, fma(step, q.hn[k], 1.0), e[k]);
+        e[k] = fma(e[k] * t, fma(step, 0.5 * (q.n[k] - 1.0), 1.0), e[k]);
       }
   } else {
     e[0] = e[1] = e[2] = 0.0;
@@ -517,7 +538,7 @@ __device__ __forceinline__ void ve_newton(const VeCoef &q, double sv, VeState &s
       it = -1;
       continue;
     }
-    if (it == nitmax - 1 && fabs(r) > q.thr_fail) { set_status(s.status, MDZ_EVE_ITER); break; }
+    if (it == nitmax - 1 && fabs(r) > q.Eii * 1.0e-11) { set_status(s.status, MDZ_EVE_ITER); break; }
     const double d = FP::newton_quotient(r, fma(q.Aup, sv, ve_S(q, s)));
     sv = fma(sv, d, sv);
     step = fp64_lt(fabs(d) * q.nmax, 1e-5) ? d : -1.0;
@@ -726,11 +747,55 @@ __device__ __forceinline__ bool ve_solve_fx(const PhaseConst &ph, const Laws &L,
   return true;
 }
 
+// Whether the normalised residual at sv is below 7e-14, formed in fixed point (ve_fx.cuh).
+// The reference's test, |r| < 1e-13 Eii on the FP64 residual, then holds too: the two forms
+// differ by their rounding, at most n ulp of a law's argument, a few 1e-15.  false also where
+// a number leaves the fixed-point formats.
+__device__ __forceinline__ bool ve_converged_fx(const VeCoef &q, const StartCoef &sc, double sv) {
+  int64_t N[K_COUNT], C[K_COUNT];
+  int nl = 0;
+  if (q.nl) {
+#pragma unroll
+    for (int k = 0; k < K_COUNT; k++)
+      if (q.nl >> k & 1) {
+        const uint64_t nb = fx_bits(q.n[k]), cb = fx_bits(sc.c[k]);
+        if (fx_hi(nb) >= 0x40600000u) return false;                     // 0 <= n < 128
+        if (fx_hi(cb) >= 0xc062a000u && fx_hi(cb) < 0xfff00000u) continue;  // c < -149: no effect on the test
+        if ((fx_hi(cb) & 0x7fffffffu) >= 0x4062a000u) return false;
+        N[k] = fx_fixed<56>(nb);
+        C[k] = fx_fixed<54>(cb);
+        nl |= 1 << k;
+      }
+  }
+  int64_t R;
+  return ve_residual_fx(nl, sc.a, N, C, sv, R) && R < 322818 && R > -322818;  // 7e-14 2^62
+}
+
 // LocalIterationViscoElastic from the start that `polish` names
 template <class FP>
 __device__ __forceinline__ void ve_general_inl(const VeArgs &v, VeState &s, int &f32_steps) {
   VeCoef q;
   ve_coef<FP>(v, q);
+  if (!FP::kFixed && start_dd(v.polish)) {
+    // The operators' perturbed solves use the converged viscosity alone.  From this start
+    // nearly every FP64 iteration stops at its first evaluation: the fixed-point residual
+    // tells so without the evaluation's logarithm and exponentials, and the viscosity is the
+    // one that iteration returns, bit for bit.  Where it does not, the iteration runs.
+    StartCoef sc;
+    start_coef(q, sc);
+    f32_steps = 0;
+    const float s0 = ve_polish_f32(q, sc, v.s_start * v.s_up, start_fp32(v.polish), f32_steps, v.s_up);
+    const double sv = ve_halley_dd(q, sc, s0, v.s_up);
+    if (ve_converged_fx(q, sc, sv)) {
+      s.eta = sv * q.eta_up;
+      s.Tii = fp64_scale(s.eta * q.Eii, 1);
+      s.e_cst = s.e_pwl = s.e_exp = s.e_lin = 0.0;
+      s.iters = 1;
+    } else {
+      ve_newton<FP>(q, sv, s, v.s_up, true);
+    }
+    return;
+  }
   ve_newton<FP>(q, ve_start(q, v.s_start * v.s_up, start_fp32(v.polish), start_dd(v.polish), f32_steps, v.s_up), s,
                 v.s_up, v.polish != 0);
 }
@@ -1039,7 +1104,8 @@ __device__ __forceinline__ double lower_viscosity(const ModelConst &M, const Law
 // exact: the local solve starts where the reference's does (start descriptor 0)
 template <class FP>
 __device__ inline void iso_setup(const ModelConst &M, const PhaseConst &ph, const NodeIn &in, const NodeCtx &c,
-                                 IsoState &S, PointOut &o, bool exact = true) {
+                                 IsoState &S, PointOut &o, bool exact = true, FdLaw *fd = nullptr,
+                                 bool fresh = true) {
   const int fl = ph.flags;
   const int constant = (fl & F_CST) != 0, diffusion = (fl & F_LIN) != 0, gs = (fl & F_GS) != 0;
   const int peierls = ((fl & F_EXPV) != 0) && c.cold;
@@ -1064,10 +1130,13 @@ __device__ inline void iso_setup(const ModelConst &M, const PhaseConst &ph, cons
   if (c.d_zero && diffusion && fp64_gt(ph.lin_m, 0.0)) set_status(o.status, MDZ_EGRAIN_ZERO);
 
   Laws &L = S.L;
-  creep_laws<FP>(M, ph, c, P, in.phi, c.lnd, peierls, L);
+  creep_laws<FP>(M, ph, c, P, in.phi, c.lnd, peierls, L, fd, fresh);
   double Tyield = 0.0, C = in.C;
   if (plastic == 1) {  // :530-539 (the operators perturb P after the node's set-up)
-    Tyield = FP::kFixed ? c.Tyield : __dadd_rn(__dmul_rn(C, c.cos_fric), __dmul_rn(P, c.sin_fric));
+    if (FP::kFixed) Tyield = c.Tyield;
+    else if (!fresh) Tyield = fd->Tyield;
+    else Tyield = __dadd_rn(__dmul_rn(C, c.cos_fric), __dmul_rn(P, c.sin_fric));
+    if (fd && fresh) fd->Tyield = Tyield;
     if ((fl & F_SLIM) ? fp64_gt_pos(Tyield, ph.Slim) : fp64_lt(ph.Slim, Tyield)) { C = ph.Slim; Tyield = ph.Slim; }
   }
   double eta_cst = 0.0, Ag = 0.0, lnd = c.lnd;
@@ -1295,9 +1364,8 @@ __device__ inline void iso_post(const ModelConst &M, const PhaseConst &ph, const
   if (in.centroid > 0 && in.want_rho) o.rho = density(M, ph, T, (in.final_update == 1) ? Pc : P, in.X0, in.phi);
 
   double inv_eta_pl = 0.0;
-  if (is_pl == 0) o.etaVE = eta_ve;
-  else if (plastic == 1) { o.etaVE = eta_vep; inv_eta_pl = FP::quotient(gdot, Tii); }
-  else { o.etaVE = eta_vep; inv_eta_pl = 2.0 * lam_dot * A_tau / Tii; }
+  o.etaVE = is_pl == 0 ? eta_ve : eta_vep;
+  if (is_pl && in.post_process != 0) inv_eta_pl = plastic == 1 ? FP::quotient(gdot, Tii) : 2.0 * lam_dot * A_tau / Tii;
   o.is_pl = is_pl;
   if (is_pl) o.mech |= MDZ_MECH_YIELD;
   o.Eii_cst = e_cst; o.Eii_pwl = e_pwl; o.Eii_exp = e_exp; o.Eii_lin = e_lin;
@@ -1558,7 +1626,7 @@ __device__ __forceinline__ void aniso_general_inl(const ModelConst &M, const VeA
       continue;
     }
     if (it == 49 && ar < 10.0 * tol * Eii) break;
-    if (it == 49 && ar > q.thr_fail) { set_status(s.status, MDZ_EANISO_ITER); break; }
+    if (it == 49 && ar > Eii * tol) { set_status(s.status, MDZ_EANISO_ITER); break; }
   }
   s.eta = sv * q.eta_up;
 }

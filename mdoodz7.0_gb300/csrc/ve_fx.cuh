@@ -150,4 +150,30 @@ FX_FN bool ve_root_fx(int nl, double a, const int64_t *N, const int64_t *C, cons
   return ok;
 }
 
+// The residual r(sv) in Q2.62, for a double sv in [2^-4, 2); nl, a, N, C as above.  false
+// where a number leaves its format.
+FX_FN bool ve_residual_fx(int nl, double a, const int64_t *N, const int64_t *C, double sv, int64_t &R) {
+  const uint64_t sb = fx_bits(sv), ab = fx_bits(a);
+  const int e0 = (int)(fx_hi(sb) >> 20) - 1023, ea = (int)(fx_hi(ab) >> 20) - 1023;  // sv > 0, a >= 0
+  const int shift = -(ea + e0);
+  if (e0 > 0 || e0 < -4 || shift < 0) return false;
+  const uint64_t m53 = fx_significand(sb);
+  const uint64_t A0 = fx_mul64hi(fx_significand(ab) << 11, m53 << 11) >> (shift > 63 ? 63 : shift);
+  bool ok = (int64_t)A0 >= 0;
+  R = (int64_t)0x4000000000000000ll - (int64_t)A0;
+  if (nl) {
+    const int64_t L = (int64_t)(fx_log_significand(m53) >> 4) + (int64_t)e0 * 0xb17217f7d1cf79all;
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+      if (nl >> k & 1) {
+        const int64_t X = fx_mul_nl(N[k], L) + C[k];
+        ok = ok && (int32_t)(X >> 32) < 2516582;  // X < 0.6
+        int m;
+        const uint64_t M = fx_exp_core(X, m);
+        R -= (int64_t)(M >> (-m > 63 ? 63 : -m));
+      }
+  }
+  return ok;
+}
+
 }  // namespace mdz

@@ -79,3 +79,19 @@ def test_host_build(tmp_path):
 def test_gpu():
     x = arguments()
     check(x, R.fx_selftest(x))
+
+
+def test_k_ln2_on_the_host(tmp_path):
+    """k ln 2 for every k that a normalisation can have: the bits of the FP64 form it stands in for (a product and a
+    fused multiply-add with ln 2 in two parts), here in exact rational arithmetic."""
+    from fractions import Fraction
+    src = tmp_path / "k.cpp"
+    src.write_text('#include "fx64.cuh"\nextern "C" double k_ln2(int k) { return mdz::fx_k_ln2(k); }\n')
+    lib = tmp_path / "k.so"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-I", R.HERE + "/csrc", str(src), "-o", str(lib)],
+                   check=True, capture_output=True)
+    f = ctypes.CDLL(str(lib)).k_ln2
+    f.restype = ctypes.c_double
+    hi, lo = float.fromhex("0x1.62e42fefa39efp-1"), float.fromhex("0x1.abc9e3b39803fp-56")
+    for k in range(-1100, 1101):
+        assert f(k) == float(Fraction(k) * Fraction(hi) + Fraction(k * lo)), k
