@@ -45,8 +45,9 @@ __device__ __forceinline__ void phase_loop(const OpArgs &A, const OpNode &nd, bo
       IsoState st;
       IsoMid m;
       bool yields = false;
+      const bool kept = laws && p < kFdPhases && !(A.ph[p].flags & F_GS);
       if (active) {
-        iso_setup<FdMath>(A.M, A.ph[p], in, ctx, st, o, A.polish == 0, laws ? laws + p : nullptr, fresh);
+        iso_setup<FdMath>(A.M, A.ph[p], in, ctx, st, o, A.polish == 0, kept ? laws + p : nullptr, fresh || !kept);
         iso_ve<FdMath>(A.M, A.ph[p], in, ctx, st, 1.0f, A.polish, o, m);
         yields = iso_yields_dp(A.M, A.ph[p], ctx, m);
       }
@@ -61,19 +62,19 @@ __device__ __forceinline__ void phase_loop(const OpArgs &A, const OpNode &nd, bo
     const double eta_vep = o.etaVE;
     const int avg = A.M.eta_average;
     // the quotients by the step, correctly rounded (fp64_div.cuh)
-    const double sv = sign * vol, de = div_by(sv * eta_vep, denom);
+    const double sv = sign * vol, de = div_by_fp64(sv * eta_vep, denom);
     if (avg == 0) detadE += de;
     else {
       const double ep = nd.centroid ? A.peta_n[p][nd.idx] : A.peta_s[p][nd.idx];
       if (avg == 1) detadE += de / (ep * ep);
       else detadE += de / ep;
     }
-    danidE += div_by(sv, denom);
+    danidE += div_by_fp64(sv, denom);
     if (is_centroid > 0) {  // a zero correction (no dilation) adds a zero
       const double dv = sv * o.div_pl;
-      if (!(fp64_is_zero(dv) && denom.fast)) ddivpdE += div_by(dv, denom);
+      if (!(fp64_is_zero(dv) && denom.fast)) ddivpdE += div_by_fp64(dv, denom);
     }
-    if (in.want_rho) *drhodP += div_by(sv * o.rho, denom);
+    if (in.want_rho) *drhodP += div_by_fp64(sv * o.rho, denom);
   }
 }
 
@@ -91,7 +92,7 @@ __device__ __forceinline__ void fd_derivatives(const OpArgs &A, const OpNode &nd
   // the node set-up once; a strain-rate perturbation then only changes the invariant
   NodeCtx base;
   AnisoNode base_an;
-  FdLaw laws[COMPACT ? MDZ_MAX_PHASES : 1];  // of the base pressure, formed by the first perturbation
+  FdLaw laws[COMPACT ? kFdPhases : 1];  // of the base pressure, formed by the first perturbation
   if (has) {
     if (ANISO) node_setup_aniso<FdMath>(A.M, b, A.need_lnd != 0, base, base_an);
     else node_setup_iso<FdMath>(A.M, b, A.need_lnd != 0, base);

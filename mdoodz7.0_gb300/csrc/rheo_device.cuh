@@ -283,9 +283,12 @@ __device__ __forceinline__ double law_inv(const Laws &L, int k) { return FP::exp
 
 //
 // What of a phase's laws does not depend on the strain rate: the operators' strain-rate
-// perturbations form it once per node and phase (the same operations, so the same bits).
+// perturbations form it once per node and phase (the same operations, so the same bits), for
+// the first kFdPhases phases without a grain-size solve (which needs more): 200 bytes of the
+// thread's stack, which keep it at the sweep kernels' size.
+constexpr int kFdPhases = 5;
 struct FdLaw {
-  double lnB_pwl, lnB_lin, lnBd, ST, nE, lnA, Tyield;
+  double lnB_pwl, lnBd, nE, lnA, Tyield;
 };
 
 // fd (operators only; may be null): filled where `fresh`, taken from it where not
@@ -345,9 +348,8 @@ __device__ __forceinline__ void creep_laws(const ModelConst &M, const PhaseConst
         if (fl & F_LIN_A) lnB -= ph.lin_an * phi;
         L.lnB_lin = lnB;
         lnBd = (fl & F_LIN_M) ? fma(ph.lin_mn, lnd, lnB) : lnB;
-        if (fd) { fd->lnB_lin = lnB; fd->lnBd = lnBd; }
+        if (fd) fd->lnBd = lnBd;
       } else {
-        L.lnB_lin = fd->lnB_lin;
         lnBd = fd->lnBd;
       }
       L.ln_inv[K_LIN] = lnEii - fma(lnEii, ph.lin_invn, lnBd);
@@ -359,9 +361,9 @@ __device__ __forceinline__ void creep_laws(const ModelConst &M, const PhaseConst
         L.ST = ph.exp_EaR * c.invT * ph.exp_g2;
         L.n[K_EXP] = L.ST + ph.exp_n;
         L.lnA_exp = ph.exp_lnA0 - ph.exp_EaR * ph.exp_om2 * c.invT;
-        if (fd) { fd->ST = L.ST; fd->nE = L.n[K_EXP]; fd->lnA = L.lnA_exp; }
+        if (fd) { fd->nE = L.n[K_EXP]; fd->lnA = L.lnA_exp; }
       } else {
-        L.ST = fd->ST; L.n[K_EXP] = fd->nE; L.lnA_exp = fd->lnA;
+        L.n[K_EXP] = fd->nE; L.lnA_exp = fd->lnA;
       }
       L.ln_inv[K_EXP] = (kLn2 + ph.exp_ln_s3gS + lnEii) - FP::quotient(lnEii - L.lnA_exp, L.n[K_EXP]);
     }
