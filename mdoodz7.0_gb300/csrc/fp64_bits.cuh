@@ -94,11 +94,10 @@ __device__ __forceinline__ bool fp64_le(double a, double b) {
 __device__ __forceinline__ bool fp64_gt(double a, double b) { return fp64_lt(b, a); }
 __device__ __forceinline__ bool fp64_ge(double a, double b) { return fp64_le(b, a); }
 
-// |x| < t, IEEE, for any x and t
+// |x| < t, IEEE, for any x and t: false for a negative t or a NaN on either side
 __device__ __forceinline__ bool fp64_abs_lt(double x, double t) {
   const unsigned long long ax = fp64_bits(x) & kFp64AbsMask, bt = fp64_bits(t);
-  if (ax > kFp64InfBits || (bt & kFp64AbsMask) > kFp64InfBits) return false;
-  return fp64_key_of_bits(ax) < fp64_key_of_bits(bt);
+  return ax < bt && bt <= kFp64InfBits;
 }
 // |x| > t, IEEE, for any x and t
 __device__ __forceinline__ bool fp64_abs_gt(double x, double t) {

@@ -590,7 +590,7 @@ __global__ void __launch_bounds__(256) k_p2m_scatter(const MarkerArgs A) {
   if (ph < 0 || ph >= A.np) { report(A, k, MDZ_EINVAL); return; }
   const double x = A.x[k], z = A.z[k];
   double v = A.val[k];
-  if (A.avg == 1) v = 1.0 / v;
+  if (A.avg == 1) v = recip_rn(v);
   else if (A.avg == 2) v = log(v);
   if (A.out_n) {
     const int Ncx = A.Nx - 1, Ncz = A.Nz - 1;

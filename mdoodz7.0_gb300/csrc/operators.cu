@@ -51,7 +51,7 @@ __device__ __forceinline__ void phase_loop(const OpArgs &A, const OpNode &nd, bo
         iso_ve<FdMath>(A.M, A.ph[p], in, ctx, st, 1.0f, A.polish, o, m);
         yields = iso_yields_dp(A.M, A.ph[p], ctx, m);
       }
-      dp_compact<false>(A.M, A.ph[p], *Q, *par, yields, m, in, ctx);
+      dp_compact(A.M, A.ph[p], *Q, *par, yields, m, in, ctx);
       if (!active) continue;
       iso_post<FdMath>(A.M, A.ph[p], in, ctx, st, o, m);
     } else if (ANISO) {

@@ -1256,9 +1256,43 @@ __device__ inline void dp_return(const ModelConst &M, const PhaseConst &ph, DpIt
   d.Tii = Tiic;
 }
 
-__device__ __forceinline__ void dp_extra(DpItem &d) {
+// The Drucker-Prager return of a sweep's item, in its own thread.  Without dilation and with a
+// linear viscoplastic term (n_vp = 1) the iteration stops at its first pass but for rounding;
+// that pass is written out here, with one reciprocal for the rate and the powers, and the
+// iteration itself (dp_return) runs out of line where it does not.  While the return took
+// some 40 FP64 instructions it was worth gathering the yielding items of a CTA into its first
+// warps; at 9 the barriers cost more than the idle lanes: 2049 x 2049 sweep 7.70 -> 7.52 ms,
+// 201 x 201 80 -> 71 us, 16-grid batch 6.60 -> 5.74 ms.
+static __device__ __noinline__ DpItem dp_return_call(const ModelConst &M, const PhaseConst &ph, DpItem d) {
+  dp_return(M, ph, d);
   d.pl_share = d.eta_ve * d.gdot * fx_recip_call(d.Tii);
   d.T_over_eta = d.Tii * fx_recip_call(d.eta_ve);
+  return d;
+}
+
+__device__ __forceinline__ void dp_return_inline(const ModelConst &M, const PhaseConst &ph, const NodeIn &in,
+                                                 const NodeCtx &c, IsoMid &m) {
+  if ((ph.flags & F_VP1) && fp64_is_zero(c.sin_dil)) {
+    const bool rigid = fp64_is_zero(ph.eta_vp);
+    // rounded one by one: the same bits in every kernel
+    const double F = __dsub_rn(m.Tii, m.Tyield);
+    const double rD = fx_recip_call(rigid ? m.eta_ve : __dadd_rn(m.eta_ve, ph.eta_vp));
+    const double gdot = __dmul_rn(F, rD), drop = __dmul_rn(m.eta_ve, gdot), Tii = __dsub_rn(m.Tii, drop);
+    const double Tyield = rigid ? m.Tyield : __fma_rn(gdot, ph.eta_vp, m.Tyield);
+    const double F1 = __dsub_rn(Tii, Tyield);
+    if ((fp64_abs_lt(F1, M.eta_tol) || fp64_abs_lt(F1, __dmul_rn(M.eta_tol, F))) && (int)fp64_hi(Tii) >= 0) {
+      m.is_pl = 1;
+      m.gdot = gdot; m.divp = 0.0; m.Pc = in.P; m.eta_vp = ph.eta_vp; m.Tyield = Tyield; m.Tii = Tii;
+      m.eta_vep = __dmul_rn(Tii, c.inv2Eii);
+      m.pl_share = __dmul_rn(drop, fx_recip_call(Tii));
+      m.T_over_eta = __dmul_rn(Tii, rigid ? rD : fx_recip_call(m.eta_ve));
+      return;
+    }
+  }
+  DpItem d;
+  dp_load(d, m, in, c);
+  d = dp_return_call(M, ph, d);
+  dp_store(m, d);
 }
 
 // Local solve (from s_start * eta_up, moved by the start stages that the descriptor
@@ -1438,10 +1472,14 @@ __device__ inline void iso_finish(const ModelConst &M, const PhaseConst &ph, con
   IsoMid m;
   iso_ve<FP>(M, ph, in, c, S, s_start, polish, o, m, eta_conv);
   if (iso_yields_dp(M, ph, c, m)) {
-    DpItem d;
-    dp_load(d, m, in, c);
-    dp_return(M, ph, d);
-    dp_store(m, d);
+    if (FP::kFixed) {
+      dp_return_inline(M, ph, in, c, m);
+    } else {
+      DpItem d;
+      dp_load(d, m, in, c);
+      dp_return(M, ph, d);
+      dp_store(m, d);
+    }
   }
   iso_post<FP>(M, ph, in, c, S, o, m);
 }
@@ -1475,7 +1513,6 @@ __device__ __forceinline__ void compact_init(CompactQueue &Q) {
 
 // par: the phase parity, flipped here.  count[par ^ 1] is cleared between the two
 // barriers, where no thread touches it; count[par] is read only between them.
-template <bool EXTRA>
 __device__ __forceinline__ void dp_compact(const ModelConst &M, const PhaseConst &ph, CompactQueue &Q, int &par,
                                            bool yields, IsoMid &m, const NodeIn &in, const NodeCtx &c) {
   const int t = threadIdx.x, lane = t & 31;
@@ -1490,7 +1527,6 @@ __device__ __forceinline__ void dp_compact(const ModelConst &M, const PhaseConst
   if (t < q) {
     DpItem d = Q.item[t];
     dp_return(M, ph, d);
-    if (EXTRA) dp_extra(d);
     Q.item[t] = d;
   }
   __syncthreads();

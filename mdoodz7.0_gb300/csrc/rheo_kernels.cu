@@ -71,24 +71,6 @@ __global__ void __launch_bounds__(128, 6) k_sweep_queue(const __grid_constant__ 
   flush_acc(A.stats, acc);
 }
 
-template <int NODES>
-__global__ void __launch_bounds__(128, 6) k_sweep_compact(const __grid_constant__ SweepArgs A) {
-  if (NODES == 1) pair_begin();
-  __shared__ CompactQueue Q;
-  compact_init(Q);
-  Acc acc = {0, 0, 0, 0, 0};
-  const long long total = NODES == 1 ? (A.ranged ? A.c_n : A.M.Nc) : (A.ranged ? A.v_n : A.M.Nv);
-  const long long lo = NODES == 1 ? (A.ranged ? A.c_lo : 0) : A.M.Nc + (A.ranged ? A.v_lo : 0);
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  int par = 0;
-  for (long long base = (long long)blockIdx.x * blockDim.x; base < total; base += stride) {  // uniform
-    const long long j = base + threadIdx.x;
-    compact_node<NODES, false>(A, j < total, lo + j, acc, Q, par);
-  }
-  flush_acc(A.stats, acc);
-  if (NODES == 2) pair_end();
-}
-
 // ---------------------------------------------------------------------------------
 // independent points: ViscosityConcise / ViscosityConciseAniso
 // ---------------------------------------------------------------------------------
@@ -163,12 +145,9 @@ static cudaError_t launch_kind(const SweepArgs &a, const LaunchShape &sh, long l
     k_sweep_queue<ANISO, NODES><<<(unsigned)sh.grid_cap, 128, 0, s>>>(a);
     return cudaGetLastError();
   }
-  const int block = (!ANISO && sh.form == SHAPE_COMPACT) ? 128 : sh.block;
+  const int block = sh.form == SHAPE_COMPACT ? 128 : sh.block;  // SHAPE_COMPACT: the default, one thread per node
   long long grid = (count + block - 1) / block;
   if (sh.grid_cap > 0 && grid > sh.grid_cap) grid = sh.grid_cap;
-  if constexpr (!ANISO)
-    if (sh.form == SHAPE_COMPACT)  // the isotropic sweep only
-      return launch_after(k_sweep_compact<NODES>, (unsigned)grid, block, s, after, a);
   if (sh.form == SHAPE_REGS255) return launch_after(k_sweep<ANISO, NODES, 2>, (unsigned)grid, block, s, after, a);
   return launch_after(k_sweep<ANISO, NODES, 6>, (unsigned)grid, block, s, after, a);
 }
@@ -205,7 +184,6 @@ void sweep_kernel_info(int aniso, int *regs, int *smem, int *max_blocks_per_sm, 
   const void *fn = aniso ? (const void *)k_sweep<true, 1, 6> : (const void *)k_sweep<false, 1, 6>;
   if (form == SHAPE_REGS255) fn = aniso ? (const void *)k_sweep<true, 1, 2> : (const void *)k_sweep<false, 1, 2>;
   if (form == SHAPE_QUEUE) fn = aniso ? (const void *)k_sweep_queue<true, 1> : (const void *)k_sweep_queue<false, 1>;
-  if (form == SHAPE_COMPACT && !aniso) fn = (const void *)k_sweep_compact<1>;
   cudaFuncGetAttributes(&fa, fn);
   *regs = fa.numRegs;
   *smem = (int)fa.sharedSizeBytes;

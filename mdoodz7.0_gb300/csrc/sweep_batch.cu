@@ -39,32 +39,16 @@ __global__ void __launch_bounds__(kBatchTile, 6) k_sweep_batch(const __grid_cons
   Acc acc = {0, 0, 0, 0, 0};
   const long long *ts = NODES == 1 ? B.tile_start_n : B.tile_start_s;
   const long long tiles = NODES == 1 ? B.tiles_n : B.tiles_s;
-  [[maybe_unused]] int par = 0;
-  if constexpr (!ANISO) {
-    __shared__ CompactQueue Q;
-    compact_init(Q);
-    for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {  // uniform over the CTA
-      const int g = batch_grid_of(ts, B.n, t);
-      const SweepArgs &A = B.grids[g];
-      const long long j = (t - __ldg(&ts[g])) * kBatchTile + threadIdx.x;
-      const bool valid = j < (NODES == 1 ? A.M.Nc : A.M.Nv);
-      const long long i = NODES == 1 ? j : A.M.Nc + j;
-      PerturbKey pk;
-      if (PERTURB) { pk.key = perturb_key(X.seed, X.sweep, g); pk.amp = X.amp; }
-      compact_node<NODES, WARM>(A, valid, i, acc, Q, par, &S, &X.mlp, PERTURB ? &pk : nullptr);
-    }
-  } else {
-    for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {  // uniform over the CTA
-      const int g = batch_grid_of(ts, B.n, t);
-      const SweepArgs &A = B.grids[g];
-      const long long j = (t - __ldg(&ts[g])) * kBatchTile + threadIdx.x;
-      const bool valid = j < (NODES == 1 ? A.M.Nc : A.M.Nv);
-      const long long i = NODES == 1 ? j : A.M.Nc + j;
-      PerturbKey pk;
-      if (PERTURB) { pk.key = perturb_key(X.seed, X.sweep, g); pk.amp = X.amp; }
-      if (WARM) warm_node<ANISO, NODES>(A, S, X.mlp, valid, i, acc, PERTURB ? &pk : nullptr);
-      else if (valid) sweep_node<ANISO, NODES>(A, i, acc, PERTURB ? &pk : nullptr);
-    }
+  for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {  // uniform over the CTA
+    const int g = batch_grid_of(ts, B.n, t);
+    const SweepArgs &A = B.grids[g];
+    const long long j = (t - __ldg(&ts[g])) * kBatchTile + threadIdx.x;
+    const bool valid = j < (NODES == 1 ? A.M.Nc : A.M.Nv);
+    const long long i = NODES == 1 ? j : A.M.Nc + j;
+    PerturbKey pk;
+    if (PERTURB) { pk.key = perturb_key(X.seed, X.sweep, g); pk.amp = X.amp; }
+    if (WARM) warm_node<ANISO, NODES>(A, S, X.mlp, valid, i, acc, PERTURB ? &pk : nullptr);
+    else if (valid) sweep_node<ANISO, NODES>(A, i, acc, PERTURB ? &pk : nullptr);
   }
   flush_acc(B.stats, acc);
 }

@@ -1,7 +1,7 @@
 // sweep_node.cuh -- the device code of one node of a sweep, shared by the plain, warm-start
 // and many-grid kernels: its load and set-up, every active phase's local solve, the averages
 // and the stores, for one node per thread (sweep_node) and for a CTA that walks its nodes'
-// phases in step (compact_node, warm_node).
+// phases in step (warm_node).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -302,17 +302,17 @@ __device__ __forceinline__ void iso_accumulate(const SweepArgs &A, const Node &n
   }
   double share = 0.0;  // S
   if (o.mech & MDZ_MECH_PEIERLS) share = m.e_exp;
-  if (fl & F_PWL) share += m.e_pwl;
+  if (fl & F_PWL) share = __dadd_rn(share, m.e_pwl);  // sums and products rounded apart: the same bits in every kernel
   if (fl & F_LIN) {
     // eta_lin = B pow(Eii_lin, 1/n-1) pow(d1, m/n) = Tii/(2 Eii_lin) (d1/d)^(m/n), d1 = gs_ref
     double l = m.e_lin;
-    if ((fl & F_LIN_M) && !(fl & F_GS)) l *= FxMath::exp(fma(ph.lin_mn, S.lnd, ph.lin_lnd));
-    share += l;
+    if ((fl & F_LIN_M) && !(fl & F_GS)) l = __dmul_rn(l, FxMath::exp(__fma_rn(ph.lin_mn, S.lnd, ph.lin_lnd)));
+    share = __dadd_rn(share, l);
   }
-  if (fl & F_CST) share += m.e_cst;
-  if (m.is_pl) share += m.pl_share;
+  if (fl & F_CST) share = __dadd_rn(share, m.e_cst);
+  if (m.is_pl) share = __dadd_rn(share, m.pl_share);
   const double ve = m.is_pl ? m.eta_vep : m.eta_ve;
-  const double etaVE = clamp_eta(M, ve), eta = clamp_eta(M, m.eta_ve * FxMath::recip(share));
+  const double etaVE = clamp_eta(M, ve), eta = clamp_eta(M, __dmul_rn(m.eta_ve, FxMath::recip(share)));
   if (m.is_pl) o.mech |= MDZ_MECH_YIELD;
   set_status(status, o.status);
   acc.calls++; acc.iters += o.iters; acc.plastic += m.is_pl; acc.f32 += o.f32_steps;
@@ -340,12 +340,12 @@ __device__ __forceinline__ void iso_accumulate(const SweepArgs &A, const Node &n
     const double ex = fma(t2, n.in.Exx, -n.in.Txx0), ez = fma(t2, n.in.Ezz, -n.in.Tzz0);
     const double exz = fma(t2, n.in.Exz, -n.in.Txz0);
     // (ex^2 + ez^2 + ey^2) / 2 + exz^2 with ey = -(ex + ez)
-    q.el = fma(perc, FxMath::sqrt(fma(exz, exz, fma(ez, ex + ez, ex * ex))), q.el);
+    q.el = fma(perc, FxMath::sqrt(__fma_rn(exz, exz, __fma_rn(ez, __dadd_rn(ex, ez), __dmul_rn(ex, ex)))), q.el);
   }
   const double rate = plastic == 2 ? 2.0 * m.lam_dot * m.A_tau : m.gdot;
   if (m.is_pl) q.pl = fma(perc, rate, q.pl);
-  const double pT = perc * m.Tii, w = pT * m.T_over_eta;
-  q.Wtot += w;
+  const double pT = __dmul_rn(perc, m.Tii), w = __dmul_rn(pT, m.T_over_eta);
+  q.Wtot = __dadd_rn(q.Wtot, w);
   q.Wdiss = fma(w, share, q.Wdiss);
   q.Wel = fma(pT, m.Tii, q.Wel);
   if ((int)fp64_hi(share) < 0 && fp64_lt(share, 0.0) && !fp64_is_zero(m.Tii)) set_status(status, MDZ_EWDISS);
@@ -398,13 +398,7 @@ __device__ __forceinline__ void iso_sweep_item(const SweepArgs &A, const Node &n
                                                int &status, double *eta_conv = nullptr) {
   IsoMid m;
   iso_ve<FxMath>(A.M, A.ph[p], n.in, n.ctx, S, s_start, polish, o, m, eta_conv);
-  if (iso_yields_dp(A.M, A.ph[p], n.ctx, m)) {
-    DpItem d;
-    dp_load(d, m, n.in, n.ctx);
-    dp_return(A.M, A.ph[p], d);
-    dp_extra(d);
-    dp_store(m, d);
-  }
+  if (iso_yields_dp(A.M, A.ph[p], n.ctx, m)) dp_return_inline(A.M, A.ph[p], n.in, n.ctx, m);
   iso_accumulate<NODES>(A, n, p, perc, S, o, m, q, acc, status);
   o.is_pl = m.is_pl;
 }
@@ -480,63 +474,6 @@ __device__ __forceinline__ void sweep_node(const SweepArgs &A, long long i, Acc 
   }
 }
 
-// Compacting form of the isotropic sweep: the CTA's 128 threads walk their nodes' phases
-// in step (the node and phase loops are uniform over the CTA), and the Drucker-Prager
-// returns of each phase's yielding items run packed into the first warps (dp_compact).
-// Same functions, so the same bits as k_sweep.
-
-// The warm-start declarations (used below with WARM)
-__device__ __forceinline__ void warm_inputs(const MlpDevice &W, const float *f, int nfeat, float *x);
-
-// One isotropic node per thread; every thread of the CTA calls it together (valid false: a
-// thread without a node, which still takes part in the CTA's barriers and, WARM, in its
-// warp's network).  WARM: the learned start, evaluated per warp, before each local solve.
-template <int NODES, bool WARM>
-__device__ __forceinline__ void compact_node(const SweepArgs &A, bool valid, long long i, Acc &acc,
-                                             CompactQueue &Q, int &par, MlpWarpShared *S = nullptr,
-                                             const MlpDevice *W = nullptr, const PerturbKey *pk = nullptr) {
-  Node n;
-  n.solid = false;
-  n.centroid = NODES == 1;
-  if (valid) node_prepare<false, NODES>(A, i, n, pk);
-  IsoAcc q;
-  iso_acc_zero(q);
-  int status = MDZ_OK;
-  const int polish = WARM ? W->polish_iters : A.polish;
-  for (int p = 0; p < A.M.np; p++) {  // uniform over the CTA
-    const double perc = (valid && n.solid) ? node_perc(A, n, p) : 0.0;
-    const bool active = fp64_abs_gt_pos(perc, 1e-13);  // :1210-1212
-    if (valid && n.solid && !active) node_iters(A, n, p, 0);
-    IsoState st;
-    PointOut o;
-    IsoMid m;
-    float s_start = 1.0f;
-    if (WARM) {
-      float f[kMlpIn], x[kMlpIn];
-#pragma unroll
-      for (int k = 0; k < kMlpIn; k++) f[k] = 0.0f;
-      if (active) {
-        iso_setup<FxMath>(A.M, A.ph[p], n.in, n.ctx, st, o, polish == 0);
-        warm_features(A.M, n.in, n.ctx, st, false, f);
-      }
-      warm_inputs(*W, f, kFeatIso, x);
-      __syncwarp();
-      const float y = mlp_warp_predict(*S, x);
-      s_start = warm_start_point(y, W->z_scale, W->z_shift);
-    } else if (active) {
-      iso_setup<FxMath>(A.M, A.ph[p], n.in, n.ctx, st, o, polish == 0);
-    }
-    bool yields = false;
-    if (active) {
-      iso_ve<FxMath>(A.M, A.ph[p], n.in, n.ctx, st, s_start, polish, o, m);
-      yields = iso_yields_dp(A.M, A.ph[p], n.ctx, m);
-    }
-    dp_compact<true>(A.M, A.ph[p], Q, par, yields, m, n.in, n.ctx);
-    if (active) iso_accumulate<NODES>(A, n, p, perc, st, o, m, q, acc, status);
-  }
-  if (valid) iso_store<NODES>(A, n, q, status);
-}
-
 // ---------------------------------------------------------------------------------
 // learned warm start, per warp: the plain sweep with the network between each phase's
 // set-up and its local solve, evaluated by the warp's 32 lanes on the tensor cores
@@ -550,10 +487,9 @@ __device__ __forceinline__ void warm_inputs(const MlpDevice &W, const float *f, 
 
 // One node per lane, the warp's 32 nodes consecutive, so every lane of a warp runs the
 // same number of node iterations and reaches the network at the same phase; lanes past
-// the end or at inactive (node, phase) items feed zeros and discard the output.
-// One node of the learned-warm-start sweep; every lane of the warp calls it together
-// (valid false: a lane without a node, which still takes part in the network).
-template <bool ANISO, int NODES>  // the anisotropic sweep; the isotropic one is compact_node<NODES, true>
+// the end or at inactive (node, phase) items feed zeros and discard the output.  Every lane
+// of the warp calls it together (valid false: a lane without a node).
+template <bool ANISO, int NODES>
 __device__ __forceinline__ void warm_node(const SweepArgs &A, MlpWarpShared &S, const MlpDevice &W, bool valid,
                                           long long i, Acc &acc, const PerturbKey *pk = nullptr) {
   const int nfeat = ANISO ? kFeatAniso : kFeatIso;
@@ -561,9 +497,11 @@ __device__ __forceinline__ void warm_node(const SweepArgs &A, MlpWarpShared &S, 
   n.solid = false;
   n.centroid = NODES == 1;
   if (valid) node_prepare<ANISO, NODES>(A, i, n, pk);
-  double out[CO_COUNT];
+  double out[CO_COUNT];  // anisotropic
+  IsoAcc q;              // isotropic
 #pragma unroll
   for (int k = 0; k < CO_COUNT; k++) out[k] = 0.0;
+  iso_acc_zero(q);
   int status = MDZ_OK;
   for (int p = 0; p < A.M.np; p++) {  // uniform over the warp
     const double perc = (valid && n.solid) ? node_perc(A, n, p) : 0.0;
@@ -575,7 +513,8 @@ __device__ __forceinline__ void warm_node(const SweepArgs &A, MlpWarpShared &S, 
 #pragma unroll
     for (int k = 0; k < kMlpIn; k++) f[k] = 0.0f;
     if (active) {
-      aniso_setup<FxMath>(A.M, A.ph[p], n.in, n.ctx, n.an, st, o, W.polish_iters == 0);
+      if constexpr (ANISO) aniso_setup<FxMath>(A.M, A.ph[p], n.in, n.ctx, n.an, st, o, W.polish_iters == 0);
+      else iso_setup<FxMath>(A.M, A.ph[p], n.in, n.ctx, st, o, W.polish_iters == 0);
       warm_features(A.M, n.in, n.ctx, st, ANISO, f);
     }
     warm_inputs(W, f, nfeat, x);
@@ -583,10 +522,18 @@ __device__ __forceinline__ void warm_node(const SweepArgs &A, MlpWarpShared &S, 
     const float y = mlp_warp_predict(S, x);
     if (!active) continue;
     const float s_start = warm_start_point(y, W.z_scale, W.z_shift);
-    aniso_finish<FxMath>(A.M, A.ph[p], n.in, n.ctx, n.an, st, s_start, W.polish_iters, o);
-    node_accumulate<ANISO>(A, n, p, perc, o, out, acc, status);
+    if constexpr (ANISO) {
+      aniso_finish<FxMath>(A.M, A.ph[p], n.in, n.ctx, n.an, st, s_start, W.polish_iters, o);
+      node_accumulate<ANISO>(A, n, p, perc, o, out, acc, status);
+    } else {
+      iso_sweep_item<NODES>(A, n, p, perc, st, s_start, W.polish_iters, o, q, acc, status);
+    }
   }
-  if (valid) node_store<ANISO>(A, n, out, status);
+  if constexpr (ANISO) {
+    if (valid) node_store<ANISO>(A, n, out, status);
+  } else {
+    if (valid) iso_store<NODES>(A, n, q, status);
+  }
 }
 
 }  // namespace mdz

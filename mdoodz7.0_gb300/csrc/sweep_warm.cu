@@ -20,20 +20,10 @@ __global__ void __launch_bounds__(128, 4) k_sweep_warm(const __grid_constant__ S
   const long long total = NODES == 1 ? A.M.Nc : A.M.Nv;
   const long long lo = NODES == 1 ? 0 : A.M.Nc;
   const long long stride = (long long)gridDim.x * blockDim.x;
-  if constexpr (ANISO) {
-    const int lane = threadIdx.x & 31;
-    for (long long base = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < total; base += stride) {
-      const long long j = base + lane;
-      warm_node<ANISO, NODES>(A, S, W, j < total, lo + j, acc);
-    }
-  } else {  // the isotropic sweep compacts its plastic returns per CTA (k_sweep_compact)
-    __shared__ CompactQueue Q;
-    compact_init(Q);
-    int par = 0;
-    for (long long base = (long long)blockIdx.x * blockDim.x; base < total; base += stride) {  // uniform
-      const long long j = base + threadIdx.x;
-      compact_node<NODES, true>(A, j < total, lo + j, acc, Q, par, &S, &W);
-    }
+  const int lane = threadIdx.x & 31;
+  for (long long base = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < total; base += stride) {
+    const long long j = base + lane;
+    warm_node<ANISO, NODES>(A, S, W, j < total, lo + j, acc);
   }
   flush_acc(A.stats, acc);
 }
