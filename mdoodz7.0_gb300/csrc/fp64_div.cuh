@@ -118,6 +118,29 @@ __device__ __forceinline__ double div_by(double a, const Divisor &d) {
   return div_by_rare(a, d.b, d.y, d.fast, d.eb, d.bman);
 }
 
+// a / s, correctly rounded, for s within 32 units of 2^-53 of 1 (a sum of weights), on the
+// integer pipe: with s = 1 - k 2^-53 and ma the significand of a, the quotient's significand is
+//     ma + (T + c) 2^-53,   T = ma k,  c = T k 2^-53 (1 + O(2^-48)) >= 0, below 2^11,
+// rounded by its fraction.  false, and nothing formed, where the fraction lies within 8 units
+// of 2^-53 below one half (c is taken to 4), where the quotient may leave a's binade, for other
+// s, and for subnormal, huge or special a.
+FX_FN bool div_near_one(double a, double s, double &out) {
+  const uint64_t ab = fx_bits(a), sb = fx_bits(s);
+  const int64_t up = (int64_t)(sb - 0x3ff0000000000000ull);  // s = 1 + up 2^-52, or 1 + up 2^-53 below 1
+  const int64_t k = up > 0 ? -2 * up : -up;
+  const uint32_t E = (fx_hi(ab) >> 20) & 0x7ffu;
+  const uint64_t ma = fx_significand(ab);
+  if ((ab << 1) == 0 && k <= 32 && k >= -32) { out = a; return true; }
+  if (k > 32 || k < -32 || E - 23u > 2000u || ma - 0x10000000000040ull > 0xfffffffffff80ull) return false;
+  const int64_t T = (int64_t)ma * k;                                  // |T| <= 2^58
+  const int64_t U = T + (((T >> 27) * k) >> 26);                      // T + c
+  const uint64_t half = 1ull << 52, frac = (uint64_t)U & (2 * half - 1);
+  if (half - 1 - frac < 8) return false;
+  const uint64_t r = ma + (uint64_t)(U >> 53) + (frac >= half ? 1 : 0);
+  out = fx_double((ab & 0xfff0000000000000ull) | (r & 0xfffffffffffffull));
+  return true;
+}
+
 // 1 / x, correctly rounded: the reciprocal of fx64.cuh, within 2 units of its 64th bit, rounded
 // unless the spare bits lie within 4 units of one half (one in 250; then, and outside
 // [2^-1000, 2^1000], the IEEE division).

@@ -66,16 +66,20 @@ __device__ __forceinline__ int cell_of(double q) { return fp64_ceil_int(q) - 1; 
 __device__ __forceinline__ bool sign_clear(double v) { return (fp64_hi(v) >> 31) == 0u; }
 
 // (a / sw, b / sw) as the reference writes them.  For sw == 1 a division returns its
-// numerator; the bilinear weights of a cell without air sum to exactly 1 for most
-// markers, and the divisions stay out of line so that a warp whose markers all have
-// sw == 1 branches past them.
+// numerator; the bilinear weights of a cell without air sum to 1 within a few ulp, which
+// div_near_one divides by on the integer pipe.  The IEEE divisions stay out of line.
 __device__ __noinline__ double2 div_pair(double a, double b, double sw) { return make_double2(a / sw, b / sw); }
 
 __device__ __forceinline__ void div_sum(double &a, double &b, double sw) {
   if (fp64_bits(sw) != 0x3ff0000000000000ull) {
-    const double2 q = div_pair(a, b, sw);
-    a = q.x;
-    b = q.y;
+    double qa, qb;
+    if (!(div_near_one(a, sw, qa) && div_near_one(b, sw, qb))) {
+      const double2 q = div_pair(a, b, sw);
+      qa = q.x;
+      qb = q.y;
+    }
+    a = qa;
+    b = qb;
   }
 }
 

@@ -95,3 +95,35 @@ def test_k_ln2_on_the_host(tmp_path):
     hi, lo = float.fromhex("0x1.62e42fefa39efp-1"), float.fromhex("0x1.abc9e3b39803fp-56")
     for k in range(-1100, 1101):
         assert f(k) == float(Fraction(k) * Fraction(hi) + Fraction(k * lo)), k
+
+
+def test_division_near_one_on_the_host(tmp_path):
+    """div_near_one against IEEE division, bit for bit: every divisor within its range, numerators random and at the
+    ends of a binade, zeros; what it declines is left to the division."""
+    src = tmp_path / "d.cpp"
+    text = open(R.HERE + "/csrc/fp64_div.cuh").read()
+    at = text.index("FX_FN bool div_near_one")
+    src.write_text('#include "fx64.cuh"\nnamespace mdz {\n' + text[at:text.index("\n}\n", at) + 3] + "}\n"
+                   'extern "C" void run(long n, const double *a, const double *s, double *q, int *ok) {\n'
+                   "  for (long i = 0; i < n; i++) ok[i] = mdz::div_near_one(a[i], s[i], q[i]);\n}\n")
+    lib = tmp_path / "d.so"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-ffp-contract=off", "-I", R.HERE + "/csrc", str(src),
+                    "-o", str(lib)], check=True, capture_output=True)
+    rng = np.random.default_rng(9)
+    n = 2_000_000
+    s = (np.int64(0x3ff0000000000000) + rng.integers(-34, 19, n)).view(np.float64)
+    man = rng.integers(0, 1 << 52, n)
+    man[::5] = rng.integers(0, 300, man[::5].size)
+    man[1::5] = (1 << 52) - 1 - rng.integers(0, 300, man[1::5].size)
+    bits = (rng.integers(0, 2, n) << 63) | (rng.integers(0, 2048, n) << 52) | man
+    a = bits.astype(np.uint64).view(np.float64)
+    a[::97] = 0.0
+    a[1::97] = -0.0
+    q, ok = np.zeros(n), np.zeros(n, np.int32)
+    f = ctypes.CDLL(str(lib)).run
+    f.argtypes = [ctypes.c_long] + [ctypes.c_void_p] * 4
+    f(n, *[x.ctypes.data for x in (a, s, q, ok)])
+    with np.errstate(all="ignore"):
+        want = a / s
+    t = ok == 1
+    assert t.mean() > 0.5 and np.array_equal(q[t].view(np.uint64), want[t].view(np.uint64))
