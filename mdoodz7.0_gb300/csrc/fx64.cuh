@@ -37,9 +37,11 @@
 #ifdef __CUDACC__
 #include <cuda_runtime.h>
 #define FX_FN __host__ __device__ __forceinline__
+#define FX_DEV __device__ __forceinline__
 #else
 #include <math.h>
 #define FX_FN static inline
+#define FX_DEV static inline
 #endif
 
 #include "fx64_tables.inc"
@@ -140,6 +142,38 @@ FX_FN double fx_normalise(uint64_t V, int e) {
   const int s = fx_clz(fx_hi(V));
   const uint64_t N = ((uint64_t)fx_funnel(fx_lo(V), fx_hi(V), s) << 32) | (uint64_t)(fx_lo(V) << s);
   return fx_assemble(N, e - s);
+}
+
+// ---- product -------------------------------------------------------------------------------
+// a b rounded to nearest even, the bits of the FP64 multiplication, on the integer pipe (about
+// 35 instructions, 16 cycles per warp and SM against 20 of a DMUL): for kernels that the FP64
+// pipe binds while the integer one idles, as a second multiplier beside it.  Operands and
+// products outside the normal range take the FP64 one.
+#if defined(__CUDACC__)
+static __device__ __noinline__ double fx_mul_rare(double a, double b) { return __dmul_rn(a, b); }
+#else
+static inline double fx_mul_rare(double a, double b) { return a * b; }
+#endif
+FX_DEV double fx_mul_rn(double a, double b) {
+  const uint64_t ab = fx_bits(a), bb = fx_bits(b);
+  const uint32_t ea = (fx_hi(ab) >> 20) & 0x7ffu, eb = (fx_hi(bb) >> 20) & 0x7ffu;
+  const uint32_t e = ea + eb;
+  // both normal and finite, and the product's exponent e - 1023 (+ 1) in [1, 2045]
+  if (ea - 1u >= 0x7feu || eb - 1u >= 0x7feu || e - 1025u >= 2043u) {
+    // a zero times a finite number is the common case here
+    if (((ab << 1) == 0 && eb != 0x7ffu) || ((bb << 1) == 0 && ea != 0x7ffu)) return fx_double((ab ^ bb) & 0x8000000000000000ull);
+    return fx_mul_rare(a, b);
+  }
+  const uint64_t x = fx_significand(ab) << 11, y = fx_significand(bb) << 11;
+  const uint64_t t0 = (uint64_t)fx_lo(x) * fx_lo(y);
+  const uint64_t t1 = (uint64_t)fx_hi(x) * fx_lo(y) + fx_hi(t0);
+  const uint64_t t2 = (uint64_t)fx_lo(x) * fx_hi(y) + fx_lo(t1);
+  uint64_t h = (uint64_t)fx_hi(x) * fx_hi(y) + fx_hi(t1) + fx_hi(t2);  // x y 2^-64
+  h |= ((fx_lo(t2) | fx_lo(t0)) != 0u) ? 1u : 0u;                      // what is below it, as a sticky bit
+  const int c = (int)(fx_hi(h) >> 31), sh = 10 + c;
+  const uint64_t r = (h + (((uint64_t)512u << c) - 1u) + ((h >> sh) & 1u)) >> sh;
+  const uint64_t q = r + ((uint64_t)(e - 1024u + (uint32_t)c) << 52);
+  return fx_double(q | ((ab ^ bb) & 0x8000000000000000ull));
 }
 
 // ---- exp -----------------------------------------------------------------------------------

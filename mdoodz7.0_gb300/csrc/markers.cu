@@ -41,8 +41,9 @@
 // cell indices come from fp64_ceil_int (the reference's ceil, on the integer pipe), and
 // a division by a weight sum that is exactly 1 is skipped (it returns its numerator),
 // so positions, weights and results are the reference's to the last bit.  The divisions run on
-// the integer pipe (fp64_div.cuh): 4.2 M markers 846 -> 663 us, P2Mastah's 9-cell form
-// 1275 -> 909 us.  The director
+// the integer pipe (fp64_div.cuh), and so do the weights' products (fx_mul_rn), which leaves
+// the two pipes about even: 4.2 M markers 846 -> 663 (divisions by the spacing) -> 526 (by
+// weight sums near 1) -> 501 us (products), P2Mastah's 9-cell form 1275 -> 868 us.  The director
 // normalisation squares by multiplication where the reference calls pow.
 #include "markers.cuh"
 
@@ -123,10 +124,10 @@ __device__ __forceinline__ double from_zero(double x) { return fp64_is_negative_
 // bilinear weights in the reference's order SW, SE, NW, NE: a = dxm/dx, b = dzm/dz
 __device__ __forceinline__ void weights(double a, double b, double w[4]) {
   const double ia = __dsub_rn(1.0, a), ib = __dsub_rn(1.0, b);
-  w[0] = __dmul_rn(ia, ib);
-  w[1] = __dmul_rn(a, ib);
-  w[2] = __dmul_rn(ia, b);
-  w[3] = __dmul_rn(a, b);
+  w[0] = fx_mul_rn(ia, ib);
+  w[1] = fx_mul_rn(a, ib);
+  w[2] = fx_mul_rn(ia, b);
+  w[3] = fx_mul_rn(a, b);
 }
 
 __device__ __forceinline__ int clamp_to(int v, int hi) { return v < 0 ? 0 : (v > hi ? hi : v); }
@@ -504,8 +505,9 @@ __global__ void __launch_bounds__(256) k_marker_update(const MarkerArgs A) {
       // an air corner lends its weight to the corner across; the increments are 0 at air
       const int cc = air(A.bcp[c[q]]) ? alt[q] : c[q];
       const double2 f = A.inc_n[cc];
-      dsx = q == 0 ? from_zero(__dmul_rn(wc[q], f.x)) : __dadd_rn(dsx, __dmul_rn(wc[q], f.x));
-      dsz = q == 0 ? from_zero(__dmul_rn(wc[q], f.y)) : __dadd_rn(dsz, __dmul_rn(wc[q], f.y));
+      const double px = fx_mul_rn(wc[q], f.x), pz = fx_mul_rn(wc[q], f.y);
+      dsx = q == 0 ? from_zero(px) : __dadd_rn(dsx, px);
+      dsz = q == 0 ? from_zero(pz) : __dadd_rn(dsz, pz);
       sw = q == 0 ? from_zero(wc[q]) : __dadd_rn(sw, wc[q]);
     }
     if (fp64_gt(sw, 1e-13)) div_sum(dsx, dsz, sw);

@@ -12,8 +12,8 @@
 // One thread per node, centroids first, then vertices; every access is coalesced.
 // Both kernels are short per node and bound by the FP64 pipe (divisions by the phase
 // constants and the moduli's reciprocals run on the integer pipe, fp64_div.cuh: both calls at
-// 1025 x 1025 cells, 5 phases, 332 -> 250 us; tests on the bits of a double too,
-// fp64_bits.cuh).  Every product and sum is
+// 1025 x 1025 cells, 5 phases, 332 -> 250 us; the averages' products too, fx64.cuh:
+// -> 214 us; tests on the bits of a double, fp64_bits.cuh).  Every product and sum is
 // written with explicit round-to-nearest intrinsics, so no FMA contraction changes a
 // bit against the reference; the per-phase constants are folded on the host with the
 // reference's own expressions.
@@ -86,9 +86,9 @@ __global__ void __launch_bounds__(256) k_softening(const SoftArgs A) {
       soften(A.ph[p], A.style, s, ks, s_nan, f, d, c);
       // a zero fraction of finite values adds a zero, which leaves the sums unchanged
       if (fp64_is_zero(w) && fp64_finite(f) && fp64_finite(d) && fp64_finite(c)) continue;
-      fric = __dadd_rn(fric, __dmul_rn(w, f));
-      dil = __dadd_rn(dil, __dmul_rn(w, d));
-      C = __dadd_rn(C, __dmul_rn(w, c));
+      fric = __dadd_rn(fric, fx_mul_rn(w, f));
+      dil = __dadd_rn(dil, fx_mul_rn(w, d));
+      C = __dadd_rn(C, fx_mul_rn(w, c));
     }
     if (A.noise == 1) {
       const double r = cen ? A.noise_n[n] : A.noise_s[n];

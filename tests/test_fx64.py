@@ -127,3 +127,32 @@ def test_division_near_one_on_the_host(tmp_path):
         want = a / s
     t = ok == 1
     assert t.mean() > 0.5 and np.array_equal(q[t].view(np.uint64), want[t].view(np.uint64))
+
+
+def test_product_on_the_host(tmp_path):
+    """fx_mul_rn against the FP64 multiplication, bit for bit: random bit patterns (every exponent, special values),
+    short significands (exact products and ties), products near the ends of the range."""
+    src = tmp_path / "m.cpp"
+    src.write_text('#include "fx64.cuh"\nextern "C" void run(long n, const double *a, const double *b, double *o) {\n'
+                   "  for (long i = 0; i < n; i++) o[i] = mdz::fx_mul_rn(a[i], b[i]);\n}\n")
+    lib = tmp_path / "m.so"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-ffp-contract=off", "-I", R.HERE + "/csrc", str(src),
+                    "-o", str(lib)], check=True, capture_output=True)
+    rng = np.random.default_rng(21)
+    n = 3_000_000
+    x, y = (rng.integers(0, 1 << 64, n, dtype=np.uint64) for _ in range(2))
+    x[::3] &= np.uint64(0xfffffffff0000000)
+    y[::3] &= np.uint64(0xffffffffff000000)
+    for v, lo in ((x, 900), (y, 1000)):  # exponents near 1, so that most products are normal
+        v[1::2] = (v[1::2] & np.uint64(0x800fffffffffffff)) | ((np.uint64(lo) + v[1::2] % np.uint64(100)) << np.uint64(52))
+    x[5::50] = np.uint64(0)
+    y[6::50] = np.uint64(1 << 63)
+    a, b = x.view(np.float64), y.view(np.float64)
+    o = np.empty(n)
+    f = ctypes.CDLL(str(lib)).run
+    f.argtypes = [ctypes.c_long] + [ctypes.c_void_p] * 3
+    f(n, a.ctypes.data, b.ctypes.data, o.ctypes.data)
+    with np.errstate(all="ignore"):
+        want = a * b
+    same = (o.view(np.uint64) == want.view(np.uint64)) | (np.isnan(o) & np.isnan(want))
+    assert same.all(), (a[~same][:3], b[~same][:3])
