@@ -67,6 +67,25 @@ static const FxPair h_fx_sincos[384] = MDZ_FX_SINCOS_TABLE;
 #define FX_TAB(name, i) (h_fx_##name[i])
 #endif
 
+// CUDA's functions for the arguments outside the fast ranges, out of line: inlined, the
+// compiler runs their first FP64 instructions ahead of the branch that selects them.
+#if defined(__CUDACC__)
+static __device__ __noinline__ double fx_exp_rare(double x) { return exp(x); }
+static __device__ __noinline__ double fx_log_rare(double x) { return log(x); }
+static __device__ __noinline__ double fx_recip_rare(double x) { return 1.0 / x; }
+static __device__ __noinline__ double fx_sqrt_rare(double x) { return sqrt(x); }
+static __device__ __noinline__ double2 fx_sincos_rare(double x) {
+  double2 r;
+  sincos(x, &r.x, &r.y);
+  return r;
+}
+#endif
+#if defined(__CUDA_ARCH__)
+#define FX_RARE(f, plain, x) fx_##f##_rare(x)
+#else
+#define FX_RARE(f, plain, x) (plain)
+#endif
+
 // ---- 32- and 64-bit pieces -----------------------------------------------------------------
 FX_FN uint32_t fx_umulhi(uint32_t a, uint32_t b) {
 #if defined(__CUDA_ARCH__)
@@ -214,7 +233,7 @@ FX_FN double fx_exp_double(uint64_t M, int m) {
 // |x| < 500; CUDA's exp elsewhere
 FX_FN double fx_exp(double x) {
   const uint64_t b = fx_bits(x);
-  if ((fx_hi(b) & 0x7fffffffu) >= 0x407f4000u) return exp(x);
+  if ((fx_hi(b) & 0x7fffffffu) >= 0x407f4000u) return FX_RARE(exp, exp(x), x);
   int m;
   const uint64_t M = fx_exp_core(fx_fixed<54>(b), m);
   return fx_exp_double(M, m);
@@ -277,9 +296,9 @@ FX_FN bool fx_log_of(int m, uint64_t F, uint32_t least, double &out) {
 FX_FN double fx_log(double x) {
   const uint64_t b = fx_bits(x);
   const uint32_t hi = fx_hi(b);
-  if (hi < 0x00100000u || hi >= 0x7ff00000u) return log(x);
+  if (hi < 0x00100000u || hi >= 0x7ff00000u) return FX_RARE(log, log(x), x);
   double r;
-  if (!fx_log_of((int)(hi >> 20) - 1023, fx_log_significand(fx_significand(b)), 0x20000000u, r)) return log(x);
+  if (!fx_log_of((int)(hi >> 20) - 1023, fx_log_significand(fx_significand(b)), 0x20000000u, r)) return FX_RARE(log, log(x), x);
   return r;
 }
 
@@ -342,7 +361,7 @@ FX_FN uint64_t fx_recip_core(uint64_t D) {
 FX_FN double fx_recip(double x) {
   const uint64_t b = fx_bits(x);
   const uint32_t E = (fx_hi(b) >> 20) & 0x7ffu;
-  if (E - 23u > 2000u) return 1.0 / x;
+  if (E - 23u > 2000u) return FX_RARE(recip, 1.0 / x, x);
   const uint64_t Y = fx_recip_core(fx_significand(b) << 11);
   const double r = fx_assemble(Y, -(int)E + 1023 - 64);
   return fx_double(fx_bits(r) | (b & 0x8000000000000000ull));
@@ -365,7 +384,7 @@ FX_FN float fx_rsqrt_estimate(float d) {
 FX_FN double fx_sqrt(double x) {
   const uint64_t b = fx_bits(x);
   const uint32_t E = fx_hi(b) >> 20;
-  if (E - 23u > 2000u) return sqrt(x);
+  if (E - 23u > 2000u) return FX_RARE(sqrt, sqrt(x), x);
   const int odd = (int)((E & 1u) ^ 1u);  // unbiased exponent E - 1023 is odd where E is even
   const uint64_t D = fx_significand(b) << (9 + odd);  // Q2.62... d = D 2^-61 in [1, 4)
   const float df = fx_float(((127u + (uint32_t)odd) << 23) | (uint32_t)((b >> 29) & 0x7fffff));
@@ -395,7 +414,8 @@ FX_FN void fx_sincos(double x, double *sn, double *cs) {
   if (ahi - 0x3fb00000u >= 0x00480000u) {
     if ((ahi | fx_lo(b)) == 0u) { *sn = x; *cs = 1.0; return; }
 #if defined(__CUDA_ARCH__)
-    sincos(x, sn, cs);
+    const double2 r = fx_sincos_rare(x);
+    *sn = r.x; *cs = r.y;
 #else
     *sn = sin(x); *cs = cos(x);
 #endif

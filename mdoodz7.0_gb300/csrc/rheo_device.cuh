@@ -65,6 +65,7 @@ struct FxMath {
   static __device__ __forceinline__ double divide(double r, double d) { return quotient(r, d); }
   static __device__ __forceinline__ double sqrt(double x) { return fx_sqrt_call(x); }
   static __device__ __forceinline__ void sincos(double x, double *s, double *c) { fx_sincos(x, s, c); }
+  static __device__ __forceinline__ double sin(double x) { return fx_sincos_rare(x).x; }
 };
 struct FdMath {
   static constexpr bool kFixed = false;
@@ -76,6 +77,7 @@ struct FdMath {
   static __device__ __forceinline__ double divide(double r, double d) { return r / d; }
   static __device__ __forceinline__ double sqrt(double x) { return ::sqrt(x); }
   static __device__ __forceinline__ void sincos(double x, double *s, double *c) { ::sincos(x, s, c); }
+  static __device__ __forceinline__ double sin(double x) { return ::sin(x); }
 };
 
 constexpr double kZeroC = 273.15;                 // MDLIB/include/mdoodz.h:4
@@ -205,7 +207,7 @@ __device__ __forceinline__ void node_common(const ModelConst &M, const NodeIn &i
   c.lnd = need_lnd ? FP::log(in.d) : 0.0;
   c.inv_d = 0.0;
   FP::sincos(in.fric, &c.sin_fric, &c.cos_fric);
-  c.sin_dil = fp64_is_zero(c.dil) ? 0.0 : sin(c.dil);
+  c.sin_dil = fp64_is_zero(c.dil) ? 0.0 : FP::sin(c.dil);
   // products and sum rounded apart: the same bits in every kernel
   c.Tyield = __dadd_rn(__dmul_rn(in.C, c.cos_fric), __dmul_rn(in.P, c.sin_fric));
 }
@@ -244,8 +246,12 @@ __device__ __forceinline__ void node_setup_iso(const ModelConst &M, const NodeIn
   node_common<FP>(M, in, need_lnd, c);
 }
 
-// EvaluateDensity, RheologyDensity.c:1761-1831 (models 0, 1, 3, 5)
-__device__ __forceinline__ double density(const ModelConst &M, const PhaseConst &ph, double T, double P,
+// EvaluateDensity, RheologyDensity.c:1761-1831 (models 0, 1, 3, 5).
+// Like the other options that few runs use (the Popov return, mixed and grain-size dependent
+// viscosities), out of line: inlined, their square roots and exponentials of a node's values
+// are moved out of the phase loop and run for every node, 40 FP64 instructions of a sweep's
+// 240 to 370 per node.
+static __device__ __noinline__ double density(const ModelConst &M, const PhaseConst &ph, double T, double P,
                                           double X, double phi) {
   double rho = 0.0;
   const int dm = ph.density_model;
@@ -841,7 +847,7 @@ struct GseIn {
   int elastic, constant, dislocation, peierls, diffusion;
 };
 
-__device__ inline void ve_gse(const GseIn &q, double &eta_io, double &Tii_o, double &d_io, double &e_cst,
+__device__ __forceinline__ void ve_gse_inl(const GseIn &q, double &eta_io, double &Tii_o, double &d_io, double &e_cst,
                               double &e_pwl, double &e_exp, double &e_lin, int &iters, int &status) {
   const int nitmax = 50, bisection_steps = 20;
   const double tol = 1.0e-11;
@@ -888,6 +894,32 @@ __device__ inline void ve_gse(const GseIn &q, double &eta_io, double &Tii_o, dou
   eta_io = eta; Tii_o = Tii; d_io = d_ve;
 }
 
+struct GseOut {
+  double eta, Tii, d, e_cst, e_pwl, e_exp, e_lin;
+  int iters, status;
+};
+static __device__ __noinline__ GseOut ve_gse_call(GseIn q, double eta, double Tii, double d) {
+  GseOut o;
+  o.eta = eta; o.Tii = Tii; o.d = d;
+  o.status = MDZ_OK;
+  ve_gse_inl(q, o.eta, o.Tii, o.d, o.e_cst, o.e_pwl, o.e_exp, o.e_lin, o.iters, o.status);
+  return o;
+}
+// (the operators, whose stack is at its limit, keep both solves inline)
+template <class FP>
+__device__ __forceinline__ void ve_gse(const GseIn &q, double &eta, double &Tii, double &d, double &e_cst,
+                                       double &e_pwl, double &e_exp, double &e_lin, int &iters, int &status) {
+  if (!FP::kFixed) {
+    ve_gse_inl(q, eta, Tii, d, e_cst, e_pwl, e_exp, e_lin, iters, status);
+    return;
+  }
+  const GseOut o = ve_gse_call(q, eta, Tii, d);
+  eta = o.eta; Tii = o.Tii; d = o.d;
+  e_cst = o.e_cst; e_pwl = o.e_pwl; e_exp = o.e_exp; e_lin = o.e_lin;
+  iters = o.iters;
+  set_status(status, o.status);
+}
+
 // solve_local_3x3, RheologyDensity.c:1082-1125
 __device__ __forceinline__ bool solve3(double J11, double J12, double J13, double J21, double J22, double J23,
                                        double J31, double J32, double J33, double R1, double R2, double R3,
@@ -903,7 +935,7 @@ __device__ __forceinline__ bool solve3(double J11, double J12, double J13, doubl
 
 // Combined mode-I/mode-II return of Popov et al. 2025 (RheologyDensity.c:710-930).
 // Returns is_pl and updates Tii, Pc, lam_dot, A_tau, A_P, eta_vp.
-__device__ inline int plastic_popov(const ModelConst &M, const PhaseConst &ph, double Tii_in, double P, double C,
+__device__ __forceinline__ int plastic_popov(const ModelConst &M, const PhaseConst &ph, double Tii_in, double P, double C,
                                     double cos_fric, double sin_fric, double sin_dil, double eta_ve, double K,
                                     double &Tii, double &Pc, double &lam_dot, double &A_tau, double &A_P,
                                     double &eta_vp, int &status) {
@@ -1103,6 +1135,30 @@ __device__ __forceinline__ double lower_viscosity(const ModelConst &M, const Law
   return eta_lo;
 }
 
+static __device__ __noinline__ double mixed_viscosity(const ModelConst &M, const PhaseConst &ph, double X0,
+                                                      double eta_cst) {
+  const double e1 = ph.eta0, e2 = ph.eta0_two;
+  if (M.diffuse_avg == 0) eta_cst = X0 * e1 + (1 - X0) * e2;
+  if (M.diffuse_avg == 1) eta_cst = pow(X0 / e1 + (1 - X0) / e2, -1.0);
+  if (M.diffuse_avg == 2) eta_cst = exp(X0 * log(e1) + (1 - X0) * log(e2));
+  return eta_cst;
+}
+
+// the wattmeter's constant Ag and grain size (:567-576); inv_pwl = 1 / eta_pwl
+struct GrainSize {
+  double Ag, d, lnd;
+};
+static __device__ __noinline__ GrainSize grain_size(const ModelConst &M, const PhaseConst &ph, double T, double eta_el,
+                                                    double Eii, double inv_pwl) {
+  GrainSize g;
+  g.Ag = ph.Kpzm * exp(-ph.Qpzm / M.R / T);
+  const double Tii0 = 2. * eta_el * Eii;
+  const double epwl0 = Tii0 / 2.0 * inv_pwl;
+  g.d = exp(log(g.Ag * ph.Gpzm / (ph.Lpzm * (1.0 / ph.cpzm) * Tii0 * epwl0 * ph.ppzm)) / (1.0 + ph.ppzm));
+  g.lnd = log(g.d);
+  return g;
+}
+
 // exact: the local solve starts where the reference's does (start descriptor 0)
 template <class FP>
 __device__ inline void iso_setup(const ModelConst &M, const PhaseConst &ph, const NodeIn &in, const NodeCtx &c,
@@ -1144,18 +1200,13 @@ __device__ inline void iso_setup(const ModelConst &M, const PhaseConst &ph, cons
   double eta_cst = 0.0, Ag = 0.0, lnd = c.lnd;
   if (constant) eta_cst = ph.eta0;
   if (fl & F_CMIX) {  // :563-565
-    const double X0 = in.X0, e1 = ph.eta0, e2 = ph.eta0_two;
-    if (M.diffuse_avg == 0) eta_cst = X0 * e1 + (1 - X0) * e2;
-    if (M.diffuse_avg == 1) eta_cst = pow(X0 / e1 + (1 - X0) / e2, -1.0);
-    if (M.diffuse_avg == 2) eta_cst = exp(X0 * log(e1) + (1 - X0) * log(e2));
+    eta_cst = mixed_viscosity(M, ph, in.X0, eta_cst);
   }
   if (gs) {  // wattmeter grain size before eta_lin (:567-576)
-    Ag = ph.Kpzm * exp(-ph.Qpzm / M.R / T);
-    const double Tii0 = 2. * eta_el * Eii;
-    const double epwl0 = Tii0 / 2.0 * law_inv<FP>(L, K_PWL);
-    const double d = exp(log(Ag * ph.Gpzm / (ph.Lpzm * (1.0 / ph.cpzm) * Tii0 * epwl0 * ph.ppzm)) / (1.0 + ph.ppzm));
-    o.d1 = d;
-    lnd = log(d);
+    const GrainSize g = grain_size(M, ph, T, eta_el, Eii, law_inv<FP>(L, K_PWL));
+    Ag = g.Ag;
+    o.d1 = g.d;
+    lnd = g.lnd;
     if (diffusion) {
       const double lnBd = (fl & F_LIN_M) ? fma(ph.lin_mn, lnd, L.lnB_lin) : L.lnB_lin;
       L.ln_inv[K_LIN] = c.lnEii - fma(c.lnEii, ph.lin_invn, lnBd);
@@ -1324,9 +1375,9 @@ __device__ inline void iso_ve(const ModelConst &M, const PhaseConst &ph, const N
     const double eta_lo = lower_viscosity<FP>(M, L, constant, eta_cst, elastic == 1, eta_el, gbs);
     GseIn g;
     g.Eii = Eii; g.eta_el = eta_el; g.eta_cst = eta_cst;
-    g.C_pwl = exp(-ph.pwl_n * (kLn2 + L.lnB_pwl)); g.n_pwl = ph.pwl_n;
-    g.C_lin = exp(-ph.lin_n * (kLn2 + L.lnB_lin)); g.n_lin = ph.lin_n; g.m_lin = ph.lin_m;
-    g.C_exp = exp(fma(L.n[K_EXP], log(ph.exp_s3gS), L.lnA_exp)); g.ST = L.ST; g.n_exp = ph.exp_n;
+    g.C_pwl = fx_exp_rare(-ph.pwl_n * (kLn2 + L.lnB_pwl)); g.n_pwl = ph.pwl_n;
+    g.C_lin = fx_exp_rare(-ph.lin_n * (kLn2 + L.lnB_lin)); g.n_lin = ph.lin_n; g.m_lin = ph.lin_m;
+    g.C_exp = fx_exp_rare(fma(L.n[K_EXP], fx_log_rare(ph.exp_s3gS), L.lnA_exp)); g.ST = L.ST; g.n_exp = ph.exp_n;
     g.eta_up = eta_up; g.eta_lo = eta_lo; g.Ag = Ag; g.gam = ph.Gpzm; g.lam = ph.Lpzm;
     g.cg = ph.cpzm; g.pg = ph.ppzm; g.elastic = elastic; g.constant = constant; g.dislocation = dislocation;
     g.peierls = peierls; g.diffusion = diffusion;
@@ -1334,7 +1385,7 @@ __device__ inline void iso_ve(const ModelConst &M, const PhaseConst &ph, const N
     Tii = 2.0 * eta_ve * Eii;
     double dd = o.d1;
     int st = MDZ_OK;
-    ve_gse(g, eta_ve, Tii, dd, e_cst, e_pwl, e_exp, e_lin, o.iters, st);
+    ve_gse<FP>(g, eta_ve, Tii, dd, e_cst, e_pwl, e_exp, e_lin, o.iters, st);
     set_status(o.status, st);
     o.d1 = dd;
     o.inv_d1 = 1.0 / dd;
@@ -1354,12 +1405,32 @@ __device__ inline void iso_ve(const ModelConst &M, const PhaseConst &ph, const N
 }
 
 // The Popov return (plastic == 2) of one (node, phase), into m.
+struct PopovIo {
+  double Tii, P, C, cos_fric, sin_fric, sin_dil, eta_ve, K;  // in
+  double Tn, Pc, lam_dot, A_tau, A_P, eta_vp;                 // in and out
+  int is_pl, status;                                          // out
+};
+static __device__ __noinline__ PopovIo popov_call(const ModelConst &M, const PhaseConst &ph, PopovIo q) {
+  q.status = MDZ_OK;
+  q.is_pl = plastic_popov(M, ph, q.Tii, q.P, q.C, q.cos_fric, q.sin_fric, q.sin_dil, q.eta_ve, q.K, q.Tn, q.Pc,
+                          q.lam_dot, q.A_tau, q.A_P, q.eta_vp, q.status);
+  return q;
+}
+
+template <class FP>
 __device__ __forceinline__ void popov_return(const ModelConst &M, const PhaseConst &ph, const NodeIn &in,
                                              const NodeCtx &c, const IsoState &S, PointOut &o, IsoMid &m) {
   int st = MDZ_OK;
   double Tn = m.Tii, A_P = 0.0;
-  m.is_pl = plastic_popov(M, ph, m.Tii, in.P, S.C, c.cos_fric, c.sin_fric, c.sin_dil, m.eta_ve, c.K, Tn, m.Pc,
-                          m.lam_dot, m.A_tau, A_P, m.eta_vp, st);
+  if (FP::kFixed) {
+    const PopovIo q = popov_call(M, ph, {m.Tii, in.P, S.C, c.cos_fric, c.sin_fric, c.sin_dil, m.eta_ve, c.K, m.Tii,
+                                         m.Pc, m.lam_dot, m.A_tau, 0.0, m.eta_vp, 0, 0});
+    m.is_pl = q.is_pl; m.Pc = q.Pc; m.lam_dot = q.lam_dot; m.A_tau = q.A_tau; m.eta_vp = q.eta_vp;
+    Tn = q.Tn; A_P = q.A_P; st = q.status;
+  } else {
+    m.is_pl = plastic_popov(M, ph, m.Tii, in.P, S.C, c.cos_fric, c.sin_fric, c.sin_dil, m.eta_ve, c.K, Tn, m.Pc,
+                            m.lam_dot, m.A_tau, A_P, m.eta_vp, st);
+  }
   set_status(o.status, st);
   if (m.is_pl) {
     m.eta_vep = Tn * c.inv2Eii;
@@ -1391,7 +1462,7 @@ __device__ inline void iso_post(const ModelConst &M, const PhaseConst &ph, const
   double eta_vp = m.eta_vp;
   if (is_pl && plastic == 1) o.Pcorr = Pc;
   if (plastic == 2) {
-    popov_return(M, ph, in, c, S, o, m);
+    popov_return<FP>(M, ph, in, c, S, o, m);
     is_pl = m.is_pl; Pc = m.Pc; lam_dot = m.lam_dot; A_tau = m.A_tau; eta_vp = m.eta_vp;
     if (is_pl) { o.Pcorr = Pc; eta_vep = m.eta_vep; Tii = m.Tii; divp = m.divp; }
   }
@@ -1696,16 +1767,16 @@ __device__ inline void aniso_finish(const ModelConst &M, const PhaseConst &ph, c
   if (fl & F_GS) {  // :429-473
     GseIn g;
     g.Eii = Eii; g.eta_el = eta_el; g.eta_cst = eta_cst;
-    g.C_pwl = exp(-ph.pwl_n * (kLn2 + L.lnB_pwl)); g.n_pwl = ph.pwl_n;
-    g.C_lin = exp(-ph.lin_n * (kLn2 + L.lnB_lin)); g.n_lin = ph.lin_n; g.m_lin = ph.lin_m;
-    g.C_exp = exp(fma(L.n[K_EXP], log(ph.exp_s3gS), L.lnA_exp)); g.ST = L.ST; g.n_exp = ph.exp_n;
+    g.C_pwl = fx_exp_rare(-ph.pwl_n * (kLn2 + L.lnB_pwl)); g.n_pwl = ph.pwl_n;
+    g.C_lin = fx_exp_rare(-ph.lin_n * (kLn2 + L.lnB_lin)); g.n_lin = ph.lin_n; g.m_lin = ph.lin_m;
+    g.C_exp = fx_exp_rare(fma(L.n[K_EXP], fx_log_rare(ph.exp_s3gS), L.lnA_exp)); g.ST = L.ST; g.n_exp = ph.exp_n;
     g.eta_up = eta_up; g.eta_lo = lower_viscosity<FP>(M, L, constant, eta_cst, elastic != 0, eta_el, false);
-    g.Ag = ph.Kpzm * exp(-ph.Qpzm / (M.R * T));
+    g.Ag = ph.Kpzm * fx_exp_rare(-ph.Qpzm / (M.R * T));
     g.gam = ph.Gpzm; g.lam = ph.Lpzm; g.cg = ph.cpzm; g.pg = ph.ppzm; g.elastic = elastic; g.constant = constant;
     g.dislocation = dislocation; g.peierls = peierls; g.diffusion = diffusion;
     double dd = in.d;
     int st = MDZ_OK;
-    ve_gse(g, eta_ve, Tii, dd, e_cst, e_pwl, e_exp, e_lin, o.iters, st);
+    ve_gse<FP>(g, eta_ve, Tii, dd, e_cst, e_pwl, e_exp, e_lin, o.iters, st);
     set_status(o.status, st);
     o.d1 = dd;
     o.inv_d1 = 1.0 / dd;

@@ -294,7 +294,7 @@ __device__ __forceinline__ void iso_accumulate(const SweepArgs &A, const Node &n
   const int fl = ph.flags;
   const int plastic = c.plastic_on ? ((fl & F_PL1) ? 1 : ((fl & F_PL2) ? 2 : 0)) : 0;
   if (plastic == 2) {
-    popov_return(M, ph, n.in, c, S, o, m);
+    popov_return<FxMath>(M, ph, n.in, c, S, o, m);
     if (m.is_pl) {
       m.pl_share = 2.0 * m.lam_dot * m.A_tau * m.eta_ve * FxMath::recip(m.Tii);
       m.T_over_eta = m.Tii * FxMath::recip(m.eta_ve);
