@@ -35,6 +35,9 @@ struct mdz_rheo_ctx {
   cudaStream_t own = nullptr, stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   DevStats *d_stats = nullptr, *h_stats = nullptr;
+  // d_stats holds its initial values: set when a call that waited has read them out
+  // (finish), cleared when any call starts (reset_stats)
+  bool stats_initial = false, recorded = false;
   std::vector<DevBuf> bufs;
   int32_t *d_iters_n = nullptr, *d_iters_s = nullptr;
   size_t cap_iters_n = 0, cap_iters_s = 0;
@@ -42,7 +45,7 @@ struct mdz_rheo_ctx {
   int last_np = 0, have_iters = 0, pending = 0;
   unsigned long long h2d = 0, d2h = 0;
   unsigned launches = 0;
-  // untuned shape, [iso, aniso]: the isotropic sweep compacts its plastic returns per CTA
+  // untuned shape, [iso, aniso]: both one thread per node
   LaunchShape shape[2] = {{128, 0, SHAPE_COMPACT}, {128, 0, SHAPE_THREAD}};
   // shapes the autotuner chose, keyed by (anisotropic, phases, reference start, nodes); a
   // sweep takes the entry of its key with the nearest node count, else shape[aniso]
@@ -244,7 +247,18 @@ int stats_from_device(mdz_rheo_ctx *ctx, mdz_sweep_stats *st, float ms) {
   return status;
 }
 
-int reset_stats(mdz_rheo_ctx *ctx) {
+// wait: the call ends with finish.  One that returns without waiting always carries its own
+// reset, since it may be recorded into a caller's graph; a graph's replays write d_stats
+// unseen, so from then on every call does.
+int reset_stats(mdz_rheo_ctx *ctx, bool wait) {
+  if (!wait && !ctx->recorded) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(ctx->stream, &cs));
+    ctx->recorded = cs != cudaStreamCaptureStatusNone;
+  }
+  const bool initial = ctx->stats_initial && !ctx->recorded;
+  ctx->stats_initial = false;
+  if (wait && initial) return MDZ_OK;
   DevStats init;
   memset(&init, 0, sizeof(init));
   init.err_key = ~0ull;
@@ -254,8 +268,9 @@ int reset_stats(mdz_rheo_ctx *ctx) {
 }
 
 int finish(mdz_rheo_ctx *ctx, mdz_sweep_stats *st) {
-  CK(cudaMemcpyAsync(ctx->h_stats, ctx->d_stats, sizeof(DevStats), cudaMemcpyDeviceToHost, ctx->stream));
+  CK(launch_stats_out(ctx->d_stats, ctx->h_stats, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
+  ctx->stats_initial = true;
   float ms = 0.f;
   cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
   return stats_from_device(ctx, st, ms);
@@ -597,7 +612,7 @@ int sweep_impl(mdz_rheo_ctx *ctx, const mdz_model *md, const mdz_materials *mat,
   const int bands = (host && mode < 0 && !(flags & MDZ_SWEEP_ITERS)) ? host_bands(ctx, md->Nz) : 1;
   if (bands > 1) {
     A.stats = ctx->d_stats;
-    if ((rc = reset_stats(ctx)) != MDZ_OK) return rc;
+    if ((rc = reset_stats(ctx, true)) != MDZ_OK) return rc;
     if ((rc = banded_sweep(ctx, A, aniso, L, f, bands)) != MDZ_OK) return rc;
     return finish(ctx, st);
   }
@@ -635,7 +650,7 @@ int sweep_impl(mdz_rheo_ctx *ctx, const mdz_model *md, const mdz_materials *mat,
     ctx->last_Nc = A.M.Nc; ctx->last_Nv = A.M.Nv; ctx->last_np = np;
   }
   A.stats = ctx->d_stats;
-  if ((rc = reset_stats(ctx)) != MDZ_OK) return rc;
+  if ((rc = reset_stats(ctx, !(flags & MDZ_SWEEP_ASYNC))) != MDZ_OK) return rc;
   // collected features / targets (device scratch when the caller's buffers are on the host)
   const size_t items = (size_t)np * (Nc + Nv);
   float *dX = X, *dY = Y;
@@ -1024,7 +1039,13 @@ int mdz_rheo_sync(mdz_rheo_ctx *c, mdz_sweep_stats *st) {
   if (!c) return MDZ_EINVAL;
   CK(cudaSetDevice(c->device));
   c->pending = 0;
-  return finish(c, st);
+  // the last call's statistics stay readable, however often they are asked for
+  if (!c->stats_initial)
+    CK(cudaMemcpyAsync(c->h_stats, c->d_stats, sizeof(DevStats), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  float ms = 0.f;
+  cudaEventElapsedTime(&ms, c->ev0, c->ev1);
+  return stats_from_device(c, st, ms);
 }
 
 int mdz_rheo_sweep(mdz_rheo_ctx *c, const mdz_model *md, const mdz_materials *m, const mdz_grid_fields *f,
@@ -1115,7 +1136,7 @@ int mdz_rheo_points(mdz_rheo_ctx *c, const mdz_model *md, const mdz_materials *m
     for (auto d : tmp) cudaFree(d);
     return MDZ_EINVAL;
   }
-  if ((rc = reset_stats(c)) != MDZ_OK) return rc;
+  if ((rc = reset_stats(c, true)) != MDZ_OK) return rc;
   c->launches = 1;
   CK(cudaEventRecord(c->ev0, c->stream));
   CK(launch_points(A, c->stream));
@@ -1369,7 +1390,7 @@ int mdz_rheo_batch_sweep(mdz_rheo_batch *b, mdz_sweep_stats *st) {
   if (!b) return MDZ_EINVAL;
   mdz_rheo_ctx *c = b->ctx;
   CK(cudaSetDevice(c->device));
-  int rc = reset_stats(c);
+  int rc = reset_stats(c, true);
   if (rc != MDZ_OK) return rc;
   c->h2d = c->d2h = 0;
   c->launches = batch_kernel_count(b->args);
@@ -1431,6 +1452,7 @@ int mdz_rheo_batch_launch(mdz_rheo_batch *b, mdz_sweep_stats *st) {
   CK(cudaSetDevice(c->device));
   c->h2d = c->d2h = 0;
   c->launches = (unsigned)b->graph_launches;
+  c->stats_initial = false;  // the graph resets and writes them
   CK(cudaEventRecord(c->ev0, c->stream));
   CK(cudaGraphLaunch(b->exec, c->stream));
   CK(cudaEventRecord(c->ev1, c->stream));
@@ -1458,8 +1480,7 @@ int mdz_rheo_autotune(mdz_rheo_ctx *c, const mdz_model *md, const mdz_materials 
     sweep_kernel_info(a, &regs, &smem, &occ, 128, SHAPE_QUEUE);
     cand.push_back({128, c->sms * (occ > 0 ? occ : 1), SHAPE_QUEUE});
   }
-  // the compacting form; the anisotropic sweep, which has no iterated plastic return, runs
-  // it as one thread per node
+  // the default form once more, under its own number (block 128 only)
   cand.push_back({128, 0, aniso ? SHAPE_THREAD : SHAPE_COMPACT});
   static_assert(MDZ_AUTOTUNE_CANDIDATES == 13, "candidate list");
   const LaunchShape keep = c->shape[a];
@@ -1584,7 +1605,7 @@ int mdz_rheo_operators(mdz_rheo_ctx *ctx, const mdz_model *md, const mdz_materia
   }
   if (mi.err) return mi.err;
   A.stats = ctx->d_stats;
-  if ((rc = reset_stats(ctx)) != MDZ_OK) return rc;
+  if ((rc = reset_stats(ctx, true)) != MDZ_OK) return rc;
   CK(cudaEventRecord(ctx->ev0, ctx->stream));
   CK(launch_operators(A, anis, jac, !(flags & MDZ_OPS_PER_NODE), ctx->stream));
   ctx->launches = 1;
@@ -1631,7 +1652,7 @@ int mdz_rheo_strain_rates(mdz_rheo_ctx *ctx, const mdz_model *md, double dx, dou
   }
   if (mi.err) return mi.err;
   int rc;
-  if ((rc = reset_stats(ctx)) != MDZ_OK) return rc;
+  if ((rc = reset_stats(ctx, !(flags & MDZ_SWEEP_ASYNC))) != MDZ_OK) return rc;
   CK(cudaEventRecord(ctx->ev0, ctx->stream));
   CK(launch_strain_rates(A, ctx->stream));
   ctx->launches = 1;
@@ -1752,7 +1773,7 @@ int mdz_rheo_marker_stress(mdz_rheo_ctx *ctx, const mdz_model *md, const mdz_mar
   A.near_z = near(A.dz_itp.b);
   A.stats = ctx->d_stats;
   int rc;
-  if ((rc = reset_stats(ctx)) != MDZ_OK) return rc;
+  if ((rc = reset_stats(ctx, !(flags & MDZ_SWEEP_ASYNC))) != MDZ_OK) return rc;
   CK(cudaEventRecord(ctx->ev0, ctx->stream));
   if (el || dir) {
     CK(launch_marker_grid(A, ctx->stream));
@@ -1841,7 +1862,7 @@ int mdz_rheo_p2mastah(mdz_rheo_ctx *ctx, const mdz_model *md, const mdz_marker_g
   A.sum_s = node_s ? (double *)ctx->bufs[S_P2M + 11].p : nullptr;
   A.stats = ctx->d_stats;
   int rc;
-  if ((rc = reset_stats(ctx)) != MDZ_OK) return rc;
+  if ((rc = reset_stats(ctx, !(flags & MDZ_SWEEP_ASYNC))) != MDZ_OK) return rc;
   if (node_n) CK(cudaMemsetAsync(A.sum_n, 0, 2 * Nc * sizeof(double), ctx->stream));
   if (node_s) CK(cudaMemsetAsync(A.sum_s, 0, 2 * Nv * sizeof(double), ctx->stream));
   CK(cudaEventRecord(ctx->ev0, ctx->stream));
@@ -1898,7 +1919,7 @@ int mdz_rheo_softening(mdz_rheo_ctx *ctx, const mdz_model *md, const mdz_prep_ma
   if (mi.err) return mi.err;
   A.fric_n = dev[0]; A.dil_n = dev[1]; A.C_n = dev[2]; A.fric_s = dev[3]; A.dil_s = dev[4]; A.C_s = dev[5];
   int rc;
-  if ((rc = reset_stats(ctx)) != MDZ_OK) return rc;
+  if ((rc = reset_stats(ctx, !(flags & MDZ_SWEEP_ASYNC))) != MDZ_OK) return rc;
   CK(cudaEventRecord(ctx->ev0, ctx->stream));
   CK(launch_softening(A, ctx->stream));
   ctx->launches = 1;
@@ -1946,7 +1967,7 @@ int mdz_rheo_shear_modulus(mdz_rheo_ctx *ctx, const mdz_model *md, const mdz_pre
   A.mu_n = dev[0]; A.bet_n = dev[1]; A.alp_n = dev[2]; A.mu_s = dev[3]; A.bet_s = dev[4];
   A.stats = ctx->d_stats;
   int rc;
-  if ((rc = reset_stats(ctx)) != MDZ_OK) return rc;
+  if ((rc = reset_stats(ctx, !(flags & MDZ_SWEEP_ASYNC))) != MDZ_OK) return rc;
   CK(cudaEventRecord(ctx->ev0, ctx->stream));
   CK(launch_moduli(A, ctx->stream));
   ctx->launches = 1;

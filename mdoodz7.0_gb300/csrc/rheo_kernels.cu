@@ -178,6 +178,25 @@ cudaError_t launch_points(const PointArgs &a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
+// A synchronous call's last launch: the statistics to the host's page-locked copy, and the
+// device's back to their initial values for the next call.  In place of one transfer by the
+// copy engine before and one after the kernels of every call, which a small call waits for:
+// 68.3 -> 62.7 us for the 201 x 201 sweep, 91 -> 86 us for the strain rates of 1025 x 1025.
+__global__ void k_stats_out(DevStats *d, DevStats *host) {
+  *host = *d;
+  DevStats init = {};
+  init.err_key = ~0ull;
+  *d = init;
+}
+
+cudaError_t launch_stats_out(DevStats *d, DevStats *host, cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(1);
+  cfg.blockDim = dim3(1);
+  cfg.stream = s;
+  return cudaLaunchKernelEx(&cfg, k_stats_out, d, host);
+}
+
 void sweep_kernel_info(int aniso, int *regs, int *smem, int *max_blocks_per_sm, int block, int form) {
   cudaFuncAttributes fa;
   // the centroid kernel: the larger of the two, it sets the launch shape

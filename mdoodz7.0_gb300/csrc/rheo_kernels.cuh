@@ -120,6 +120,7 @@ cudaError_t launch_sweep_tiles(const SweepArgs &a, const WarmArgs &w, bool aniso
 // the learned warm start evaluated per warp (mlp_warp.cuh): one launch per kind of node
 cudaError_t launch_sweep_warm(const SweepArgs &a, const MlpDevice &w, bool aniso, cudaStream_t s);
 int tiles_blocks_per_sm(bool aniso, int mode);
+cudaError_t launch_stats_out(DevStats *d, DevStats *host, cudaStream_t s);
 void sweep_kernel_info(int aniso, int *regs, int *smem, int *max_blocks_per_sm, int block, int form);
 
 }  // namespace mdz
