@@ -33,7 +33,7 @@ struct OpNode {
 // as point_iso, so the same bits.
 template <bool ANISO, bool COMPACT>
 __device__ __forceinline__ void phase_loop(const OpArgs &A, const OpNode &nd, bool has, const NodeIn &in,
-                                           const NodeCtx &ctx, const AnisoNode &an, int is_centroid, double sign,
+                                           const NodeCtx &ctx, const AnisoNode &an, int is_centroid, bool minus,
                                            const Divisor &denom, double &detadE, double &ddivpdE, double &danidE,
                                            double *drhodP, CompactQueue *Q, int *par, FdLaw *laws, bool fresh) {
   for (int p = 0; p < A.M.np; p++) {
@@ -62,18 +62,18 @@ __device__ __forceinline__ void phase_loop(const OpArgs &A, const OpNode &nd, bo
     const double eta_vep = o.etaVE;
     const int avg = A.M.eta_average;
     // the quotients by the step, correctly rounded (fp64_div.cuh)
-    const double sv = sign * vol, de = div_by_fp64(sv * eta_vep, denom);
+    const double sv = __longlong_as_double((long long)(fp64_bits(vol) ^ (minus ? 1ull << 63 : 0ull)));
+    const double de = div_by_fp64(sv * eta_vep, denom);
     if (avg == 0) detadE += de;
     else {
       const double ep = nd.centroid ? A.peta_n[p][nd.idx] : A.peta_s[p][nd.idx];
       if (avg == 1) detadE += de / (ep * ep);
       else detadE += de / ep;
     }
-    danidE += div_by_fp64(sv, denom);
-    if (is_centroid > 0) {  // a zero correction (no dilation) adds a zero
-      const double dv = sv * o.div_pl;
-      if (!(fp64_is_zero(dv) && denom.fast)) ddivpdE += div_by_fp64(dv, denom);
-    }
+    // the isotropic centroids' coefficients multiply danidE by zero (newton_store's Axx, Azz)
+    if (ANISO || is_centroid == 0) danidE += div_by_fp64(sv, denom);
+    if (is_centroid > 0 && !(fp64_is_zero(o.div_pl) && denom.fast))  // no dilation: a zero
+      ddivpdE += div_by_fp64(sv * o.div_pl, denom);
     if (in.want_rho) *drhodP += div_by_fp64(sv * o.rho, denom);
   }
 }
@@ -118,7 +118,7 @@ __device__ __forceinline__ void fd_derivatives(const OpArgs &A, const OpNode &nd
         else node_strain_iso<FdMath>(A.M, in, ctx);
         node_strain_update<FdMath>(ctx);
       }
-      phase_loop<ANISO, COMPACT>(A, nd, has, in, ctx, an, is_centroid, sign, denom, d[dir],
+      phase_loop<ANISO, COMPACT>(A, nd, has, in, ctx, an, is_centroid, s == 1, denom, d[dir],
                                  nd.centroid ? v[dir] : vscratch, a[dir], &drhodp, Q, par,
                                  COMPACT && dir < 3 ? laws : nullptr, !COMPACT || dir == 3 || (dir == 0 && s == 0));
     }
@@ -311,11 +311,13 @@ __global__ void __launch_bounds__(128, ANISO ? 3 : 4) k_operators(const __grid_c
 // The isotropic Newton operator with its Drucker-Prager returns compacted per CTA: the
 // node loop, the 8 perturbations and the phase loop are uniform over the CTA, and the
 // returns of each phase's yielding items run packed into the first warps (dp_compact).
-// The same bits as k_operators<false, true>.  Per perturbed solve it takes about 100 FP64
+// The same bits as k_operators<false, true>.  Per perturbed solve it takes about 92 FP64
 // instructions (149 before the convergence test of the default start moved to fixed point,
-// the quotients by the step to the known-divisor form, and the strain-rate-independent part
-// of the laws out of the strain-rate perturbations: 513 x 513 cells 6.98 -> 5.44 ms).  CTAs
-// per SM: 5.59, 5.44 and 5.41 ms at 5, 6 and 8.
+// the quotients by the step to the known-divisor form, the strain-rate-independent part of
+// the laws out of the strain-rate perturbations, and the quotients that the coefficients
+// multiply by zero went: 513 x 513 cells 6.98 -> 5.30 ms).  CTAs per SM: 5.59, 5.44 and 5.41
+// ms at 5, 6 and 8 (before the last of these), 5.43 at 4 after it.  CTAs of 64 take 6.01 ms,
+// the returns in their own threads 5.88.
 __global__ void __launch_bounds__(128, 6) k_operators_compact(const __grid_constant__ OpArgs A) {
   __shared__ CompactQueue Q;
   compact_init(Q);
