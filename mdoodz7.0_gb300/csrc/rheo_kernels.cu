@@ -8,15 +8,8 @@
 // its own kind's work (vertices skip the per-phase outputs only centroids keep), per-phase
 // tables in the kernel's constant parameter bank (uniform across a warp, so every lookup
 // is a broadcast), SoA loads and stores coalesced along the node index.  k_sweep_queue is
-// the same sweep as a persistent grid on a work counter; k_sweep_warm puts the learned
-// warm start (evaluated per warp on the tensor cores) before each local solve;
-// k_sweep_batch sweeps many grids in one launch per kind of node.
-//
-// k_sweep_tiles<ANISO, MODE, NODES> walks the same index space in tiles of 128 nodes, one tile
-// per CTA at a time, with the phase loop uniform over the CTA so that a block-wide stage
-// can sit between each phase's set-up and its local solve: the learned warm start
-// (MODE_WARM: the tcgen05 network's guess, then the start stages) or the training-data dump
-// (MODE_COLLECT, from the reference's own start).
+// the same sweep as a persistent grid on a work counter.  The warm-start forms are in
+// sweep_warm.cu, many grids per launch in sweep_batch.cu.
 #include <cuda_runtime.h>
 
 #include "sweep_node.cuh"
@@ -25,15 +18,18 @@ namespace mdz {
 
 // One sweep is two launches: the centroids (NODES 1), then the vertices (NODES 2), each
 // over its whole range or over the band of rows a banded sweep gives it.
-// MINB: CTAs of 128 per SM that the register allocation is capped for.  6 (80 registers, with
-// spills) by default: a node's code is a long chain of dependent integer and FP64
-// instructions, and more resident warps hide more of its latency than the spills cost.  At 4,
-// 6 and 8 CTAs per SM the isotropic sweep (5 phases) took 157.7, 134.7 and 137.8 us at 201 x
-// 201 cells, 595, 571 and 535 us at 513 x 513, 2107, 1956 and 1975 us at 1025 x 1025, the
-// anisotropic one (3 phases) 108.8, 94.1 and 94.2 us, 394, 380 and 365 us, 1416, 1324 and
-// 1297 us.  2 (255 registers, no spills) wins where local solves take many FP64 evaluations;
-// the autotuner times both.
-template <bool ANISO, int NODES, int MINB = 6>
+// MINB: CTAs of 128 per SM that the register allocation is capped for.  A node's code is a
+// long chain of dependent integer and FP64 instructions, and more resident warps hide more of
+// its latency than the spills cost: 7 (72 registers) by default.  A sweep of a few waves
+// loses more to its last, partly empty one, and 5 (96 registers) wins there (sweep_ctas).
+// Per call, in us, at 5, 6, 7 and 8 CTAs per SM:
+//   isotropic, 5 phases     201^2: 124, 126, 124, 121    401^2: 328, 344, 351, 347
+//     513^2: 493, 505, 446, 463    717^2: 937, 903, 840, 885    1025^2: 1862, 1787, 1703, 1757
+//   anisotropic, 3 phases   201^2: 94, 91, 91, 90        401^2: 253, 261, 270, 255
+//     513^2: 377, 375, 355, 364    717^2: 695, 667, 651, 656    1025^2: 1357, 1303, 1283, 1264
+// 2 (255 registers, no spills) is for local solves of many FP64 evaluations; the autotuner
+// times it too.
+template <bool ANISO, int NODES, int MINB>
 __global__ void __launch_bounds__(128, MINB) k_sweep(const __grid_constant__ SweepArgs A) {
   if (NODES == 1) pair_begin();
   Acc acc = {0, 0, 0, 0, 0};
@@ -139,17 +135,29 @@ static cudaError_t launch_after(K fn, unsigned grid, int block, cudaStream_t s, 
   return cudaLaunchKernelEx(&cfg, fn, a);
 }
 
+// CTAs of 128 per SM for a sweep of so many nodes, centroids and vertices together (their
+// kernels overlap): 5 between one and 3.5 waves of the 152 SMs' 7 CTAs, where the last wave's
+// idle SMs cost more than the fifth to seventh CTA's warps gain (517 x 389 cells with air, 3
+// waves: 289, 300 and 308 us at 5, 6 and 7; 513 x 513, 3.9 waves: 493, 505 and 446).
+static int sweep_ctas(long long nodes) {
+  const long long wave = 152LL * 7 * 128;
+  return (nodes > wave && 2 * nodes < 7 * wave) ? 5 : 7;
+}
+
 template <bool ANISO, int NODES>
-static cudaError_t launch_kind(const SweepArgs &a, const LaunchShape &sh, long long count, cudaStream_t s, bool after) {
+static cudaError_t launch_kind(const SweepArgs &a, const LaunchShape &sh, long long count, long long nodes,
+                               cudaStream_t s, bool after) {
   if (sh.form == SHAPE_QUEUE) {
     k_sweep_queue<ANISO, NODES><<<(unsigned)sh.grid_cap, 128, 0, s>>>(a);
     return cudaGetLastError();
   }
   const int block = sh.form == SHAPE_COMPACT ? 128 : sh.block;  // SHAPE_COMPACT: the default, one thread per node
   long long grid = (count + block - 1) / block;
+  const bool few = sh.grid_cap <= 0 && sweep_ctas(nodes) == 5;
   if (sh.grid_cap > 0 && grid > sh.grid_cap) grid = sh.grid_cap;
   if (sh.form == SHAPE_REGS255) return launch_after(k_sweep<ANISO, NODES, 2>, (unsigned)grid, block, s, after, a);
-  return launch_after(k_sweep<ANISO, NODES, 6>, (unsigned)grid, block, s, after, a);
+  if (few) return launch_after(k_sweep<ANISO, NODES, 5>, (unsigned)grid, block, s, after, a);
+  return launch_after(k_sweep<ANISO, NODES, 7>, (unsigned)grid, block, s, after, a);
 }
 
 cudaError_t launch_sweep(const SweepArgs &a, bool aniso, cudaStream_t s, const LaunchShape &shape) {
@@ -162,10 +170,10 @@ cudaError_t launch_sweep(const SweepArgs &a, bool aniso, cudaStream_t s, const L
     if (counts[kind] <= 0) continue;
     cudaError_t e;
     const bool after = kind == 1 && counts[0] > 0 && sh.form != SHAPE_QUEUE;
-    if (kind == 0 && aniso) e = launch_kind<true, 1>(a, sh, counts[kind], s, false);
-    else if (kind == 0) e = launch_kind<false, 1>(a, sh, counts[kind], s, false);
-    else if (aniso) e = launch_kind<true, 2>(a, sh, counts[kind], s, after);
-    else e = launch_kind<false, 2>(a, sh, counts[kind], s, after);
+    if (kind == 0 && aniso) e = launch_kind<true, 1>(a, sh, counts[kind], counts[0] + counts[1], s, false);
+    else if (kind == 0) e = launch_kind<false, 1>(a, sh, counts[kind], counts[0] + counts[1], s, false);
+    else if (aniso) e = launch_kind<true, 2>(a, sh, counts[kind], counts[0] + counts[1], s, after);
+    else e = launch_kind<false, 2>(a, sh, counts[kind], counts[0] + counts[1], s, after);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -200,7 +208,7 @@ cudaError_t launch_stats_out(DevStats *d, DevStats *host, cudaStream_t s) {
 void sweep_kernel_info(int aniso, int *regs, int *smem, int *max_blocks_per_sm, int block, int form) {
   cudaFuncAttributes fa;
   // the centroid kernel: the larger of the two, it sets the launch shape
-  const void *fn = aniso ? (const void *)k_sweep<true, 1, 6> : (const void *)k_sweep<false, 1, 6>;
+  const void *fn = aniso ? (const void *)k_sweep<true, 1, 7> : (const void *)k_sweep<false, 1, 7>;
   if (form == SHAPE_REGS255) fn = aniso ? (const void *)k_sweep<true, 1, 2> : (const void *)k_sweep<false, 1, 2>;
   if (form == SHAPE_QUEUE) fn = aniso ? (const void *)k_sweep_queue<true, 1> : (const void *)k_sweep_queue<false, 1>;
   cudaFuncGetAttributes(&fa, fn);

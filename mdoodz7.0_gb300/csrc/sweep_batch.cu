@@ -28,10 +28,10 @@ __device__ __forceinline__ int batch_grid_of(const long long *tile_start, int n,
 // start (WARM) is evaluated per warp as in k_sweep_warm.  PERTURB: the strain rates are
 // multiplied by the sweep's perturbation factors as they are loaded, in place (the
 // captured multi-sweep graph), instead of by a separate pass over them.
-// 6 CTAs per SM (80 registers), as the single grid's kernels: 16 grids of 65-513 cells a side,
-// 5 captured sweeps, took 6.98, 6.60 and 6.62 ms at 4, 6 and 8.
+// 7 CTAs per SM (72 registers), as a large single grid's kernels: 16 grids of 65-513 cells a
+// side, 5 captured sweeps, took 5.41, 5.18, 5.04 and 5.25 ms at 5, 6, 7 and 8.
 template <bool ANISO, int NODES, bool WARM, bool PERTURB>
-__global__ void __launch_bounds__(kBatchTile, 6) k_sweep_batch(const __grid_constant__ BatchArgs B,
+__global__ void __launch_bounds__(kBatchTile, WARM ? 6 : 7) k_sweep_batch(const __grid_constant__ BatchArgs B,
                                                              const __grid_constant__ BatchSweepArgs X) {
   extern __shared__ __align__(16) unsigned char smem_batch[];
   MlpWarpShared &S = *reinterpret_cast<MlpWarpShared *>(smem_batch);
