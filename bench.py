@@ -52,37 +52,35 @@ UNIT = "point-updates/s"
 
 # FP64 work of the sweep per point-update, in flops (DFMA = 2, DADD/DMUL = 1): ncu's
 # thread-level FP64 instruction counters of one sweep's two launches (centroids, then
-# vertices; default start, default form: k_sweep_compact for the isotropic sweep, k_sweep
-# for the anisotropic one), summed, on the same field distributions at 513 x 513 cells
-# (527,365 nodes), per workload (profiles/k_sweep_plain_large_513.md,
-# profiles/k_sweep_aniso_513.md).  `roofline.achieved` = this x nodes / the CUDA-event
+# vertices; default start, default form), summed, on the same field distributions at 513 x
+# 513 cells (527,365 nodes), per workload (profiles/kernels_fixed_point.md).  `roofline.achieved` = this x nodes / the CUDA-event
 # time of one sweep (events before the first launch and after the second).
-FP64_FLOPS_PER_POINT = {"plain_large": 1448.7, "aniso": 1038.4}
+FP64_FLOPS_PER_POINT = {"plain_large": 292.2, "aniso": 379.9}
 # FP64 work of the batched many-grid sweep per local solve (phase call), same convention:
 # the two k_sweep_batch launches of one sweep of an 8-grid batch of the many-grid
-# distribution (5,096,155 phase calls; profiles/k_sweep_batch_many_grids.md); the grids
+# distribution (5,096,155 phase calls; profiles/kernels_fixed_point.md); the grids
 # have 2 to 5 phases, so the work is counted per phase call.
-FP64_FLOPS_PER_PHASE_CALL = {"many_grids": 288.8}
+FP64_FLOPS_PER_PHASE_CALL = {"many_grids": 59.9}
 # DRAM bytes (read + write) per point-update of one sweep's two launches at 1025 x 1025
-# cells (0.7 GB of fields, five times L2; profiles/k_sweep_spills_and_dram_1025.md: the
-# default forms at 4 CTAs per SM, whose register spills reach DRAM in part), scaled to a
+# cells (0.7 GB of fields, five times L2; profiles/kernels_fixed_point.md: the default
+# forms at 7 CTAs per SM, whose register spills reach DRAM in part), scaled to a
 # sweep by its node count.
-DRAM_BYTES_PER_POINT = {"plain_large": 414.6, "aniso": 364.2}
+DRAM_BYTES_PER_POINT = {"plain_large": 1038.8, "aniso": 704.0}
 # FP64 work of k_marker_update per marker (inactive ones included), same convention:
 # thread-level counters of one launch at 513 x 513 cells with 16 markers per cell
-# (4,210,704 markers) per option set (profiles/k_marker_update_513.md).
-FP64_FLOPS_PER_MARKER = {"jaumann_stencil1": 90.48, "analytical_director_stencil9": 218.31}
+# (4,210,704 markers) per option set (profiles/kernels_fixed_point.md).
+FP64_FLOPS_PER_MARKER = {"jaumann_stencil1": 36.41, "analytical_director_stencil9": 157.93}
 # FP64 work of the Newton operator per perturbed local solve, same convention: one launch of
 # k_operators_compact at 513 x 513 cells (21,094,600 perturbed solves;
-# profiles/k_operators_newton_257.md).
-FP64_FLOPS_PER_OPERATOR_SOLVE = 224.7
+# profiles/kernels_fixed_point.md).
+FP64_FLOPS_PER_OPERATOR_SOLVE = 128.0
 # FP64-pipe thread instructions (DFMA, DADD, DMUL and the few conversions; each takes a
 # pipe slot whether it carries two flops or one) per unit, from the same captures:
 # `fp64_issue_frac` = this x units / time / (measured DFMA rate / 2) is how busy the FP64
 # pipe is with useful lanes, the figure the flop fraction understates by the DADD/DMUL share.
-FP64_THREAD_INSTS = {"plain_large": 954.4, "aniso": 671.0, "many_grids": 190.0,
-                     "jaumann_stencil1": 77.23, "analytical_director_stencil9": 183.50,
-                     "newton_operator": 148.7}
+FP64_THREAD_INSTS = {"plain_large": 206.3, "aniso": 252.5, "many_grids": 42.4,
+                     "jaumann_stencil1": 36.38, "analytical_director_stencil9": 139.27,
+                     "newton_operator": 87.7}
 
 
 def issue_frac(insts_per_unit, units, ms, peak_tflops):
@@ -1082,10 +1080,7 @@ def main():
                        "parallelism": f"{ws} independent grid(s), one per GPU"},
             "roofline": roof, "cpu_baseline": cpu, "e2e": e2e, "clocks": clk_summary,
             "gpu_launches": launches, "kernel_ms_per_sweep": launch_ms,
-            "sweep_kernels": ("k_sweep over the centroids, then k_sweep over the vertices: 2 launches per sweep"
-                              if aniso else
-                              "k_sweep_compact over the centroids, then k_sweep_compact over the vertices "
-                              "(plastic returns compacted per CTA): 2 launches per sweep"),
+            "sweep_kernels": "k_sweep over the centroids, then k_sweep over the vertices: 2 launches per sweep",
             "median_kernel_ms_per_sweep": statistics.median(kernel_ms),
             "reference_start": ref_r, "warm_start": warm, "autotune": tune, "newton_operator": newton_op,
             "strain_rates": strain, "input_preparation": prep, "marker_stress": markers, "configs": configs}

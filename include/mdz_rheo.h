@@ -568,17 +568,16 @@ int mdz_rheo_batch_set_grid(mdz_rheo_batch *batch, int ctas);
  * context of the same kind: anisotropic or not, phase count, start (MDZ_SWEEP_REF_START or
  * not) and, among tuned sizes, the nearest node count (a cache keyed by those; other
  * sweeps use the last shape tuned for their kind, aniso 0/1).  Candidates, in this order:
- *   0-4   128 threads per block, 4 CTAs per SM (128 registers): one thread per node, then a
+ *   0-4   128 threads per block, 7 CTAs per SM (72 registers; 5 for one thread
+ *         per node of a middling grid): one thread per node, then a
  *         grid-stride loop over 1, 2, 4 or 8 waves of the resident CTAs;
  *   5-9   the same with 64 threads per block;
  *   10    128 threads per block, one thread per node, 2 CTAs per SM (255 registers, no
  *         spills);
  *   11    persistent: one wave of resident CTAs whose warps pull 32-node chunks from a
  *         work counter (one atomic per chunk, lanes past the end retired by a ballot);
- *   12    compacting (isotropic): the CTA's threads walk their nodes' phases in step and,
- *         after each phase's visco-elastic solve, run the Drucker-Prager returns of the
- *         yielding items packed into the first threads (gathered by ballot into shared
- *         memory); the anisotropic sweep runs this candidate as one thread per node.
+ *   12    the form that sweeps take untuned: candidate 0's kernel, at 128 threads per block
+ *         only (its own form number for the isotropic sweep).
  * Each candidate runs one warm-up and `reps` timed sweeps; ms_out (may be NULL) receives
  * MDZ_AUTOTUNE_CANDIDATES mean kernel times and best_out (may be NULL) the chosen index.
  * No candidate changes a result bit: every node is computed by the same code, by one
@@ -589,9 +588,9 @@ int mdz_rheo_batch_set_grid(mdz_rheo_batch *batch, int ctas);
 int mdz_rheo_autotune(mdz_rheo_ctx *ctx, const mdz_model *model, const mdz_materials *mat,
                       const mdz_grid_fields *f, int aniso, int flags, int reps, double *ms_out,
                       int *best_out);
-/* The kernel form of that shape: 0 one thread per node or grid-stride (128 registers),
- * 1 the 255-register form, 2 the persistent work-counter form, 3 the compacting form
- * (isotropic, block 128). */
+/* The kernel form of that shape: 0 one thread per node or grid-stride (72 or 96 registers),
+ * 1 the 255-register form, 2 the persistent work-counter form, 3 the untuned isotropic
+ * sweep's form (one thread per node, block 128). */
 int mdz_rheo_get_launch_form(mdz_rheo_ctx *ctx, int aniso, int *form);
 /* Set the shape of sweeps of this kind by hand (block 64 or 128, grid cap as above, form
  * 0/1/2; form 2 with grid_cap 0 takes one wave of resident CTAs), dropping the tuned

@@ -3,9 +3,11 @@
 // One call of `point_iso` is one ViscosityConcise (MDLIB/RheologyDensity.c:385-1080);
 // `point_aniso` is ViscosityConciseAniso (MDLIB/AnisotropyRoutines.c:282-727).
 //
-// GB300 issues FP64 at 1/64 of its FP32 rate, and this path is bound by the FP64 pipe,
-// so the formulation minimises FP64 instructions while keeping every quantity
-// well conditioned:
+// GB300 issues FP64 at 1/64 of its FP32 rate: one FP64 instruction of a warp costs an SM
+// about as much as 15 to 40 integer ones.  So the formulation minimises FP64 instructions
+// while keeping every quantity well conditioned, and the sweeps and points (FxMath) run the
+// elementary functions and the local solve in 64-bit fixed point (fx64.cuh, ve_fx.cuh); the
+// operators (FdMath) keep the FP64 forms, whose last bits their difference quotients show:
 //  * per-phase constants (log pre-factors, 1/(R n), 1/n, ...) are folded on the host;
 //  * each creep law k is carried as the logarithm of the reciprocal of its isolated
 //    viscosity at the node's strain rate, ln(1/eta_k), a sum of well-conditioned logs
@@ -1221,19 +1223,19 @@ struct IsoMid {
   double eta_ve, Tii, Tii_ve, Tyield, e_cst, e_pwl, e_exp, e_lin;  // e_*: over Eii (sweeps, points)
   double gdot, divp, Pc, eta_vep, lam_dot, A_tau, A_P, eta_vp;
   int is_pl;
-  // what the sweeps' averages need of a yielding item (dp_extra): eta_ve gdot / Tii (the
+  // what the sweeps' averages need of a yielding item: eta_ve gdot / Tii (the
   // plastic rate beside the creep rates, over the stress) and Tii / eta_ve
   double pl_share, T_over_eta;
 };
 
 // Inputs and results of the Drucker-Prager return of one (node, phase) (plastic == 1,
 // RheologyDensity.c:655-707).  It depends only on these and on the phase's constants, so a
-// CTA can run the returns of all its yielding items together, one per thread
-// (k_sweep_compact), with the bits of the inline return.
+// CTA can run the returns of all its yielding items together, one per thread (dp_compact),
+// with the bits of the inline return.
 struct DpItem {
   double Tii, Tyield, eta_ve, P, K, sin_fric, sin_dil, Eii, inv2Eii;  // in; Tii, Tyield out
   double gdot, divp, Pc, eta_vp, eta_vep;                              // out
-  double pl_share, T_over_eta;                                         // out (dp_extra)
+  double pl_share, T_over_eta;                                         // out (dp_return_call)
 };
 
 __device__ __forceinline__ bool iso_yields_dp(const ModelConst &M, const PhaseConst &ph, const NodeCtx &c,
@@ -1251,7 +1253,6 @@ __device__ __forceinline__ void dp_store(IsoMid &m, const DpItem &d) {
   m.is_pl = 1;
   m.Tii = d.Tii; m.Tyield = d.Tyield; m.gdot = d.gdot; m.divp = d.divp; m.Pc = d.Pc; m.eta_vp = d.eta_vp;
   m.eta_vep = d.eta_vep;
-  m.pl_share = d.pl_share; m.T_over_eta = d.T_over_eta;
 }
 
 // The Drucker-Prager return (:655-707) of an item that yields (Tii - Tyield > 1e-17).
@@ -1344,6 +1345,7 @@ __device__ __forceinline__ void dp_return_inline(const ModelConst &M, const Phas
   dp_load(d, m, in, c);
   d = dp_return_call(M, ph, d);
   dp_store(m, d);
+  m.pl_share = d.pl_share; m.T_over_eta = d.T_over_eta;
 }
 
 // Local solve (from s_start * eta_up, moved by the start stages that the descriptor
@@ -1563,7 +1565,9 @@ __device__ inline void point_iso(const ModelConst &M, const PhaseConst &ph, cons
   iso_finish<FP>(M, ph, in, c, S, 1.0f, polish, o);
 }
 
-// CTA-level compaction of the Drucker-Prager returns.  The return of an item that yields
+// CTA-level compaction of the Drucker-Prager returns (the Newton operator, whose returns keep
+// the iteration's bits; the sweeps' take nine FP64 instructions and stay in their own thread,
+// dp_return_inline).  The return of an item that yields
 // takes a few iterations with a division each, and about one item in eleven yields: inline,
 // nearly every warp carries one or two yielding lanes through the return while the other
 // lanes wait.  A kernel whose CTA (at most 128 threads) walks its items' phases in step

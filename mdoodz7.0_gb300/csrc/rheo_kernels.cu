@@ -27,8 +27,9 @@ namespace mdz {
 //     513^2: 493, 505, 446, 463    717^2: 937, 903, 840, 885    1025^2: 1862, 1787, 1703, 1757
 //   anisotropic, 3 phases   201^2: 94, 91, 91, 90        401^2: 253, 261, 270, 255
 //     513^2: 377, 375, 355, 364    717^2: 695, 667, 651, 656    1025^2: 1357, 1303, 1283, 1264
-// 2 (255 registers, no spills) is for local solves of many FP64 evaluations; the autotuner
-// times it too.
+// 2 (255 registers, no spills) is the form that callers may ask for and the autotuner times:
+// 2049 x 2049 cells 8.33 ms for 6.72, from the reference's start (1 to 8 evaluations) 28.3
+// for 25.8.
 template <bool ANISO, int NODES, int MINB>
 __global__ void __launch_bounds__(128, MINB) k_sweep(const __grid_constant__ SweepArgs A) {
   if (NODES == 1) pair_begin();

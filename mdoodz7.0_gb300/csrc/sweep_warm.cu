@@ -32,7 +32,10 @@ __global__ void __launch_bounds__(128, 4) k_sweep_warm(const __grid_constant__ S
 // tiled sweep with a block-wide stage per phase (learned warm start / data collection)
 // ---------------------------------------------------------------------------------
 // NODES 1 sweeps the centroids, NODES 2 the vertices (one launch each, with the node
-// bodies of the plain sweep's two kernels).
+// bodies of the plain sweep's two kernels).  A tile is one CTA's, its phase loop uniform over
+// the CTA, so that a block-wide stage can sit between each phase's set-up and its local
+// solve: the tcgen05 network's guess (MODE_WARM) or the dump of training pairs from the
+// reference's own start (MODE_COLLECT).
 template <bool ANISO, int MODE, int NODES>
 __global__ void __launch_bounds__(128, 2) k_sweep_tiles(const __grid_constant__ SweepArgs A,
                                                      const __grid_constant__ WarmArgs W) {
