@@ -36,7 +36,9 @@ struct mdz_rheo_ctx {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   DevStats *d_stats = nullptr, *h_stats = nullptr;
   // d_stats holds its initial values: set when a call that waited has read them out
-  // (finish), cleared when any call starts (reset_stats)
+  // (finish), cleared when any call starts (reset_stats).  recorded: a call of this context
+  // was captured into a caller's graph, whose replays write d_stats unseen; stats_initial
+  // stays false from then on.
   bool stats_initial = false, recorded = false;
   std::vector<DevBuf> bufs;
   int32_t *d_iters_n = nullptr, *d_iters_s = nullptr;
@@ -248,15 +250,14 @@ int stats_from_device(mdz_rheo_ctx *ctx, mdz_sweep_stats *st, float ms) {
 }
 
 // wait: the call ends with finish.  One that returns without waiting always carries its own
-// reset, since it may be recorded into a caller's graph; a graph's replays write d_stats
-// unseen, so from then on every call does.
+// reset, since it may be recorded into a caller's graph; once one was, every call does.
 int reset_stats(mdz_rheo_ctx *ctx, bool wait) {
   if (!wait && !ctx->recorded) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(ctx->stream, &cs));
     ctx->recorded = cs != cudaStreamCaptureStatusNone;
   }
-  const bool initial = ctx->stats_initial && !ctx->recorded;
+  const bool initial = ctx->stats_initial;
   ctx->stats_initial = false;
   if (wait && initial) return MDZ_OK;
   DevStats init;
@@ -268,9 +269,12 @@ int reset_stats(mdz_rheo_ctx *ctx, bool wait) {
 }
 
 int finish(mdz_rheo_ctx *ctx, mdz_sweep_stats *st) {
-  CK(launch_stats_out(ctx->d_stats, ctx->h_stats, ctx->stream));
+  if (ctx->recorded)
+    CK(cudaMemcpyAsync(ctx->h_stats, ctx->d_stats, sizeof(DevStats), cudaMemcpyDeviceToHost, ctx->stream));
+  else
+    CK(launch_stats_out(ctx->d_stats, ctx->h_stats, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
-  ctx->stats_initial = true;
+  ctx->stats_initial = !ctx->recorded;
   float ms = 0.f;
   cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
   return stats_from_device(ctx, st, ms);
@@ -1039,7 +1043,8 @@ int mdz_rheo_sync(mdz_rheo_ctx *c, mdz_sweep_stats *st) {
   if (!c) return MDZ_EINVAL;
   CK(cudaSetDevice(c->device));
   c->pending = 0;
-  // the last call's statistics stay readable, however often they are asked for
+  // the last call's statistics stay readable, however often they are asked for; a replay's are
+  // in d_stats only
   if (!c->stats_initial)
     CK(cudaMemcpyAsync(c->h_stats, c->d_stats, sizeof(DevStats), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
