@@ -268,6 +268,15 @@ int reset_stats(mdz_rheo_ctx *ctx, bool wait) {
   return MDZ_OK;
 }
 
+// Device time of the context's last call, 0 where its events were recorded by a capture only
+// (their query fails, and the error must not stay for the next launch's check to find).
+float elapsed(mdz_rheo_ctx *ctx) {
+  float ms = 0.f;
+  if (cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1) == cudaSuccess) return ms;
+  cudaGetLastError();
+  return 0.f;
+}
+
 int finish(mdz_rheo_ctx *ctx, mdz_sweep_stats *st) {
   if (ctx->recorded)
     CK(cudaMemcpyAsync(ctx->h_stats, ctx->d_stats, sizeof(DevStats), cudaMemcpyDeviceToHost, ctx->stream));
@@ -275,9 +284,7 @@ int finish(mdz_rheo_ctx *ctx, mdz_sweep_stats *st) {
     CK(launch_stats_out(ctx->d_stats, ctx->h_stats, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   ctx->stats_initial = !ctx->recorded;
-  float ms = 0.f;
-  cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
-  return stats_from_device(ctx, st, ms);
+  return stats_from_device(ctx, st, elapsed(ctx));
 }
 
 // slot numbering of the host-mode mirrors
@@ -1048,9 +1055,7 @@ int mdz_rheo_sync(mdz_rheo_ctx *c, mdz_sweep_stats *st) {
   if (!c->stats_initial)
     CK(cudaMemcpyAsync(c->h_stats, c->d_stats, sizeof(DevStats), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
-  float ms = 0.f;
-  cudaEventElapsedTime(&ms, c->ev0, c->ev1);
-  return stats_from_device(c, st, ms);
+  return stats_from_device(c, st, elapsed(c));
 }
 
 int mdz_rheo_sweep(mdz_rheo_ctx *c, const mdz_model *md, const mdz_materials *m, const mdz_grid_fields *f,

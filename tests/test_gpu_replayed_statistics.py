@@ -52,3 +52,18 @@ def test_sync_reports_the_failure_of_a_replay(between):
             assert rc == st.status == R.MDZ_EGRAIN_ZERO and st.error_node == 77
     finally:
         ctx.close()
+
+
+def test_sync_of_a_replay_leaves_no_error_behind():
+    """The context's events were recorded by the capture only, so no time can be read from them."""
+    vel = W.velocity_field(seed=9, ncx=40)
+    sr = on_device(vel)
+    ctx = R.Context(0)
+    try:
+        run = lambda flags: ctx.strain_rates(vel.model, vel.info["dx"], vel.info["dz"], sr, mem=R.MEM_DEVICE, flags=flags)
+        replay = captured(ctx, lambda: run(R.SWEEP_ASYNC))
+        replay()
+        assert ctx.sync()[0] == R.MDZ_OK
+        assert run(0)[0] == R.MDZ_OK
+    finally:
+        ctx.close()
