@@ -260,11 +260,7 @@ int reset_stats(mdz_rheo_ctx *ctx, bool wait) {
   const bool initial = ctx->stats_initial;
   ctx->stats_initial = false;
   if (wait && initial) return MDZ_OK;
-  DevStats init;
-  memset(&init, 0, sizeof(init));
-  init.err_key = ~0ull;
-  *ctx->h_stats = init;
-  CK(cudaMemcpyAsync(ctx->d_stats, ctx->h_stats, sizeof(DevStats), cudaMemcpyHostToDevice, ctx->stream));
+  CK(launch_stats_out(ctx->d_stats, nullptr, ctx->stream));
   return MDZ_OK;
 }
 
