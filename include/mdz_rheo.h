@@ -306,7 +306,10 @@ int mdz_rheo_host_access(mdz_rheo_ctx *ctx, int *pageable);
  * double-float Halley step (MDZ_DEFAULT_START); it still iterates to the reference's
  * residual tolerance (|r| < 1e-13 Eii), so results agree with the reference to that
  * tolerance.  MDZ_SWEEP_REF_START starts exactly where the reference does (same
- * iteration counts). */
+ * iteration counts).
+ * Outputs should be arrays of their own: the vertices are updated beside the centroids.
+ * Where an array used in place is passed twice (p_corr = p_in, say), every centroid is
+ * updated before the first vertex, which then reads what the centroids wrote. */
 int mdz_rheo_sweep(mdz_rheo_ctx *ctx, const mdz_model *model, const mdz_materials *mat,
                    const mdz_grid_fields *f, int final_update, int mem, int flags,
                    mdz_sweep_stats *stats);

@@ -121,7 +121,9 @@ __global__ void __launch_bounds__(128) k_points(const __grid_constant__ PointArg
 // A sweep's vertex kernel reads none of the centroid kernel's outputs, so it is launched as a
 // programmatic dependent of it: its CTAs start once every centroid CTA has (pair_begin), in
 // the SMs that the centroid kernel's last wave leaves idle -- all of them where a small grid
-// is one wave -- and end after it (pair_end).
+// is one wave -- and end after it (pair_end).  Where the caller passes one array in two
+// places and the kernels share it after all (kernels_share), the vertex kernel follows the
+// centroid kernel as any launch of a stream does.
 template <class K>
 static cudaError_t launch_after(K fn, unsigned grid, int block, cudaStream_t s, bool after, const SweepArgs &a) {
   cudaLaunchConfig_t cfg = {};
@@ -134,6 +136,44 @@ static cudaError_t launch_after(K fn, unsigned grid, int block, cudaStream_t s, 
   cfg.attrs = at;
   cfg.numAttrs = after ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, fn, a);
+}
+
+// Byte ranges of the arrays that a kernel reads or writes; null arrays are empty ranges.
+struct Ranges {
+  static constexpr int kMax = CI_COUNT + VI_COUNT + CO_COUNT + 2 * MDZ_MAX_PHASES + 8;
+  uintptr_t lo[kMax], hi[kMax];
+  int n = 0;
+  void add(const void *p, long long bytes) {
+    lo[n] = (uintptr_t)p;
+    hi[n++] = p ? (uintptr_t)p + (uintptr_t)bytes : 0;
+  }
+};
+
+static bool overlap(const Ranges &x, const Ranges &y) {
+  unsigned any = 0;
+  for (int i = 0; i < x.n; i++)
+    for (int j = 0; j < y.n; j++) any |= (unsigned)(x.lo[i] < y.hi[j]) & (unsigned)(y.lo[j] < x.hi[i]);
+  return any != 0;
+}
+
+// Whether one of a sweep's two kernels writes memory that the other one reads or writes (an
+// output passed as an input too, or one array for two outputs).  Under 1 us of host time.
+static bool kernels_share(const SweepArgs &a) {
+  const long long cn = a.M.Nc * 8, vn = a.M.Nv * 8;
+  Ranges cr, cw, vr, vw;
+  for (int i = 0; i < CI_COUNT; i++) cr.add(a.ci[i], cn);
+  for (int i = 0; i < CO_COUNT; i++) cw.add(a.co[i], cn);
+  for (int i : {(int)CI_T, (int)CI_p_in, (int)CI_d0, (int)CI_phi0}) vr.add(a.ci[i], cn);  // interpolated
+  for (int i = 0; i < VI_COUNT; i++) vr.add(a.vi[i], vn);
+  for (int i = 0; i < VO_COUNT; i++) vw.add(a.vo[i], vn);
+  for (int p = 0; p < a.M.np; p++) {
+    cr.add(a.perc_n[p], cn); cw.add(a.peta_n[p], cn);
+    vr.add(a.perc_s[p], vn); vw.add(a.peta_s[p], vn);
+  }
+  cr.add(a.bcp, a.M.Nc);
+  vr.add(a.bcp, a.M.Nc);
+  vr.add(a.bcg, a.M.Nv);
+  return overlap(cw, vr) || overlap(cw, vw) || overlap(cr, vw);
 }
 
 // CTAs of 128 per SM for a sweep of so many nodes, centroids and vertices together (their
@@ -170,7 +210,7 @@ cudaError_t launch_sweep(const SweepArgs &a, bool aniso, cudaStream_t s, const L
   for (int kind = 0; kind < 2; kind++) {
     if (counts[kind] <= 0) continue;
     cudaError_t e;
-    const bool after = kind == 1 && counts[0] > 0 && sh.form != SHAPE_QUEUE;
+    const bool after = kind == 1 && counts[0] > 0 && sh.form != SHAPE_QUEUE && !kernels_share(a);
     if (kind == 0 && aniso) e = launch_kind<true, 1>(a, sh, counts[kind], counts[0] + counts[1], s, false);
     else if (kind == 0) e = launch_kind<false, 1>(a, sh, counts[kind], counts[0] + counts[1], s, false);
     else if (aniso) e = launch_kind<true, 2>(a, sh, counts[kind], counts[0] + counts[1], s, after);
