@@ -210,8 +210,8 @@ FX_FN uint64_t fx_exp_core(int64_t X, int &m) {
   // X = (256 m + j) ln2/256 + r with 0 <= r < (1 + 2^-10) ln2/256: the quotient from the
   // high word, biased down by 2^-11 so that r is never negative
   const int k = (fx_mulhi((int32_t)(X >> 32), 774541002) - 1) >> 11;
-  const uint64_t R = ((uint64_t)X << 10) - ((uint64_t)((int64_t)k * (int64_t)0xb17217f7d1cf7a) +
-                                            (uint64_t)(int64_t)fx_mulhi(k, -1412832332));  // Q0.64
+  const uint64_t R = ((uint64_t)X << 10) - ((uint64_t)(int64_t)k * 0xb17217f7d1cf7aull +
+                                            (uint64_t)(int64_t)fx_mulhi(k, -1412832332));  // Q0.64, modulo 1
   const uint64_t T = FX_TAB(exp2, k & 255);
   m = k >> 8;
   // exp(r) - 1 = r + r^2/2 + r^3 (1/6 + r/24 + r^2/120) + O(r^6/720), r < 2^-8.5
@@ -353,7 +353,7 @@ FX_FN uint64_t fx_recip_core(uint64_t D) {
   const int32_t e32 = (int32_t)(e >> 16);               // Q.47, |.| < 2^26
   const int64_t t = e + (((int64_t)e32 * e32) >> 31);    // e + e^2, Q.63
   // y t in Q.64: y (Q.32) times the two words of t (Q.63)
-  const int64_t corr = (((int64_t)(int32_t)(t >> 32) * (int64_t)y) << 1) + (int64_t)(((uint64_t)fx_lo((uint64_t)t) * y) >> 31);
+  const int64_t corr = 2 * ((int64_t)(int32_t)(t >> 32) * (int64_t)y) + (int64_t)(((uint64_t)fx_lo((uint64_t)t) * y) >> 31);
   return ((uint64_t)y << 32) + (uint64_t)corr;
 }
 
@@ -400,7 +400,7 @@ FX_FN double fx_sqrt(double x) {
   const int64_t t = (e >> 1) + ((3 * e2) >> 3);              // Q.61
   // s t in Q.61: s in [2^61, 2^62) (31 bits of it are enough), |t| < 2^41 in Q.61
   const int32_t sh = (int32_t)(s >> 32);                     // Q.29, < 2^30
-  const int64_t corr = ((int64_t)(int32_t)(t >> 32) * sh << 3) + (int64_t)(((uint64_t)fx_lo((uint64_t)t) * (uint32_t)sh) >> 29) +
+  const int64_t corr = 8 * ((int64_t)(int32_t)(t >> 32) * sh) + (int64_t)(((uint64_t)fx_lo((uint64_t)t) * (uint32_t)sh) >> 29) +
                        (((int64_t)(int32_t)(t >> 11) * (int32_t)(fx_lo(s) >> 1)) >> 49);
   const uint64_t S = s + (uint64_t)corr;
   return fx_normalise(S, -61 + (((int)E - 1023 - odd) >> 1));

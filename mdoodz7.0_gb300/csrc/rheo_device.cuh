@@ -702,10 +702,10 @@ __device__ __forceinline__ bool ve_solve_fx(const PhaseConst &ph, const Laws &L,
   if (L.mech & F_CST) { inv_cst = FP::recip(eta_cst); A += inv_cst; }
   int nl = 0, tiny = 0;  // tiny: laws below e^-150, left out of the residual
   float nmax = 0.0f;
-  // k2 ln 2 = k2 - k2 (1 - ln 2) in Q.54; 1 - ln2 = 0x4e8de808 2e308654 2^-64
+  // k2 ln 2 = k2 - k2 (1 - ln 2) in Q.54, modulo 2^10 (|k2 ln 2| may pass 512, its sum with a
+  // law's logarithm below does not); 1 - ln2 = 0x4e8de808 2e308654 2^-64
   const int64_t p0 = (int64_t)k2 * 0x2e308654, p1 = (int64_t)k2 * 0x4e8de808 + (p0 >> 32);
-  const int64_t kln2 = (int64_t)((uint64_t)(int64_t)k2 << 54) - (int64_t)((uint64_t)p1 << 22) -
-                       (int64_t)(fx_lo((uint64_t)p0) >> 10);
+  const uint64_t kln2 = ((uint64_t)(int64_t)k2 << 54) - ((uint64_t)p1 << 22) - (uint64_t)(fx_lo((uint64_t)p0) >> 10);
 #pragma unroll
   for (int k = 0; k < K_COUNT; k++) {
     const int bit = (k == K_PWL) ? F_PWL : ((k == K_EXP) ? F_EXPV : F_LIN);
@@ -726,7 +726,7 @@ __device__ __forceinline__ bool ve_solve_fx(const PhaseConst &ph, const Laws &L,
         if (!(cf[k] < 149.0f && fabsf(df) < 500.0f)) return false;
         nl |= 1 << k;
         N[k] = fx_fixed<56>(nb);
-        X[k] = fx_mul_nd(N[k], fx_fixed<54>(lb) + kln2);
+        X[k] = fx_mul_nd(N[k], (int64_t)((uint64_t)fx_fixed<54>(lb) + kln2));
         cf[k] = (float)(int32_t)(X[k] >> 31) * 1.1920929e-7f;  // 2^-23
         nmax = fmaxf(nmax, nf[k]);
       }

@@ -27,7 +27,7 @@ namespace mdz {
 FX_FN int64_t fx_mulq62(uint64_t E, int64_t F) {
   const int32_t eh = (int32_t)fx_hi(E), fh = (int32_t)(F >> 32);
   const uint32_t fl = fx_lo((uint64_t)F);
-  return ((int64_t)eh * fh << 2) + (int64_t)(((uint64_t)(uint32_t)eh * fl) >> 30) +
+  return 4 * ((int64_t)eh * fh) + (int64_t)(((uint64_t)(uint32_t)eh * fl) >> 30) +
          (((int64_t)(int32_t)(fx_lo(E) >> 1) * fh) >> 29);
 }
 
@@ -42,7 +42,7 @@ FX_FN int64_t fx_mul_nl(int64_t N, int64_t L) {
   // the middle products with 4 more bits, so that their sum is rounded once
   const int64_t mid = (int64_t)((uint64_t)(uint32_t)nh * ll >> 26) + (((int64_t)lh * (int32_t)(nl >> 1)) >> 25) +
                       (int64_t)(fx_umulhi(nl, ll) >> 26);
-  return ((int64_t)nh * lh << 2) + ((mid + 8) >> 4);
+  return 4 * ((int64_t)nh * lh) + ((mid + 8) >> 4);
 }
 
 // n d in Q9.54 for n = N in Q7.56 and d = L in Q9.54 (signed), |n d| < 512
@@ -58,7 +58,7 @@ FX_FN int64_t fx_mul_nd(int64_t N, int64_t L) {
 FX_FN int64_t fx_mul_ntiny(int64_t N, int64_t L) {
   const int32_t nh = (int32_t)(N >> 32), lh = (int32_t)(L >> 32);
   const uint32_t nl = fx_lo((uint64_t)N), ll = fx_lo((uint64_t)L);
-  return ((int64_t)nh * lh << 8) + (int64_t)(((uint64_t)(uint32_t)nh * ll) >> 24) +
+  return 256 * ((int64_t)nh * lh) + (int64_t)(((uint64_t)(uint32_t)nh * ll) >> 24) +
          (((int64_t)lh * (int32_t)(nl >> 1)) >> 23) + (int64_t)(fx_umulhi(nl, ll) >> 24);
 }
 
@@ -69,6 +69,12 @@ FX_FN int32_t fx_rint(float x) {
   return !(x > -2147483648.0f) ? INT32_MIN : (x < 2147483648.0f ? (int32_t)lrintf(x) : INT32_MAX);
 #endif
 }
+
+// a shift count held to [0, 63]; one below 0 is of a number that has left its format, which
+// the caller's checks see
+FX_FN int fx_shift(int sh) { return (unsigned)sh > 63u ? 63 : sh; }
+// R - E modulo 2^64: sums of Q2.62 numbers that have left their format wrap
+FX_FN int64_t fx_sub(int64_t R, uint64_t E) { return (int64_t)((uint64_t)R - E); }
 
 struct VeFxRoot {
   uint64_t S;          // s, Q2.62
@@ -93,7 +99,7 @@ FX_FN bool ve_root_fx(int nl, double a, const int64_t *N, const int64_t *C, cons
   const uint64_t am = fx_significand(ab) << 11;
   const uint64_t A0 = ((uint64_t)fx_hi(am) * (m24 << 8) + fx_umulhi(fx_lo(am), m24 << 8)) >> (shift > 63 ? 63 : shift);
   ok = ok && (int64_t)A0 >= 0;
-  int64_t R = (int64_t)0x4000000000000000ll - (int64_t)A0;
+  int64_t R = fx_sub(0x4000000000000000ll, A0);
   float D = (float)fx_hi(A0) * 9.31322575e-10f, Q = 0.0f;  // 2^-30
   if (nl) {
     // ln s0 in Q4.60
@@ -105,8 +111,8 @@ FX_FN bool ve_root_fx(int nl, double a, const int64_t *N, const int64_t *C, cons
         ok = ok && (int32_t)(X >> 32) < 2516582;  // X < 0.6 (and above -505)
         o.M[k] = fx_exp_core(X, o.m[k]);
         const int sh = -o.m[k];
-        const uint64_t E = o.M[k] >> (sh > 63 ? 63 : sh);
-        R -= (int64_t)E;
+        const uint64_t E = o.M[k] >> fx_shift(sh);
+        R = fx_sub(R, E);
         const float ne = nf[k] * ((float)fx_hi(E) * 9.31322575e-10f);
         D += ne;
         Q = fmaf(ne, nf[k] - 1.0f, Q);
@@ -119,12 +125,12 @@ FX_FN bool ve_root_fx(int nl, double a, const int64_t *N, const int64_t *C, cons
   ok = ok && fabsf(q) < 6.0e-5f;
   const int32_t qi = fx_rint(q * 17592186044416.0f);  // Q.44, below 2^30; exact from here on
   const int64_t sq = (int64_t)qi * qi;                        // Q.88
-  const int64_t q62 = (int64_t)qi << 18;
+  const int64_t q62 = (int64_t)qi * 262144;
   // log1p(q) = q - q^2/2 + q^3/3
   const int64_t lam = q62 - (sq >> 27) + ((((sq >> 44) * (int64_t)qi) >> 26) * 21845 >> 16);
   const uint64_t S0 = (uint64_t)m24 << (39 + e0);
   const uint64_t S1 = S0 + (uint64_t)fx_mulq62(S0, q62);
-  R = (int64_t)0x4000000000000000ll - (int64_t)A0 - fx_mulq62(A0, q62);
+  R = fx_sub(fx_sub(0x4000000000000000ll, A0), (uint64_t)fx_mulq62(A0, q62));
   if (nl) {
 #pragma unroll
     for (int k = 0; k < 3; k++)
@@ -135,9 +141,9 @@ FX_FN bool ve_root_fx(int nl, double a, const int64_t *N, const int64_t *C, cons
         ok = ok && (int32_t)(t >> 48) >= -1 && (int32_t)(t >> 48) < 1;
         const int64_t t2 = (int64_t)ts * ts;    // Q.90
         const int64_t f = t + (t2 >> 29) + ((((t2 >> 45) * (int64_t)ts) >> 28) * 10923 >> 16);
-        o.M[k] += (uint64_t)fx_mulq62(o.M[k] >> 1, f << 1);
+        o.M[k] += (uint64_t)fx_mulq62(o.M[k] >> 1, 2 * f);
         const int sh = -o.m[k];
-        R -= (int64_t)(o.M[k] >> (sh > 63 ? 63 : sh));
+        R = fx_sub(R, o.M[k] >> fx_shift(sh));
       }
   }
   ok = ok && R < (1ll << 27) && R > -(1ll << 27);
@@ -160,7 +166,7 @@ FX_FN bool ve_residual_fx(int nl, double a, const int64_t *N, const int64_t *C, 
   const uint64_t m53 = fx_significand(sb);
   const uint64_t A0 = fx_mul64hi(fx_significand(ab) << 11, m53 << 11) >> (shift > 63 ? 63 : shift);
   bool ok = (int64_t)A0 >= 0;
-  R = (int64_t)0x4000000000000000ll - (int64_t)A0;
+  R = fx_sub(0x4000000000000000ll, A0);
   if (nl) {
     const int64_t L = (int64_t)(fx_log_significand(m53) >> 4) + (int64_t)e0 * 0xb17217f7d1cf79all;
 #pragma unroll
@@ -170,7 +176,7 @@ FX_FN bool ve_residual_fx(int nl, double a, const int64_t *N, const int64_t *C, 
         ok = ok && (int32_t)(X >> 32) < 2516582;  // X < 0.6
         int m;
         const uint64_t M = fx_exp_core(X, m);
-        R -= (int64_t)(M >> (-m > 63 ? 63 : -m));
+        R = fx_sub(R, M >> fx_shift(-m));
       }
   }
   return ok;
