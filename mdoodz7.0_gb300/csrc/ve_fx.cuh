@@ -16,8 +16,8 @@
 // 1025 x 1025 one from 2.58 to 1.63 ms; no local solve of either declines.
 //
 // The fast form declines (returns false, nothing written) where a number would leave its
-// format: a point that the FP32 steps did not settle, s0 outside [2^-4, 2), exponents n_k of
-// 128 and more, |c_k| of 150 and more.  The caller then takes the FP64 iteration.
+// format: a point that the FP32 steps did not settle, terms well above 1, s0 outside [2^-4, 2),
+// exponents n_k of 128 and more, |c_k| of 150 and more.  The caller then takes the FP64 iteration.
 #pragma once
 #include "fx64.cuh"
 
@@ -76,6 +76,12 @@ FX_FN int fx_shift(int sh) { return (unsigned)sh > 63u ? 63 : sh; }
 // R - E modulo 2^64: sums of Q2.62 numbers that have left their format wrap
 FX_FN int64_t fx_sub(int64_t R, uint64_t E) { return (int64_t)((uint64_t)R - E); }
 
+// Bounds on the residual's terms: a s below 1.05 (in Q2.30), each law's argument below 0.05
+// (in Q9.22), so each law's term below 1.052.  At the root every term is at most 1.  Within the
+// bounds r is above -3.21, so where the sum wraps, modulo 4, it lands above 0.79: never near 0.
+constexpr uint32_t kVeMaxLinear = 1127428915u;
+constexpr int32_t kVeMaxArgument = 209715;
+
 struct VeFxRoot {
   uint64_t S;          // s, Q2.62
   uint64_t M[3];       // law terms exp(n_k ln s + c_k) = M 2^(m - 62)
@@ -98,7 +104,7 @@ FX_FN bool ve_root_fx(int nl, double a, const int64_t *N, const int64_t *C, cons
   if (shift < 0) return false;  // a s0 >= 2, Inf or NaN
   const uint64_t am = fx_significand(ab) << 11;
   const uint64_t A0 = ((uint64_t)fx_hi(am) * (m24 << 8) + fx_umulhi(fx_lo(am), m24 << 8)) >> (shift > 63 ? 63 : shift);
-  ok = ok && (int64_t)A0 >= 0;
+  ok = ok && fx_hi(A0) < kVeMaxLinear;
   int64_t R = fx_sub(0x4000000000000000ll, A0);
   float D = (float)fx_hi(A0) * 9.31322575e-10f, Q = 0.0f;  // 2^-30
   if (nl) {
@@ -108,7 +114,7 @@ FX_FN bool ve_root_fx(int nl, double a, const int64_t *N, const int64_t *C, cons
     for (int k = 0; k < 3; k++)
       if (nl >> k & 1) {
         const int64_t X = fx_mul_nl(N[k], L) + C[k];
-        ok = ok && (int32_t)(X >> 32) < 2516582;  // X < 0.6 (and above -505)
+        ok = ok && (int32_t)(X >> 32) < kVeMaxArgument;  // (and above -505)
         o.M[k] = fx_exp_core(X, o.m[k]);
         const int sh = -o.m[k];
         const uint64_t E = o.M[k] >> fx_shift(sh);
@@ -165,7 +171,7 @@ FX_FN bool ve_residual_fx(int nl, double a, const int64_t *N, const int64_t *C, 
   if (e0 > 0 || e0 < -4 || shift < 0) return false;
   const uint64_t m53 = fx_significand(sb);
   const uint64_t A0 = fx_mul64hi(fx_significand(ab) << 11, m53 << 11) >> (shift > 63 ? 63 : shift);
-  bool ok = (int64_t)A0 >= 0;
+  bool ok = fx_hi(A0) < kVeMaxLinear;
   R = fx_sub(0x4000000000000000ll, A0);
   if (nl) {
     const int64_t L = (int64_t)(fx_log_significand(m53) >> 4) + (int64_t)e0 * 0xb17217f7d1cf79all;
@@ -173,7 +179,7 @@ FX_FN bool ve_residual_fx(int nl, double a, const int64_t *N, const int64_t *C, 
     for (int k = 0; k < 3; k++)
       if (nl >> k & 1) {
         const int64_t X = fx_mul_nl(N[k], L) + C[k];
-        ok = ok && (int32_t)(X >> 32) < 2516582;  // X < 0.6
+        ok = ok && (int32_t)(X >> 32) < kVeMaxArgument;
         int m;
         const uint64_t M = fx_exp_core(X, m);
         R = fx_sub(R, M >> fx_shift(-m));
