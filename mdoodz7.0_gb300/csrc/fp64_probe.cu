@@ -13,6 +13,7 @@
 // mdz_rheo_ceil_selftest: the integer-pipe ceil of fp64_bits.cuh next to CUDA's ceil.
 // mdz_rheo_fx_selftest: the fixed-point exp, log, reciprocal, square root, sine and cosine
 // of fx64.cuh, for the accuracy tests.
+// mdz_rheo_fx_pair_selftest: those of two arguments.
 // mdz_rheo_dd_selftest: the double-float conversion, exp and log of dd_math.cuh, for the
 // accuracy tests.
 #include <cuda_runtime.h>
@@ -59,6 +60,13 @@ __global__ void k_div(const double *a, long long n, mdz::Divisor d, double *fast
 }
 
 // out[6][n]: exp, log, 1/x, sqrt, sin, cos of x
+__global__ void k_fx_pair(const double *a, const double *b, long long n, double *out) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  out[i] = mdz::fx_pow(a[i], b[i]);
+  out[n + i] = pow(a[i], b[i]);
+}
+
 __global__ void k_fx(const double *x, long long n, double *out) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -114,6 +122,26 @@ extern "C" int mdz_rheo_dd_selftest(int device, const double *x, int64_t n, floa
     if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) rc = MDZ_ECUDA;
   }
   if (rc == MDZ_OK && cudaMemcpy(out, dout, bo, cudaMemcpyDeviceToHost) != cudaSuccess) rc = MDZ_ECUDA;
+  cudaFree(d);
+  return rc;
+}
+
+extern "C" int mdz_rheo_fx_pair_selftest(int device, const double *a, const double *b, int64_t n, double *out) {
+  if (!a || !b || n < 0 || !out) return MDZ_EINVAL;
+  if (n == 0) return MDZ_OK;
+  if (cudaSetDevice(device) != cudaSuccess) return MDZ_ECUDA;
+  const size_t bytes = (size_t)n * sizeof(double);
+  double *d = nullptr;
+  if (cudaMalloc(&d, 4 * bytes) != cudaSuccess) return MDZ_ENOMEM;
+  int rc = MDZ_OK;
+  if (cudaMemcpy(d, a, bytes, cudaMemcpyHostToDevice) != cudaSuccess ||
+      cudaMemcpy(d + n, b, bytes, cudaMemcpyHostToDevice) != cudaSuccess)
+    rc = MDZ_ECUDA;
+  if (rc == MDZ_OK) {
+    k_fx_pair<<<(unsigned)((n + 255) / 256), 256>>>(d, d + n, n, d + 2 * n);
+    if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) rc = MDZ_ECUDA;
+  }
+  if (rc == MDZ_OK && cudaMemcpy(out, d + 2 * n, 2 * bytes, cudaMemcpyDeviceToHost) != cudaSuccess) rc = MDZ_ECUDA;
   cudaFree(d);
   return rc;
 }

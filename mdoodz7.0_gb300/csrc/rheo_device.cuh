@@ -57,6 +57,7 @@ static __device__ __noinline__ double fx_exp_call(double x) { return fx_exp(x); 
 static __device__ __noinline__ double fx_log_call(double x) { return fx_log(x); }
 static __device__ __noinline__ double fx_recip_call(double x) { return fx_recip(x); }
 static __device__ __noinline__ double fx_sqrt_call(double x) { return fx_sqrt(x); }
+static __device__ __noinline__ double fx_pow_call(double x, double y) { return fx_pow(x, y); }
 struct FxMath {
   static constexpr bool kFixed = true;  // local solves in fixed point where the start asks for it (ve_solve_fx)
   static __device__ __forceinline__ double exp(double x) { return fx_exp_call(x); }
@@ -68,6 +69,7 @@ struct FxMath {
   static __device__ __forceinline__ double sqrt(double x) { return fx_sqrt_call(x); }
   static __device__ __forceinline__ void sincos(double x, double *s, double *c) { fx_sincos(x, s, c); }
   static __device__ __forceinline__ double sin(double x) { return fx_sincos_rare(x).x; }
+  static __device__ __forceinline__ double pow(double x, double y) { return fx_pow_call(x, y); }
 };
 struct FdMath {
   static constexpr bool kFixed = false;
@@ -80,6 +82,7 @@ struct FdMath {
   static __device__ __forceinline__ double sqrt(double x) { return ::sqrt(x); }
   static __device__ __forceinline__ void sincos(double x, double *s, double *c) { ::sincos(x, s, c); }
   static __device__ __forceinline__ double sin(double x) { return ::sin(x); }
+  static __device__ __forceinline__ double pow(double x, double y) { return ::pow(x, y); }
 };
 
 constexpr double kZeroC = 273.15;                 // MDLIB/include/mdoodz.h:4
@@ -1256,6 +1259,7 @@ __device__ __forceinline__ void dp_store(IsoMid &m, const DpItem &d) {
 }
 
 // The Drucker-Prager return (:655-707) of an item that yields (Tii - Tyield > 1e-17).
+template <class FP>
 __device__ inline void dp_return(const ModelConst &M, const PhaseConst &ph, DpItem &d) {
   const int fl = ph.flags;
   const double Tii = d.Tii, eta_ve = d.eta_ve, P = d.P, dt = M.dt;
@@ -1270,8 +1274,8 @@ __device__ inline void dp_return(const ModelConst &M, const PhaseConst &ph, DpIt
   const double Kdt = __dmul_rn(d.K, dt);
   const double ksd = __dmul_rn(__dmul_rn(Kdt, d.sin_fric), d.sin_dil);
   double Tiic = 0.0, divp = 0.0, Pc = P;
-  double eta_vp = vp1 ? eta_vp0 : eta_vp0 * pow(d.Eii, 1.0 / n_vp - 1);
-  double gdot = quotient(F, eta_ve + eta_vp + ksd);
+  double eta_vp = vp1 ? eta_vp0 : eta_vp0 * FP::pow(d.Eii, 1.0 / n_vp - 1);
+  double gdot = FP::quotient(F, eta_ve + eta_vp + ksd);
   const double F0 = F, tolF0 = tol * F0;
   // with n_vp == 1, eta_vp / n_vp is eta_vp exactly and the derivative is a constant
   const double dF1 = __dsub_rn(__dsub_rn(-eta_ve, eta_vp0), ksd);
@@ -1287,12 +1291,12 @@ __device__ inline void dp_return(const ModelConst &M, const PhaseConst &ph, DpIt
     const unsigned long long g0 = fp64_bits(gdot), y0 = fp64_bits(Tyield);
     divp = __dmul_rn(gdot, d.sin_dil);
     Pc = __dadd_rn(P, __dmul_rn(Kdt, divp));
-    eta_vp = vp1 ? eta_vp0 : eta_vp0 * pow(fabs(gdot), 1.0 / n_vp - 1.0);
+    eta_vp = vp1 ? eta_vp0 : eta_vp0 * FP::pow(fabs(gdot), 1.0 / n_vp - 1.0);
     Tyield = __dadd_rn(Tyield, __dmul_rn(gdot, eta_vp));
     Tiic = __dsub_rn(Tii, __dmul_rn(eta_ve, gdot));
     F = Tiic - Tyield;
     if (fp64_abs_lt(F, tol) || fp64_abs_lt(F, tolF0)) break;
-    gdot -= F / (vp1 ? dF1 : (-eta_ve - eta_vp / n_vp - ksd));
+    gdot -= FP::divide(F, vp1 ? dF1 : (-eta_ve - FP::divide(eta_vp, n_vp) - ksd));
     if (it == last) break;
     const unsigned long long gn = fp64_bits(gdot), yn = fp64_bits(Tyield);
     if (gn == g0 && yn == y0) break;  // period 1: iteration 19 would be this one
@@ -1314,12 +1318,14 @@ __device__ inline void dp_return(const ModelConst &M, const PhaseConst &ph, DpIt
 // iteration itself (dp_return) runs out of line where it does not.  While the return took
 // some 40 FP64 instructions it was worth gathering the yielding items of a CTA into its first
 // warps; at 9 the barriers cost more than the idle lanes: 2049 x 2049 sweep 7.70 -> 7.52 ms,
-// 201 x 201 80 -> 71 us, 16-grid batch 6.60 -> 5.74 ms.
-static __device__ __noinline__ DpItem dp_return_call(const ModelConst &M, const PhaseConst &ph, DpItem d) {
-  dp_return(M, ph, d);
+// 201 x 201 80 -> 71 us, 16-grid batch 6.60 -> 5.74 ms.  That holds for the iteration with its
+// power and quotients on the integer pipe; with CUDA's pow and divisions, up to 20 times for
+// the few yielding lanes of nearly every warp, a 1025 x 1025 sweep with n_vp = 2 took 24.9 ms
+// (15.3 gathered per CTA), and takes 5.4; with dilation and n_vp = 1 3.9 -> 3.3.
+static __device__ __noinline__ void dp_return_call(const ModelConst &M, const PhaseConst &ph, DpItem &d) {
+  dp_return<FxMath>(M, ph, d);
   d.pl_share = d.eta_ve * d.gdot * fx_recip_call(d.Tii);
   d.T_over_eta = d.Tii * fx_recip_call(d.eta_ve);
-  return d;
 }
 
 __device__ __forceinline__ void dp_return_inline(const ModelConst &M, const PhaseConst &ph, const NodeIn &in,
@@ -1343,7 +1349,7 @@ __device__ __forceinline__ void dp_return_inline(const ModelConst &M, const Phas
   }
   DpItem d;
   dp_load(d, m, in, c);
-  d = dp_return_call(M, ph, d);
+  dp_return_call(M, ph, d);
   dp_store(m, d);
   m.pl_share = d.pl_share; m.T_over_eta = d.T_over_eta;
 }
@@ -1550,7 +1556,7 @@ __device__ inline void iso_finish(const ModelConst &M, const PhaseConst &ph, con
     } else {
       DpItem d;
       dp_load(d, m, in, c);
-      dp_return(M, ph, d);
+      dp_return<FdMath>(M, ph, d);
       dp_store(m, d);
     }
   }
@@ -1601,7 +1607,7 @@ __device__ __forceinline__ void dp_compact(const ModelConst &M, const PhaseConst
   if (t == 0) Q.count[par ^ 1] = 0;
   if (t < q) {
     DpItem d = Q.item[t];
-    dp_return(M, ph, d);
+    dp_return<FdMath>(M, ph, d);
     Q.item[t] = d;
   }
   __syncthreads();

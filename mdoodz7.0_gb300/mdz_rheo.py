@@ -408,6 +408,7 @@ def load_library(path: str = LIB_PATH):
     lib.mdz_rheo_dd_selftest.argtypes = [C.c_int, C.c_void_p, C.c_int64, C.c_void_p]
     lib.mdz_rheo_quotient_selftest.argtypes = [C.c_int, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p]
     lib.mdz_rheo_fx_selftest.argtypes = [C.c_int, C.c_void_p, C.c_int64, C.c_void_p]
+    lib.mdz_rheo_fx_pair_selftest.argtypes = [C.c_int, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p]
     lib.mdz_rheo_points_static.argtypes = [C.POINTER(Model), C.POINTER(Materials), C.POINTER(PointInputs),
                                            C.POINTER(PointOutputs), C.c_int64, C.c_int, C.c_int, C.c_void_p,
                                            C.POINTER(SweepStats)]
@@ -527,6 +528,16 @@ def fx_selftest(x: np.ndarray, device: int = 0):
     rc = load_library().mdz_rheo_fx_selftest(device, x.ctypes.data, x.size, out.ctypes.data)
     if rc != MDZ_OK:
         raise RheoError(rc, "mdz_rheo_fx_selftest")
+    return tuple(out)
+
+
+def fx_pair_selftest(a: np.ndarray, b: np.ndarray, device: int = 0):
+    """(a^b by the fixed-point power, by CUDA's pow) of the float64 arrays a, b on the GPU."""
+    a, b = np.ascontiguousarray(a, np.float64), np.ascontiguousarray(b, np.float64)
+    out = np.empty((2, a.size), np.float64)
+    rc = load_library().mdz_rheo_fx_pair_selftest(device, a.ctypes.data, b.ctypes.data, a.size, out.ctypes.data)
+    if rc != MDZ_OK:
+        raise RheoError(rc, "mdz_rheo_fx_pair_selftest")
     return tuple(out)
 
 

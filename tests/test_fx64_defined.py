@@ -16,7 +16,7 @@ static void functions(double x) {
   keep(fx_exp(x)); keep(fx_log(x)); keep(fx_recip(x)); keep(fx_sqrt(x));
   double s, c;
   fx_sincos(x, &s, &c);
-  keep(s); keep(c); keep(fx_mul_rn(x, s)); keep(fx_mul_rn(x, x));
+  keep(s); keep(c); keep(fx_mul_rn(x, s)); keep(fx_mul_rn(x, x)); keep(fx_pow(fabs(x), 0.9 * s));
 }
 static void solves(std::mt19937_64 &g, bool far) {
   std::uniform_real_distribution<double> u(0.0, 1.0);

@@ -1,0 +1,44 @@
+"""Times of calls with rarely used options, as multiples of the same call's ordinary time on the same GPU: a guard against an
+option becoming several times slower than it has to be.  Each limit lies well above the multiple that the option takes
+and well below one that it once took, both stated."""
+import statistics
+
+import pytest
+
+import mdz_rheo as R
+import mdz_workloads as W
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def on_device(a):
+    d = {k: ([torch.from_numpy(x).cuda() for x in v] if isinstance(v, list) else torch.from_numpy(v).cuda())
+         for k, v in a.items()}
+    torch.cuda.synchronize()
+    return d
+
+
+def kernel_ms(call, reps=9):
+    for _ in range(3):
+        call()
+    return statistics.median(call()[1].elapsed_ms for _ in range(reps))
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = R.Context(0)
+    yield c
+    c.close()
+
+
+def test_power_law_viscoplasticity(ctx):
+    """n_vp = 2 against n_vp = 1 at 1025 x 1025 cells: 3.1 times (14 with CUDA's pow in every pass)."""
+    w = W.plain_large(seed=3, ncx=1025)
+    F = R.FieldSet(on_device(w.arrays))
+    plain = kernel_ms(lambda: ctx.sweep(w.model, w.mat, F, mem=R.MEM_DEVICE))
+    for p in range(5):
+        w.mat.eta_vp[p], w.mat.n_vp[p] = 1e12, 2.0
+    power = kernel_ms(lambda: ctx.sweep(w.model, w.mat, F, mem=R.MEM_DEVICE, check=False))
+    print("n_vp", power / plain)
+    assert power < 6.0 * plain
