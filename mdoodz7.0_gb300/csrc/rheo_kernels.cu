@@ -71,7 +71,13 @@ __global__ void __launch_bounds__(128, 6) k_sweep_queue(const __grid_constant__ 
 // ---------------------------------------------------------------------------------
 // independent points: ViscosityConcise / ViscosityConciseAniso
 // ---------------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) k_points(const __grid_constant__ PointArgs A) {
+// 3 CTAs per SM (168 registers); left alone the compiler takes 196, which makes it 2, and a
+// launch of more than two CTAs per SM then waits for another round of them.  2 against 3: 45,000
+// points of mixed creep laws 69 -> 50 us, 1,000,000 608 -> 520, 2,000 46 -> 45; 48,000 points of
+// the grain-size solve 1.76 -> 1.33 ms, 80,000 of the Popov return 391 -> 328 us.  4 (128
+// registers): 2,000 points 47 us, 1,000,000 512, 114,000 of the grain-size solve 3.06 ms for
+// 2.63.
+__global__ void __launch_bounds__(128, 3) k_points(const __grid_constant__ PointArgs A) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   Acc acc = {0, 0, 0, 0, 0};
   const bool bad_phase = (i < A.n) && (A.in.phase[i] < 0 || A.in.phase[i] >= A.M.np);

@@ -2,11 +2,14 @@
 option becoming several times slower than it has to be.  Each limit lies well above the multiple that the option takes
 and well below one that it once took, both stated."""
 import statistics
+import time
 
+import numpy as np
 import pytest
 
 import mdz_rheo as R
 import mdz_workloads as W
+from golden.cases import alloc_point_outputs, point_case
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
@@ -33,7 +36,7 @@ def ctx():
 
 
 def test_power_law_viscoplasticity(ctx):
-    """n_vp = 2 against n_vp = 1 at 1025 x 1025 cells: 3.1 times (14 with CUDA's pow in every pass)."""
+    """n_vp = 2 against n_vp = 1 at 1025 x 1025 cells: 3.5 times (14 with CUDA's pow in every pass)."""
     w = W.plain_large(seed=3, ncx=1025)
     F = R.FieldSet(on_device(w.arrays))
     plain = kernel_ms(lambda: ctx.sweep(w.model, w.mat, F, mem=R.MEM_DEVICE))
@@ -42,3 +45,23 @@ def test_power_law_viscoplasticity(ctx):
     power = kernel_ms(lambda: ctx.sweep(w.model, w.mat, F, mem=R.MEM_DEVICE, check=False))
     print("n_vp", power / plain)
     assert power < 6.0 * plain
+
+
+def test_points_with_the_grain_size_solve(ctx):
+    """48,000 points against 12,000 (less than one CTA of 128 per SM): 2.7 times with three CTAs on an SM (3.6 with two)."""
+    md, m, pin, aniso, centroid, fu = point_case("gse")
+
+    def seconds(rep):
+        n = pin["T"].size * rep
+        p, o = on_device({k: np.tile(v, rep) for k, v in pin.items()}), on_device(alloc_point_outputs(n))
+        args = R.make_points(p, o, centroid=centroid, final_update=fu)
+        t = []
+        for _ in range(12):
+            t0 = time.perf_counter()
+            assert ctx.points(md, m, *args, n, mem=R.MEM_DEVICE) == R.MDZ_OK
+            t.append(time.perf_counter() - t0)
+        return statistics.median(t[3:])
+
+    few, many = seconds(100), seconds(400)
+    print("points", many / few)
+    assert many < 3.15 * few
