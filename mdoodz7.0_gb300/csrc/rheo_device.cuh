@@ -295,9 +295,12 @@ __device__ __forceinline__ double law_inv(const Laws &L, int k) { return FP::exp
 //
 // What of a phase's laws does not depend on the strain rate: the operators' strain-rate
 // perturbations form it once per node and phase (the same operations, so the same bits), for
-// the first kFdPhases phases without a grain-size solve (which needs more): 200 bytes of the
-// thread's stack, which keep it at the sweep kernels' size.
-constexpr int kFdPhases = 5;
+// the first kFdPhases phases without a grain-size solve (which needs more).  They are on the
+// thread's stack, 40 bytes each.  A kernel whose stack exceeds the 1,024 bytes per thread that
+// CUDA reserves by default makes its first launch take device memory (10 MiB with 7 phases
+// kept, 1,056 bytes); 6 are the most that stay within it (1,008).  More would gain little:
+// 257 x 257 cells with 7 phases take 2.32, 2.34 and 2.29 ms with 5, 6 and 7 of them kept.
+constexpr int kFdPhases = 6;
 struct FdLaw {
   double lnB_pwl, lnBd, nE, lnA, Tyield;
 };
