@@ -670,8 +670,10 @@ int mdz_rheo_quotient_selftest(int device, const double *r, const double *den, i
  * k = 0..5 is exp, log, 1/x, sqrt, sin and cos of x[i], for n host arguments.  No reference
  * counterpart. */
 int mdz_rheo_fx_selftest(int device, const double *x, int64_t n, double *out);
-/* The same for functions of two arguments: out[k n + i] for k = 0, 1 is a[i] to the power
- * b[i] by fx64.cuh and by CUDA. */
+/* The same for functions of two arguments: out[k n + i] for k = 0..5 is a[i] to the power
+ * b[i] by fx64.cuh and by CUDA, then the correctly rounded forms of fx64.cuh and
+ * fp64_div.cuh: a b, 1 / a, a / b for b near 1 and a / b with a divisor formed on the
+ * device. */
 int mdz_rheo_fx_pair_selftest(int device, const double *a, const double *b, int64_t n, double *out);
 /* Self-check of the cell-index ceil used by mdz_rheo_marker_stress: ceil(q[i]) from the
  * bits of q (saturated to +-2^30 beyond that range and for NaN) and CUDA's ceil, for n

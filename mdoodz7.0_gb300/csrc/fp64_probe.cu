@@ -63,8 +63,14 @@ __global__ void k_div(const double *a, long long n, mdz::Divisor d, double *fast
 __global__ void k_fx_pair(const double *a, const double *b, long long n, double *out) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  out[i] = mdz::fx_pow(a[i], b[i]);
-  out[n + i] = pow(a[i], b[i]);
+  const double x = a[i], y = b[i];
+  out[i] = mdz::fx_pow(x, y);
+  out[n + i] = pow(x, y);
+  out[2 * n + i] = mdz::fx_mul_rn(x, y);
+  out[3 * n + i] = mdz::recip_rn(x);
+  double q;
+  out[4 * n + i] = mdz::div_near_one(x, y, q) ? q : x / y;
+  out[5 * n + i] = mdz::div_by_fp64(x, mdz::make_divisor(y));
 }
 
 __global__ void k_fx(const double *x, long long n, double *out) {
@@ -132,7 +138,7 @@ extern "C" int mdz_rheo_fx_pair_selftest(int device, const double *a, const doub
   if (cudaSetDevice(device) != cudaSuccess) return MDZ_ECUDA;
   const size_t bytes = (size_t)n * sizeof(double);
   double *d = nullptr;
-  if (cudaMalloc(&d, 4 * bytes) != cudaSuccess) return MDZ_ENOMEM;
+  if (cudaMalloc(&d, 8 * bytes) != cudaSuccess) return MDZ_ENOMEM;
   int rc = MDZ_OK;
   if (cudaMemcpy(d, a, bytes, cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(d + n, b, bytes, cudaMemcpyHostToDevice) != cudaSuccess)
@@ -141,7 +147,7 @@ extern "C" int mdz_rheo_fx_pair_selftest(int device, const double *a, const doub
     k_fx_pair<<<(unsigned)((n + 255) / 256), 256>>>(d, d + n, n, d + 2 * n);
     if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) rc = MDZ_ECUDA;
   }
-  if (rc == MDZ_OK && cudaMemcpy(out, d + 2 * n, 2 * bytes, cudaMemcpyDeviceToHost) != cudaSuccess) rc = MDZ_ECUDA;
+  if (rc == MDZ_OK && cudaMemcpy(out, d + 2 * n, 6 * bytes, cudaMemcpyDeviceToHost) != cudaSuccess) rc = MDZ_ECUDA;
   cudaFree(d);
   return rc;
 }

@@ -532,9 +532,10 @@ def fx_selftest(x: np.ndarray, device: int = 0):
 
 
 def fx_pair_selftest(a: np.ndarray, b: np.ndarray, device: int = 0):
-    """(a^b by the fixed-point power, by CUDA's pow) of the float64 arrays a, b on the GPU."""
+    """(a^b by the fixed-point power, a^b by CUDA's pow, and by the correctly rounded forms a b, 1 / a, a / b for b near 1,
+    a / b with a divisor formed on the device) of the float64 arrays a, b on the GPU."""
     a, b = np.ascontiguousarray(a, np.float64), np.ascontiguousarray(b, np.float64)
-    out = np.empty((2, a.size), np.float64)
+    out = np.empty((6, a.size), np.float64)
     rc = load_library().mdz_rheo_fx_pair_selftest(device, a.ctypes.data, b.ctypes.data, a.size, out.ctypes.data)
     if rc != MDZ_OK:
         raise RheoError(rc, "mdz_rheo_fx_pair_selftest")

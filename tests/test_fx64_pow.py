@@ -59,7 +59,7 @@ def test_host_build(tmp_path):
 @pytest.mark.gpu
 def test_gpu():
     x, y = arguments()
-    fixed, cuda = R.fx_pair_selftest(x, y)
+    fixed, cuda = R.fx_pair_selftest(x, y)[:2]
     check(x, y, fixed)
     with np.errstate(all="ignore"):
         ref = np.power(x.astype(LD), y.astype(LD))
