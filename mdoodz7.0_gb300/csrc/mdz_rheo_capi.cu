@@ -1672,6 +1672,15 @@ int mdz_rheo_strain_rates(mdz_rheo_ctx *ctx, const mdz_model *md, double dx, dou
   return finish(ctx, st);
 }
 
+// The marker kernels' mesh spacing.  Their cell index reads the magnitude of the divisor only;
+// a spacing that is not positive takes the division itself, which puts every marker outside the
+// grid (MDZ_EMARKER_OUT).
+static Divisor marker_spacing(double d) {
+  Divisor r = make_divisor(d);
+  if (!(d > 0.0)) r.fast = 0;
+  return r;
+}
+
 int mdz_rheo_marker_stress(mdz_rheo_ctx *ctx, const mdz_model *md, const mdz_marker_opts *o, mdz_marker_grid *g,
                            mdz_markers *mk, int mem, int flags, mdz_sweep_stats *st) {
   if (!ctx || !md || !o || !g || !mk) return MDZ_EINVAL;
@@ -1705,7 +1714,7 @@ int mdz_rheo_marker_stress(mdz_rheo_ctx *ctx, const mdz_model *md, const mdz_mar
     for (int p = 0; p < A.np; p++) A.G[p] = make_divisor(o->G[p]);
   }
   A.dt = md->dt;
-  A.dx = make_divisor(g->dx); A.dz = make_divisor(g->dz);
+  A.dx = marker_spacing(g->dx); A.dz = marker_spacing(g->dz);
   // P2Mastah's weight lengths, by its own expressions (ParticleRoutines.c:2218-2221)
   A.dx_itp = make_divisor(o->interp_stencil == 9 ? 3.0 * g->dx / 2.0 : g->dx / 2.0);
   A.dz_itp = make_divisor(o->interp_stencil == 9 ? 3.0 * g->dz / 2.0 : g->dz / 2.0);
@@ -1836,7 +1845,7 @@ int mdz_rheo_p2mastah(mdz_rheo_ctx *ctx, const mdz_model *md, const mdz_marker_g
   const size_t n = (size_t)mk->n;
   A.n = mk->n; A.Nx = md->Nx; A.Nz = md->Nz; A.periodic_x = md->periodic_x; A.np = md->Nb_phases;
   A.stencil = interp_stencil; A.avg = avg;
-  A.dx = make_divisor(g->dx); A.dz = make_divisor(g->dz);
+  A.dx = marker_spacing(g->dx); A.dz = marker_spacing(g->dz);
   // P2Mastah's weight lengths, by its own expressions (ParticleRoutines.c:2218-2221)
   A.dx_itp = make_divisor(interp_stencil == 9 ? 3.0 * g->dx / 2.0 : g->dx / 2.0);
   A.dz_itp = make_divisor(interp_stencil == 9 ? 3.0 * g->dz / 2.0 : g->dz / 2.0);
