@@ -95,9 +95,12 @@ extern "C" {
                                      (the same bits; for comparison) */
 #define MDZ_DEFAULT_POLISH   4    /* FP32 Newton steps before each FP64 local solve, by default */
 /* Start descriptor of the local solves (mdz_rheo_set_warmstart): FP32 Newton steps in the
- * low byte, plus MDZ_START_DD for one Halley step evaluated in double-float (FP32 pairs)
- * after them.  The default takes both, which puts the FP64 Newton's start within its
- * stopping tolerance, so it stops at its first evaluation. */
+ * low byte, plus MDZ_START_DD for a closing step from the point they reach.  With both (the
+ * default) sweeps and points close the solve in 64-bit fixed point: one evaluation of the
+ * residual, a Halley and a Newton step, which leave it below the reference's tolerance and
+ * count as one evaluation.  Where a number leaves the fixed-point formats, with MDZ_START_DD
+ * alone, and in mdz_rheo_operators, the closing step is a Halley step in double-float (FP32
+ * pairs) before the FP64 Newton, which then mostly stops at its first evaluation. */
 #define MDZ_START_DD         0x100
 #define MDZ_DEFAULT_START    (MDZ_DEFAULT_POLISH | MDZ_START_DD)
 
@@ -282,7 +285,9 @@ int mdz_rheo_destroy(mdz_rheo_ctx *ctx);
 /* Run the context's work on an external CUDA stream (cudaStream_t passed as
  * void*); NULL restores the context's own stream. */
 int mdz_rheo_set_stream(mdz_rheo_ctx *ctx, void *stream);
-/* Wait for an MDZ_SWEEP_ASYNC sweep and fetch its statistics. */
+/* Wait for an MDZ_SWEEP_ASYNC call and fetch its statistics.  An MDZ_SWEEP_ASYNC call may
+ * be captured into a caller's CUDA graph; after a replay this returns the replay's status
+ * and counts (elapsed_ms: of the last call if that was not the captured one, else 0). */
 int mdz_rheo_sync(mdz_rheo_ctx *ctx, mdz_sweep_stats *stats);
 /* Sweeps of host arrays (MDZ_MEM_HOST) run in bands of grid rows, so that the copies of
  * one band overlap the kernels of the others (with page-locked host arrays).  bands = 0
@@ -301,11 +306,10 @@ int mdz_rheo_host_access(mdz_rheo_ctx *ctx, int *pageable);
  * final stress.  `mem` is MDZ_MEM_HOST or MDZ_MEM_DEVICE; `stats` may be NULL.
  * Start of the local solves: the reference starts its visco-elastic Newton at the
  * smallest isolated viscosity (RheologyDensity.c:582-592; after 10 bisection steps in
- * the anisotropic routine, AnisotropyRoutines.c:474-497).  By default the FP64 Newton
- * here starts after MDZ_DEFAULT_POLISH FP32 Newton steps from that point and one
- * double-float Halley step (MDZ_DEFAULT_START); it still iterates to the reference's
- * residual tolerance (|r| < 1e-13 Eii), so results agree with the reference to that
- * tolerance.  MDZ_SWEEP_REF_START starts exactly where the reference does (same
+ * the anisotropic routine, AnisotropyRoutines.c:474-497).  By default the solve here
+ * takes MDZ_DEFAULT_POLISH FP32 Newton steps from that point and closes in fixed point
+ * (MDZ_DEFAULT_START); its residual still ends below the reference's tolerance
+ * (|r| < 1e-13 Eii), so results agree with the reference to that tolerance.  MDZ_SWEEP_REF_START starts exactly where the reference does (same
  * iteration counts).
  * Outputs should be arrays of their own: the vertices are updated beside the centroids.
  * Where an array used in place is passed twice (p_corr = p_in, say), every centroid is

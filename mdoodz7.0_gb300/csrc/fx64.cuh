@@ -26,7 +26,7 @@
 // step on a 24-bit estimate for the reciprocal and the reciprocal square root; the addition
 // theorems on a table of step 1/256 for sine and cosine.  Every intermediate carries 56 or
 // more bits behind the result's leading one, so the results are within 0.7 ulp (exp
-// and log: 1 ulp) of the exact values; arguments outside the ranges stated at each function take
+// and log: 0.8) of the exact values; arguments outside the ranges stated at each function take
 // CUDA's own function, special values included.
 //
 // The code compiles for the host too (the CPU test runs it there); only the starting

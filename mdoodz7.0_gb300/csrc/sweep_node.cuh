@@ -23,7 +23,9 @@ __device__ __forceinline__ void record_error(DevStats *st, long long node, int s
 __device__ __forceinline__ void pair_begin() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void pair_end() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-struct Acc {  // of one thread: below 2^32 for any grid that fits the device (a thread's items x 70)
+// Counts of one thread.  Below 2^32 for launches of any ordinary length: an item adds at most 70
+// to each, so it takes 60 M items in one thread, hours of a launch of one CTA (grid cap 1).
+struct Acc {
   unsigned int calls, iters, plastic, maxit;
   unsigned int f32;  // FP32 Newton steps of the starts
 };

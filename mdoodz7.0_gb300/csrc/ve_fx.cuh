@@ -12,7 +12,7 @@
 // Before, the same start was moved by a Halley step in double-float (FP32 pairs) and then
 // confirmed by one FP64 evaluation of r, a logarithm, an exponential per law and the
 // residual: about 36 FP64 instructions, 20 cycles each, and as many FP32 ones as this takes
-// integer ones.  The 2049 x 2049 sweep went from 15.58 to 9.92 ms and the anisotropic
+// integer ones.  The 2049 x 2049 sweep went from 15.58 to 9.97 ms and the anisotropic
 // 1025 x 1025 one from 2.58 to 1.63 ms; no local solve of either declines.
 //
 // The fast form declines (returns false, nothing written) where a number would leave its
