@@ -1241,7 +1241,6 @@ struct IsoMid {
 struct DpItem {
   double Tii, Tyield, eta_ve, P, K, sin_fric, sin_dil, Eii, inv2Eii;  // in; Tii, Tyield out
   double gdot, divp, Pc, eta_vp, eta_vep;                              // out
-  double pl_share, T_over_eta;                                         // out (dp_return_call)
 };
 
 __device__ __forceinline__ bool iso_yields_dp(const ModelConst &M, const PhaseConst &ph, const NodeCtx &c,
@@ -1325,10 +1324,9 @@ __device__ inline void dp_return(const ModelConst &M, const PhaseConst &ph, DpIt
 // power and quotients on the integer pipe; with CUDA's pow and divisions, up to 20 times for
 // the few yielding lanes of nearly every warp, a 1025 x 1025 sweep with n_vp = 2 took 24.9 ms
 // (15.3 gathered per CTA), and takes 5.4; with dilation and n_vp = 1 3.9 -> 3.3.
-static __device__ __noinline__ void dp_return_call(const ModelConst &M, const PhaseConst &ph, DpItem &d) {
-  dp_return<FxMath>(M, ph, d);
-  d.pl_share = d.eta_ve * d.gdot * fx_recip_call(d.Tii);
-  d.T_over_eta = d.Tii * fx_recip_call(d.eta_ve);
+static __device__ __noinline__ DpItem dp_return_call(const ModelConst &M, const PhaseConst &ph, DpItem d) {
+  dp_return<FxMath>(M, ph, d);  // on a copy of its own: through a reference the iteration's state stays in memory
+  return d;
 }
 
 __device__ __forceinline__ void dp_return_inline(const ModelConst &M, const PhaseConst &ph, const NodeIn &in,
@@ -1352,9 +1350,10 @@ __device__ __forceinline__ void dp_return_inline(const ModelConst &M, const Phas
   }
   DpItem d;
   dp_load(d, m, in, c);
-  dp_return_call(M, ph, d);
+  d = dp_return_call(M, ph, d);
   dp_store(m, d);
-  m.pl_share = d.pl_share; m.T_over_eta = d.T_over_eta;
+  m.pl_share = d.eta_ve * d.gdot * fx_recip_call(d.Tii);
+  m.T_over_eta = d.Tii * fx_recip_call(d.eta_ve);
 }
 
 // Local solve (from s_start * eta_up, moved by the start stages that the descriptor
