@@ -21,7 +21,7 @@ namespace mdz {
 // MINB: CTAs of 128 per SM that the register allocation is capped for.  A node's code is a
 // long chain of dependent integer and FP64 instructions, and more resident warps hide more of
 // its latency than the spills cost: 7 (72 registers) by default.  A sweep of a few waves
-// loses more to its last, partly empty one, and 5 (96 registers) wins there (sweep_ctas).
+// may lose more to its last, partly empty one, and take 5 (96 registers; sweep_ctas).
 // Per call, in us, at 5, 6, 7 and 8 CTAs per SM:
 //   isotropic, 5 phases     201^2: 124, 126, 124, 121    401^2: 328, 344, 351, 347
 //     513^2: 493, 505, 446, 463    717^2: 937, 903, 840, 885    1025^2: 1862, 1787, 1703, 1757
@@ -183,12 +183,21 @@ static bool kernels_share(const SweepArgs &a) {
 }
 
 // CTAs of 128 per SM for a sweep of so many nodes, centroids and vertices together (their
-// kernels overlap): 5 between one and 3.5 waves of the 152 SMs' 7 CTAs, where the last wave's
-// idle SMs cost more than the fifth to seventh CTA's warps gain (517 x 389 cells with air, 3
-// waves: 289, 300 and 308 us at 5, 6 and 7; 513 x 513, 3.9 waves: 493, 505 and 446).
+// kernels overlap).  A call's time steps up where the nodes pass 1, 2 and 4 waves of the
+// resident CTAs, with 5 CTAs per SM at 5/7 of the nodes but from a lower level, so each form is
+// the faster one in turn.  In us at 5 and 7, without air and with a fifth of the rows air, whose
+// nodes cost nothing and shift the steps to 5/4 of the nodes (waves of 152 x 7 CTAs):
+//   1.0: 159, 170  1.2: 174, 181; 154, 140  1.4: 191, 194; 168, 176    5 (2-7 %, or loses 10 %)
+//   1.7: 276, 214; 184, 189       2.0: 286, 252; 259, 208              7 (13-29 %)
+//   2.3: 306, 334; 274, 224       2.6: 326, 356; 281, 295              5 (9 %, or loses 20 %)
+//   3.0: 407, 374; 311, 337       3.5: 440, 403; 340, 361              5 with air, 7 without
+//   3.9: 472, 437; 409, 376                                            7
+// 5 also up to 3.5, for grids with air (517 x 389 cells: 289, 300 and 308 us at 5, 6 and 7).
+// The anisotropic sweep steps alike (1.4: 153, 161; 1.7: 203, 172; 2.6: 258, 269).
 static int sweep_ctas(long long nodes) {
-  const long long wave = 152LL * 7 * 128;
-  return (nodes > wave && 2 * nodes < 7 * wave) ? 5 : 7;
+  const long long wave = 152LL * 7 * 128, wave5 = 152LL * 5 * 128;
+  if (nodes <= wave || 2 * nodes >= 7 * wave) return 7;
+  return (nodes > 2 * wave5 && nodes <= 2 * wave + wave / 40) ? 7 : 5;
 }
 
 template <bool ANISO, int NODES>

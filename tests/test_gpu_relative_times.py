@@ -65,3 +65,15 @@ def test_points_with_the_grain_size_solve(ctx):
     few, many = seconds(100), seconds(400)
     print("points", many / few)
     assert many < 3.15 * few
+
+
+def test_sweep_between_one_and_two_waves(ctx):
+    """340 x 340 cells against 310 x 310 (1.2 times the nodes, both two waves of resident CTAs at 7 per SM): 1.1 times
+    (1.45 where the larger grid ran 5 CTAs per SM, in three waves)."""
+    t = {}
+    for n in (310, 340):
+        w = W.plain_large(seed=3, ncx=n)
+        F = R.FieldSet(on_device(w.arrays))
+        t[n] = kernel_ms(lambda: ctx.sweep(w.model, w.mat, F, mem=R.MEM_DEVICE), 25)
+    print("340 / 310", t[340] / t[310])
+    assert t[340] < 1.3 * t[310]
