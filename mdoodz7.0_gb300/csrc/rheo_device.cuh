@@ -440,9 +440,13 @@ struct VeState {
   int iters, status;
 };
 
-// strain rates over Eii
+// What the strain rates of sweeps and points are divided by inside: Eii, or 1 where that is not
+// finite, so that the rate of a law that is off stays 0.
+__device__ __forceinline__ double rate_unit(double Eii) { return fp64_finite(Eii) ? Eii : 1.0; }
+
+// strain rates over rate_unit(Eii)
 __device__ __forceinline__ void ve_normalise(VeState &s, double Eii) {
-  const double i = fx_recip_call(Eii);
+  const double i = fx_recip_call(rate_unit(Eii));
   s.e_cst *= i; s.e_pwl *= i; s.e_exp *= i; s.e_lin *= i;
 }
 
@@ -743,7 +747,9 @@ __device__ __forceinline__ bool ve_solve_fx(const PhaseConst &ph, const Laws &L,
   VeFxRoot r;
   if (!ve_root_fx(nl, lin, N, X, nf, s0, r)) return false;
   s.eta = fx_normalise(r.S, k2 - 62);
-  s.Tii = fp64_scale(s.eta * c.Eii, 1);
+  const double half = s.eta * c.Eii;
+  if (!fp64_finite(half)) return false;  // nor is Eii, of which Newtonian laws know nothing (tested here for free)
+  s.Tii = fp64_scale(half, 1);
   s.e_cst = (L.mech & F_CST) ? s.eta * inv_cst : 0.0;
   double e[K_COUNT];
 #pragma unroll
@@ -1400,7 +1406,7 @@ __device__ inline void iso_ve(const ModelConst &M, const PhaseConst &ph, const N
     o.d1 = dd;
     o.inv_d1 = 1.0 / dd;
     if (FP::kFixed) {
-      const double i = FP::recip(Eii);
+      const double i = FP::recip(rate_unit(Eii));
       e_cst *= i; e_pwl *= i; e_exp *= i; e_lin *= i;
     }
   }
@@ -1464,7 +1470,7 @@ __device__ inline void iso_post(const ModelConst &M, const PhaseConst &ph, const
   const double eta_cst = S.eta_cst, C = S.C, lnd = S.lnd;
   (void)T;
   const double eta_ve = m.eta_ve, Tii_ve = m.Tii_ve;
-  const double unit = FP::kFixed ? Eii : 1.0;
+  const double unit = FP::kFixed ? rate_unit(Eii) : 1.0;
   const double e_cst = m.e_cst * unit, e_pwl = m.e_pwl * unit, e_exp = m.e_exp * unit, e_lin = m.e_lin * unit;
   double Tii = m.Tii;
   int is_pl = m.is_pl;
@@ -1756,6 +1762,10 @@ static __device__ __noinline__ VeOut aniso_general_fx(const ModelConst &M, VeArg
   o.s.status = MDZ_OK;
   aniso_general_inl<FxMath>(M, v, o.s, o.f32_steps);
   ve_normalise(o.s, v.Eii);
+  if (fp64_is_inf(v.Eii)) {  // no viscosity, an infinite stress (and MDZ_EANISO_NAN from the residual)
+    o.s.eta = __longlong_as_double(0x7ff8000000000000ll);
+    o.s.Tii = v.Eii;
+  }
   return o;
 }
 
@@ -1814,7 +1824,7 @@ __device__ inline void aniso_finish(const ModelConst &M, const PhaseConst &ph, c
     set_status(o.status, s.status);
     eta_ve = s.eta;
     o.iters = s.iters;
-    const double unit = FP::kFixed ? Eii : 1.0;
+    const double unit = FP::kFixed ? rate_unit(Eii) : 1.0;
     Tii = s.Tii; e_cst = s.e_cst * unit; e_pwl = s.e_pwl * unit; e_exp = s.e_exp * unit; e_lin = s.e_lin * unit;
   }
   eta_ve = clamp_eta(M, eta_ve);  // :589-603

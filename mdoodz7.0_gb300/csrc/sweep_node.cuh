@@ -375,10 +375,11 @@ __device__ __forceinline__ void iso_store(const SweepArgs &A, const Node &n, Iso
     if (NODES == 1) {
       out[CO_eII_el] = c.elastic ? q.el * fp64_scale(c.inv_eta_el, -1) : 0.0;
       out[CO_eII_pl] = fp64_scale(q.pl, -1);
-      out[CO_eII_pwl] = q.pwl * c.Eii;
-      out[CO_eII_exp] = q.exp * c.Eii;
-      out[CO_eII_lin] = q.lin * c.Eii;
-      out[CO_eII_cst] = q.cst * c.Eii;
+      const double unit = rate_unit(c.Eii);
+      out[CO_eII_pwl] = q.pwl * unit;
+      out[CO_eII_exp] = q.exp * unit;
+      out[CO_eII_lin] = q.lin * unit;
+      out[CO_eII_cst] = q.cst * unit;
       out[CO_d] = q.d;
       out[CO_Wtot] = q.Wtot;
       out[CO_Wdiss] = q.Wdiss;
