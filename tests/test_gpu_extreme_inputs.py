@@ -68,3 +68,14 @@ def test_sweeps_with_a_strain_rate_that_is_not_finite(ctx, field, avg):
     same_nan(got, ref, ["eta_n", "eta_s", "sxxd", "szzd", "sxz_n", "sxxd_s", "sxz", "eII_pl", "eII_pwl", "eII_lin", "p_corr"])
     for s in "ns":
         same_nan(dict(enumerate(got["phase_eta_" + s])), dict(enumerate(ref["phase_eta_" + s])), range(5))
+
+
+@pytest.mark.parametrize("value", [0.0, 1e-310, 1e-300, np.nan])
+def test_sweeps_without_a_finite_bulk_modulus_over_a_step(ctx, value):
+    """K dt is infinite: a yielding node's return has no pressure, and the harmonic average is an error."""
+    for avg in (0, 1):
+        w = W.plain_large(seed=3, ncx=24, eta_average=avg)
+        for s in "ns":
+            w.arrays["bet_" + s][::5] = value
+        got, ref = run_sweeps(ctx, w)
+        same_nan(got, ref, ["eta_n", "eta_s", "sxxd", "sxz_n", "sxxd_s", "p_corr"])
