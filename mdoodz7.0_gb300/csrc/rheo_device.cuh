@@ -195,6 +195,19 @@ __device__ __forceinline__ double clamp_eta(const ModelConst &M, double x) {
   return x;
 }
 
+// the same with the lower limit first, as the anisotropic routine applies it to eta_ve and
+// eta_vep (AnisotropyRoutines.c:589-603): the upper one holds where the limits cross
+__device__ __forceinline__ double clamp_eta_low(const ModelConst &M, double x) {
+  if (M.eta_pos) {
+    if (fp64_lt_pos(x, M.min_eta)) x = M.min_eta;
+    if (fp64_gt_pos(x, M.max_eta)) x = M.max_eta;
+  } else {
+    if (fp64_lt(x, M.min_eta)) x = M.min_eta;
+    if (fp64_gt(x, M.max_eta)) x = M.max_eta;
+  }
+  return x;
+}
+
 // ---------------------------------------------------------------------------------------
 // node set-up: invariants and switches shared by the phases (RheologyDensity.c:461-496)
 // ---------------------------------------------------------------------------------------
@@ -1828,7 +1841,7 @@ __device__ inline void aniso_finish(const ModelConst &M, const PhaseConst &ph, c
     const double unit = FP::kFixed ? rate_unit(Eii) : 1.0;
     Tii = s.Tii; e_cst = s.e_cst * unit; e_pwl = s.e_pwl * unit; e_exp = s.e_exp * unit; e_lin = s.e_lin * unit;
   }
-  eta_ve = clamp_eta(M, eta_ve);  // :589-603
+  eta_ve = clamp_eta_low(M, eta_ve);  // :589-603
   const double Tii_ve = Tii;
   if (eta_conv) *eta_conv = eta_ve;
   double Tr_xx = 2.0 * eta_ve * an.Er_xx, Tr_zz = 2.0 * eta_ve * an.Er_zz, Tr_xz = 2.0 * eta_ve * an.Er_xz / in.ani_fac;
@@ -1857,7 +1870,7 @@ __device__ inline void aniso_finish(const ModelConst &M, const PhaseConst &ph, c
     o.Txz = lxlz * Tr_xx - lxlz * Tr_zz + (lx2 - nz2) * Tr_xz;
   }
   o.Pcorr = Pc;
-  eta_vep = clamp_eta(M, eta_vep);
+  eta_vep = clamp_eta_low(M, eta_vep);
   o.etaVE = eta_vep;
   o.is_pl = is_pl;
   if (is_pl) o.mech |= MDZ_MECH_YIELD;

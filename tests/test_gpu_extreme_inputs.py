@@ -79,3 +79,13 @@ def test_sweeps_without_a_finite_bulk_modulus_over_a_step(ctx, value):
             w.arrays["bet_" + s][::5] = value
         got, ref = run_sweeps(ctx, w)
         same_nan(got, ref, ["eta_n", "eta_s", "sxxd", "sxz_n", "sxxd_s", "p_corr"])
+
+
+@pytest.mark.parametrize("low,high", [(1e18, 1e17), (1e18, 1e-5), (1e18, 0.0)])
+def test_anisotropic_limits_that_cross(ctx, low, high):
+    """The upper limit is applied last to the visco-elastic and the visco-plastic viscosity."""
+    w = W.aniso(seed=3, ncx=24)
+    w.model.min_eta, w.model.max_eta = low, high
+    got, ref = run_sweeps(ctx, w, aniso=True)
+    for k in ("eta_n", "eta_s"):
+        assert np.allclose(got[k], ref[k], rtol=1e-12, atol=0.0, equal_nan=True), k
