@@ -350,7 +350,10 @@ __device__ __forceinline__ void iso_accumulate(const SweepArgs &A, const Node &n
   q.Wtot = __dadd_rn(q.Wtot, w);
   q.Wdiss = fma(w, share, q.Wdiss);
   q.Wel = fma(pT, m.Tii, q.Wel);
-  if ((int)fp64_hi(share) < 0 && fp64_lt(share, 0.0) && !fp64_is_zero(m.Tii)) set_status(status, MDZ_EWDISS);
+  // Tii^2 share / eta_ve below zero (:1045-1050)
+  if ((int)(fp64_hi(share) ^ fp64_hi(m.eta_ve)) < 0 && fp64_abs_gt(share, 0.0) && fp64_abs_gt(m.eta_ve, 0.0) &&
+      !fp64_is_zero(m.Tii))
+    set_status(status, MDZ_EWDISS);
   if (m.is_pl && (fp64_bits(m.Pc) != fp64_bits(n.in.P) || !fp64_is_zero(m.divp))) {
     q.dP = fma(perc, m.Pc - n.in.P, q.dP);
     q.div_pl = fma(perc, m.divp, q.div_pl);

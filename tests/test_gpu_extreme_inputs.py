@@ -89,3 +89,10 @@ def test_anisotropic_limits_that_cross(ctx, low, high):
     got, ref = run_sweeps(ctx, w, aniso=True)
     for k in ("eta_n", "eta_s"):
         assert np.allclose(got[k], ref[k], rtol=1e-12, atol=0.0, equal_nan=True), k
+
+
+def test_sweep_with_a_negative_shear_modulus(ctx):
+    """Stress and viscosity are negative, and the dissipation is not: no error."""
+    w = W.plain_large(seed=3, ncx=24)
+    w.arrays["mu_n"][::7] = -1.0
+    run_sweeps(ctx, w)
