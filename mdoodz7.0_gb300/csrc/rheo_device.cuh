@@ -1351,7 +1351,7 @@ static __device__ __noinline__ DpItem dp_return_call(const ModelConst &M, const 
 __device__ __forceinline__ void dp_return_inline(const ModelConst &M, const PhaseConst &ph, const NodeIn &in,
                                                  const NodeCtx &c, IsoMid &m) {
   // (K dt that is not finite leaves no pressure in the iteration, whose zero dilation it multiplies)
-  if ((ph.flags & F_VP1) && fp64_is_zero(c.sin_dil) && fp64_exponent(c.inv_Kdt) - 1u < 0x7feu) {
+  if ((ph.flags & F_VP1) && fp64_exponent(c.inv_Kdt) - 1u < 0x7feu && fp64_is_zero(c.sin_dil)) {
     const bool rigid = fp64_is_zero(ph.eta_vp);
     // rounded one by one: the same bits in every kernel
     const double F = __dsub_rn(m.Tii, m.Tyield);

@@ -287,6 +287,11 @@ struct IsoAcc {
   double el, pl, pwl, exp, lin, cst, d, Wtot, Wel, Wdiss, dP, div_pl, OverS, rho;  // centroids
 };
 
+// Tii^2 share / eta_ve below zero (:1045-1050); asked where the signs differ, so out of line
+static __device__ __noinline__ bool dissipation_negative(double share, double eta_ve, double Tii) {
+  return Tii * Tii * (share / eta_ve) < 0.0;
+}
+
 template <int NODES>
 __device__ __forceinline__ void iso_accumulate(const SweepArgs &A, const Node &n, int p, double perc, const IsoState &S,
                                                PointOut &o, IsoMid &m, IsoAcc &q, Acc &acc, int &status) {
@@ -350,9 +355,7 @@ __device__ __forceinline__ void iso_accumulate(const SweepArgs &A, const Node &n
   q.Wtot = __dadd_rn(q.Wtot, w);
   q.Wdiss = fma(w, share, q.Wdiss);
   q.Wel = fma(pT, m.Tii, q.Wel);
-  // Tii^2 share / eta_ve below zero (:1045-1050)
-  if ((int)(fp64_hi(share) ^ fp64_hi(m.eta_ve)) < 0 && fp64_abs_gt(share, 0.0) && fp64_abs_gt(m.eta_ve, 0.0) &&
-      !fp64_is_zero(m.Tii))
+  if ((int)(fp64_hi(share) ^ fp64_hi(m.eta_ve)) < 0 && dissipation_negative(share, m.eta_ve, m.Tii))
     set_status(status, MDZ_EWDISS);
   if (m.is_pl && (fp64_bits(m.Pc) != fp64_bits(n.in.P) || !fp64_is_zero(m.divp))) {
     q.dP = fma(perc, m.Pc - n.in.P, q.dP);
