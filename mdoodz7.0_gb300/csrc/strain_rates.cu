@@ -15,7 +15,7 @@
 // the FP64 instruction count low wherever that leaves every result bit unchanged.
 // The divisions by the mesh spacing run on the integer pipe (fp64_div.cuh), as do products
 // with powers of two: 1025 x 1025 cells 134 -> 107 -> 92 us; 283 -> 140 us where all velocities
-// are equal (zeros take a call, not the integer forms).
+// are equal, whose zeros are answered before the FP64 forms.
 //
 // Every operation rounds as the reference's does (divisions by the mesh spacing are
 // correctly rounded, fp64_div.cuh; the products and sums that a compiler could contract
@@ -78,8 +78,8 @@ __global__ void __launch_bounds__(kSrTx * kSrTz) k_strain_rates(const StrainArgs
       double dv = 0.0, ex = 0.0, ez = 0.0;
       if (in) {
         const long long c1 = ck + (long long)cl * Nx, c2 = ck + (long long)cl * (Nx + 1);
-        const double dvxdx = div_by(A.u[c1 + 1 + Nx] - A.u[c1 + Nx], dx);
-        const double dvzdz = div_by(A.v[c2 + Nx + 2] - A.v[c2 + 1], dz);
+        const double dvxdx = div_by<true>(A.u[c1 + 1 + Nx] - A.u[c1 + Nx], dx);
+        const double dvzdz = div_by<true>(A.v[c2 + Nx + 2] - A.v[c2 + 1], dz);
         const double s = __dadd_rn(dvxdx, dvzdz);
         // (a zero share of a finite s leaves s)
         dv = fp64_is_zero(A.oop_half) && fp64_finite(s) ? s : __dadd_rn(s, __dmul_rn(A.oop_half, s));
@@ -96,8 +96,8 @@ __global__ void __launch_bounds__(kSrTx * kSrTz) k_strain_rates(const StrainArgs
       const bool in = A.bcg[c1] != 30;
       double e = 0.0, w = 0.0;
       if (in) {
-        const double dvxdz = div_by(A.u[c1 + Nx] - A.u[c1], dz);
-        const double dvzdx = div_by(A.v[c2 + 1] - A.v[c2], dx);
+        const double dvxdz = div_by<true>(A.u[c1 + Nx] - A.u[c1], dz);
+        const double dvzdx = div_by<true>(A.v[c2 + 1] - A.v[c2], dx);
         e = fp64_scale(__dadd_rn(dvxdz, dvzdx), -1);
         w = fp64_scale(__dsub_rn(dvzdx, dvxdz), -1);
       }
